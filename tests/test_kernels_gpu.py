@@ -758,15 +758,17 @@ def test_a_bounded_wait_that_runs_out_is_reported_and_the_device_stays_usable():
 
 
 @pytest.mark.parametrize("lens, nh, nkv, d, page, window, subset", [
-    ([0, 63, 64, 700, 5, 1300] * 30, 14, 2, 64, 16, None, False),  # shares too short to cut: a CTA an item
-    ([0, 63, 64, 4000, 5, 1300, 900] * 10, 28, 4, 128, 16, None, False),  # items cut over CTAs, several items a CTA
-    ([9000, 3, 128, 2000] * 10, 8, 8, 64, 64, None, True),  # one item over many CTAs; only some requests of the step
+    ([0, 63, 64, 700, 5, 1300] * 30, 14, 2, 64, 16, None, False),  # a CTA an item
+    ([0, 63, 64, 4000, 5, 1300, 900] * 10, 28, 4, 128, 16, None, False),
+    ([9000, 3, 128, 2000] * 10, 8, 8, 64, 64, None, True),  # one item over several CTAs; only some requests of the step
     ([3000, 200, 1023, 4096] * 30, 4, 2, 128, 8, 1024, False),  # a window
-    ([40] * 384, 4, 2, 64, 16, None, False),  # the most requests, more items than CTAs
+    ([40] * 384, 4, 2, 64, 16, None, False),  # more items than CTAs are resident
 ])
 def test_attention_mma_walks_the_tiles_of_all_requests(lens, nh, nkv, d, page, window, subset):
-    """One wave of CTAs shares the key tiles of all (request, KV head) items: against float64 within bfloat16's rounding of the
+    """Large batches of unequal lengths with the engine's key splits: against float64 within bfloat16's rounding of the
     weights and the result (2 x 2^-8 of the values' size), twice in a row (the arrival counters go back to zero)."""
+    from torchlet_b200.parts.attention_bf16 import decode_splits
+
     ops = _ops()
     g, R = torch.Generator(device=DEV).manual_seed(7), len(lens)
     counts = [n // page + 1 for n in lens]
@@ -793,11 +795,11 @@ def test_attention_mma_walks_the_tiles_of_all_requests(lens, nh, nkv, d, page, w
     indptr = torch.arange(R + 1, dtype=torch.int32, device=DEV)
     before = torch.tensor(lens, dtype=torch.int32, device=DEV)
     tile_req = torch.tensor(chosen, dtype=torch.int32, device=DEV) if subset else None
-    assert ops.decode_walk_supported(len(chosen), page)
+    splits = decode_splits(len(chosen), nkv, max(lens) + 1)
     for _ in range(2):
         out = torch.full((R, nh * d), float("nan"), device=DEV, dtype=torch.bfloat16)
         ops.attention_mma(qkv, pages, table, indptr, before, tile_req, None, len(chosen), out, R, nh, nkv, d, page, window,
-                          d ** -0.5, True, splits=0)
+                          d ** -0.5, True, splits=splits)
         assert torch.equal(torch.isnan(out), torch.isnan(want))
         assert (out.double() - want).nan_to_num().abs().max() <= 2 * 2.0 ** -8 * want.nan_to_num().abs().max()
 

@@ -45,8 +45,6 @@ __device__ int g_error_word = 0;
 constexpr int WARPS = 4;
 constexpr int THREADS = WARPS * 32;
 constexpr int BLOCK_N = 64;  // keys per tile
-constexpr int WALK_MAX = 384;  // WALK: requests whose lengths a CTA keeps
-constexpr int WALK_LEAST = 8;  // WALK: key tiles of a share below which a CTA takes a whole item instead (no partial results)
 
 struct Params {
   const __nv_bfloat16* q;  // packed qkv rows; query head h of token t at q + t*q_stride + h*D
@@ -64,7 +62,6 @@ struct Params {
   float* part_ml;   // [tiles*nh][splits][2]
   int* arrivals;    // [tiles*nkv] zero between launches: splits of a (tile, KV head) that have written (null: a second kernel merges)
   int nh, nkv, page_size, window, splits;
-  int tiles;       // row tiles (WALK: requests) in all
   int num_pages;   // pages in the pool (checked in the debug build)
   int page_shift;  // log2(page_size) when it is a power of two, else -1
   int overlap_max_tiles;  // host only: overlapped launch up to this many row tiles
@@ -245,21 +242,9 @@ __device__ __forceinline__ int effective_splits(int splits, int key_tiles) {
 
 // STAGES: key/value tiles in shared memory; 2, or 3 with the TMA loader where the grid leaves
 // room for only two CTAs an SM anyway.
-// WALK: the CTAs of a one-wave grid share the key tiles of ALL (request, KV head) items evenly.  The items' tiles are counted
-// through in order (a prefix sum over the requests' lengths, taken by every CTA); CTA c walks tiles [c W, (c + 1) W) of that
-// count, one SEGMENT of an item after the other.  An item that lies in one CTA is finished there, one that several share by the
-// last of them to arrive (part_acc / part_ml: two entries a CTA, for the segment that continues an item of the CTAs before
-// and for the one that begins an item of the CTAs behind).  Shares of fewer than WALK_LEAST tiles are not worth their partial
-// results: then every CTA takes one item.
-// What the walk is for: with more items than SMs the launch that is not walked has room for one or two CTAs an item, and the
-// longest requests' run on alone.  64 requests of 300 to 3,000 tokens, 4 KV heads of 128: 74 -> 54 us (3,310 -> 4,520 GB/s of
-// keys and values), all at 3,000: 76 -> 71, 128 at 2,048: 109 -> 95, 40 of up to 2,000: 34 -> 30; 64 at 1,024: 32.6 -> 33.2.  With
-// fewer items than SMs (24 of up to 2,100 tokens, split four ways: 21 us against 23) the prefix sum and the partial results of
-// its segments cost more than the even shares give.
-template <int D, bool ROWS16, bool TMA, int STAGES, bool EXTRAS, bool WALK>
+template <int D, bool ROWS16, bool TMA, int STAGES, bool EXTRAS>
 __global__ void __launch_bounds__(THREADS, STAGES == 2 ? 3 : 2)
 attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
-  static_assert(!WALK || TMA, "only the TMA tiles are walked");
   static_assert(!TMA || ROWS16, "the TMA loader serves the 16-row tiles");
   static_assert(STAGES == 2 || TMA, "more than two stages need the TMA loader");
   // The wait on the preceding kernel comes further down: the step's metadata is written
@@ -288,107 +273,20 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(full + STAGES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int req = p.tile_req ? p.tile_req[blockIdx.x] : blockIdx.x;
+  const int row_start = p.tile_row ? p.tile_row[blockIdx.x] : 0;
+  const int kvh = blockIdx.y;
+  const int split = blockIdx.z;
   const int g = p.nh / p.nkv;
-  if constexpr (TMA) {
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], 1);
-      *abort_flag = 0;
-      tc::mbar_fence_init();
-      tc::prefetch_tensormap(&map_kv);
-    }
-  }
-  // ---- WALK: this CTA's share of the key tiles of all items
-  int walked = 0, walk_end = 0, share = 1;  // next tile, end and length of the share
-  bool whole = false;                       // one item a CTA
-  // of every request: key tiles of a KV head up to and with it, cached tokens, first token of the step
-  int* tiles_through = reinterpret_cast<int*>(full + STAGES + 1);
-  int* cached_of = tiles_through + WALK_MAX;
-  int* token_of = cached_of + WALK_MAX;
-  if constexpr (WALK) {
-    __shared__ int warp_tiles[WARPS];
-    int before_these = 0;
-    for (int base = 0; base < p.tiles; base += THREADS) {
-      const int i = base + threadIdx.x;
-      int n = 0;
-      if (i < p.tiles) {
-        const int r = p.tile_req ? p.tile_req[i] : i, last = p.kv_before[r], token = p.req_indptr[r];
-        if (p.req_indptr[r + 1] > token) n = last / BLOCK_N + 1 - tl::first_key(last, p.window) / BLOCK_N;
-        cached_of[i] = last;
-        token_of[i] = token;
-      }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int below = __shfl_up_sync(0xffffffffu, n, o);
-        if (lane >= o) n += below;
-      }
-      if (lane == 31) warp_tiles[warp] = n;
-      __syncthreads();
-      int all_here = 0;
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) {
-        if (w < warp) n += warp_tiles[w];
-        all_here += warp_tiles[w];
-      }
-      if (i < p.tiles) tiles_through[i] = before_these + n;
-      before_these += all_here;
-      __syncthreads();
-    }
-    const int all = tiles_through[p.tiles - 1] * p.nkv;
-    share = (all + (int)gridDim.x - 1) / (int)gridDim.x;
-    whole = share < WALK_LEAST && p.tiles * p.nkv <= (int)gridDim.x;
-    if (whole) {
-      const int r = blockIdx.x / p.nkv;
-      if (r < p.tiles) {
-        const int before_it = r > 0 ? tiles_through[r - 1] : 0, mine = tiles_through[r] - before_it;
-        walked = before_it * p.nkv + (int)(blockIdx.x % p.nkv) * mine;
-        walk_end = walked + mine;
-      }
-    } else {
-      walked = min(all, (int)blockIdx.x * share);
-      walk_end = min(all, walked + share);
-    }
-    if (walked >= walk_end) {
-      tl::pdl_wait();
-      return;
-    }
-  } else if constexpr (TMA) {
-    __syncthreads();
-  }
-
-  int done = 0;  // tiles of earlier segments: the stages and their barriers' phases run on
-  do {
-  int item_tile = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;  // (WALK: tile, KV head and number of the segment of its item)
-  int segment_begin = 0, segment_tiles = 0, first_cta = 0, my_splits = 1;
-  if constexpr (WALK) {
-    int lo = 0, hi = p.tiles - 1;  // the first request whose tiles reach past ``walked``
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (tiles_through[mid] * p.nkv > walked) hi = mid;
-      else lo = mid + 1;
-    }
-    item_tile = lo;
-    const int before_it = lo > 0 ? tiles_through[lo - 1] : 0, mine = tiles_through[lo] - before_it;
-    const int within = walked - before_it * p.nkv;
-    kvh = within / mine;
-    segment_begin = within - kvh * mine;
-    segment_tiles = min(mine - segment_begin, walk_end - walked);
-    const int item_first = walked - segment_begin;
-    first_cta = item_first / share;
-    split = whole ? 0 : (int)blockIdx.x - first_cta;
-    my_splits = whole ? 1 : (item_first + mine - 1) / share - first_cta + 1;
-    walked += segment_tiles;
-  }
-  const int req = p.tile_req ? p.tile_req[item_tile] : item_tile;
-  const int row_start = p.tile_row ? p.tile_row[item_tile] : 0;
-  const int tok0 = WALK ? token_of[item_tile] : p.req_indptr[req];
-  const int q_len = WALK ? 1 : p.req_indptr[req + 1] - tok0;
-  const int before = WALK ? cached_of[item_tile] : p.kv_before[req];
+  const int tok0 = p.req_indptr[req];
+  const int q_len = p.req_indptr[req + 1] - tok0;
+  const int before = p.kv_before[req];
   const int total_rows = q_len * g;
   const int* table = p.block_table + (size_t)req * p.table_width;
 
   // rows of this tile: [row_start, row_end)
   const int row_end = min(total_rows, row_start + BLOCK_M);
-  if (!WALK && row_start >= row_end) {
+  if (row_start >= row_end) {
     tl::pdl_wait();
     return;
   }
@@ -398,10 +296,8 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
 
   // key tiles of this CTA
   int tile_begin = lo_key / BLOCK_N, tile_end = hi_key / BLOCK_N + 1;
-  if constexpr (WALK) {
-    tile_begin += segment_begin;
-    tile_end = tile_begin + segment_tiles;
-  } else if (p.splits > 1) {
+  int my_splits = 1;
+  if (p.splits > 1) {
     my_splits = effective_splits(p.splits, tile_end - tile_begin);
     if (split >= my_splits) {  // the request is too short to need this CTA
       tl::pdl_wait();
@@ -411,6 +307,15 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
     tile_begin = tile_begin + split * per;
     tile_end = min(tile_end, tile_begin + per);
   }
+  if constexpr (TMA) {
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], 1);
+      *abort_flag = 0;
+      tc::mbar_fence_init();
+      tc::prefetch_tensormap(&map_kv);
+    }
+    __syncthreads();
+  }
 
   // ---- key/value tiles that earlier steps wrote may be requested before the wait
   constexpr int STAGE_ELEMS = 2 * BLOCK_N * D;
@@ -418,10 +323,9 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   int issued = 0;  // tiles requested so far, counted from tile_begin
   if constexpr (ROWS16) {
     while (issued < min(STAGES, num_tiles) && (tile_begin + issued) * BLOCK_N + BLOCK_N - 1 < before) {
-      const int s_next = (done + issued) % STAGES;
-      __nv_bfloat16* stage = kv + s_next * STAGE_ELEMS;
+      __nv_bfloat16* stage = kv + issued * STAGE_ELEMS;
       if constexpr (TMA) {
-        if (warp == 0) tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin + issued, hi_key, stage, &full[s_next], lane);
+        if (warp == 0) tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin + issued, hi_key, stage, &full[issued], lane);
       } else {
         load_kv_tile<D>(p, table, kvh, (tile_begin + issued) * BLOCK_N, lo_key, hi_key, stage, stage + BLOCK_N * D);
         cp_async_commit();
@@ -432,10 +336,8 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   // q and this step's keys and values are written and visible after the wait.  With late_wait the
   // kernel before this one is the prompt portions' attention, which is independent of this one and
   // whose every CTA had waited for them before this grid could start: the wait moves to the end.
-  if (done == 0) {
-    if (!p.late_wait) tl::pdl_wait();
-    tl::pdl_launch_dependents();  // the next kernel may start its own prologue
-  }
+  if (!p.late_wait) tl::pdl_wait();
+  tl::pdl_launch_dependents();  // the next kernel may start its own prologue
 
   // ---- Q rows into shared memory (zero for rows past the tile's end)
   for (int i = threadIdx.x; i < BLOCK_M * (D / 8); i += THREADS) {
@@ -449,8 +351,7 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   cp_async_commit();
   if (issued == 0 && num_tiles > 0) {
     if constexpr (TMA) {
-      const int s_next = done % STAGES;
-      if (warp == 0) tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin, hi_key, kv + s_next * STAGE_ELEMS, &full[s_next], lane);
+      if (warp == 0) tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin, hi_key, kv, &full[0], lane);
     } else {
       load_kv_tile<D>(p, table, kvh, tile_begin * BLOCK_N, lo_key, hi_key, kv, kv + BLOCK_N * D);
     }
@@ -497,13 +398,13 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   auto process_tile = [&](const int tile, auto edge_tag) {
     constexpr bool EDGE = decltype(edge_tag)::value;
     const int index = tile - tile_begin;
-    const int stage = (done + index) % STAGES;
+    const int stage = index % STAGES;
     __nv_bfloat16* ks_tile = kv + stage * STAGE_ELEMS;
     __nv_bfloat16* vs_tile = ks_tile + BLOCK_N * D;
     if constexpr (TMA) {
       // keep STAGES tiles requested: the stage of tile index - 1 is free since the barrier that ended it
       while (issued < min(num_tiles, index + STAGES)) {
-        const int s_next = (done + issued) % STAGES;
+        const int s_next = issued % STAGES;
         if (warp == 0)
           tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin + issued, hi_key, kv + s_next * STAGE_ELEMS, &full[s_next], lane);
         ++issued;
@@ -514,7 +415,7 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
       ++issued;
     }
     if constexpr (TMA) {
-      tc::mbar_wait(&full[stage], ((done + index) / STAGES) & 1, abort_flag, &g_error_word, 1);  // this tile is here
+      tc::mbar_wait(&full[stage], (index / STAGES) & 1, abort_flag, &g_error_word, 1);  // this tile is here
       // Whole pages were copied: value rows of keys outside [lo_key, hi_key] hold whatever the page
       // held before (another request's values, page 0).  Their weights are exactly 0, but 0 x NaN
       // is NaN, so the warp clears those of its own 16 rows before it multiplies.
@@ -675,11 +576,10 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
       }
       const int row = row_start + r;
       const int token = tok0 + row / g, head = kvh * g + row % g;
-      if (WALK ? my_splits > 1 : p.splits > 1) {
-        // key splits serve tiles of ONE token: the partial sums are indexed by (tile, head), WALK: by the CTA's entry
+      if (p.splits > 1) {
+        // key splits serve tiles of ONE token: the partial sums are indexed by (tile, head)
         if (row >= g) continue;
-        const size_t item = WALK ? ((size_t)blockIdx.x * 2 + (split == 0)) * g + r
-                                 : ((size_t)blockIdx.x * p.nh + head) * p.splits + split;
+        const size_t item = ((size_t)blockIdx.x * p.nh + head) * p.splits + split;
         p.part_acc[item * D + c] = acc;
         if (c == 0) {
           p.part_ml[item * 2] = m_all;
@@ -693,12 +593,12 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
             __float2bfloat16_rn(acc / with_sink<EXTRAS>(p, head, l, m_all) * gate_of<EXTRAS>(p, token, head, D, c));
       }
     }
-    if (WALK ? my_splits > 1 : p.splits > 1 && p.arrivals != nullptr) {
+    if (p.splits > 1 && p.arrivals) {
       // The split that writes last merges all of them: no second kernel.  The last CTA reads the
       // others' partial results from the L2.
       __shared__ int last_to_arrive;
       __syncthreads();  // every thread's partial results are written ...
-      int* counter = p.arrivals + (size_t)item_tile * p.nkv + kvh;
+      int* counter = p.arrivals + (size_t)blockIdx.x * p.nkv + kvh;
       if (threadIdx.x == 0) {
         int ticket;  // ... and released to the GPU by the arrival itself; the last one acquires the others'
         asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
@@ -712,9 +612,8 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
         for (int i = threadIdx.x; i < g * (D / 4); i += THREADS) {
           const int r = i / (D / 4), c = (i % (D / 4)) * 4;
           const size_t item = ((size_t)blockIdx.x * p.nh + kvh * g + r) * p.splits;
-          const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
-          const float4* src = reinterpret_cast<const float4*>(p.part_acc) + c / 4;
-          auto entry = [&](int j) { return WALK ? ((size_t)(first_cta + j) * 2 + (j == 0)) * g + r : item + j; };
+          const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + item;
+          const float4* src = reinterpret_cast<const float4*>(p.part_acc + item * D + c);
           float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
           float m_ref = -INFINITY, l = 0.f;
           for (int sp = 0; sp < my_splits; sp += 16) {
@@ -723,8 +622,8 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               const bool used = sp + j < my_splits;
-              w[j] = used ? __ldcg(ml + entry(sp + j)) : make_float2(-INFINITY, 0.f);
-              v[j] = used ? __ldcg(src + entry(sp + j) * (D / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              w[j] = used ? __ldcg(ml + sp + j) : make_float2(-INFINITY, 0.f);
+              v[j] = used ? __ldcg(src + (size_t)(sp + j) * (D / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             float m_new = m_ref;
 #pragma unroll
@@ -787,14 +686,6 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
       }
     }
   }
-  if constexpr (WALK) {
-    done += num_tiles;
-    if (walked < walk_end) {  // the stages take key tiles again
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-    }
-  }
-  } while (WALK && walked < walk_end);
   // this grid is complete only when the one before it is: the next kernel waits for this one alone
   if (p.late_wait) tl::pdl_wait();
 }
@@ -900,42 +791,29 @@ bool cached_map(CUtensorMap* out, const void* base, uint64_t rows, uint32_t cols
   return true;
 }
 
-int sm_count() {
-  static int sms = 0;
-  if (sms <= 0) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  return sms;
-}
-int walk_ctas() { return 3 * sm_count(); }  // as many as are resident
-
-template <int D, bool ROWS16, bool TMA, int STAGES, bool EXTRAS, bool WALK = false>
+template <int D, bool ROWS16, bool TMA, int STAGES, bool EXTRAS>
 int launch(const CUtensorMap& map_kv, const Params& p, int tiles, cudaStream_t stream) {
   constexpr int BLOCK_M = ROWS16 ? 16 : 64;
   // 16-row tiles: STAGES key/value stages and Q behind them; 64-row tiles: two stages, Q inside the second.
   // TMA: room to start the stages on a 1024-byte boundary, the barriers and the abort word
-  constexpr int SMEM = ((ROWS16 ? STAGES : 2) * 2 * BLOCK_N * D + (ROWS16 ? BLOCK_M * D : 0)) * 2 + (TMA ? 1024 + 64 : 0) +
-                       (WALK ? WALK_MAX * 12 : 0);
+  constexpr int SMEM = ((ROWS16 ? STAGES : 2) * 2 * BLOCK_N * D + (ROWS16 ? BLOCK_M * D : 0)) * 2 + (TMA ? 1024 + 64 : 0);
   static_assert(BLOCK_M * D <= 2 * BLOCK_N * D, "the Q rows fit one stage");
   static_assert(!ROWS16 || WARPS * 16 * (D + 2) * 4 <= 2 * 2 * BLOCK_N * D * 2, "merge buffer fits the stages");
   static_assert((STAGES == 2 ? 3 : 2) * (SMEM + 1024) <= 227 * 1024, "three CTAs an SM with two stages, two with three");
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(attention_mma_kernel<D, ROWS16, TMA, STAGES, EXTRAS, WALK>,
+    cudaError_t err = cudaFuncSetAttribute(attention_mma_kernel<D, ROWS16, TMA, STAGES, EXTRAS>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
-  const dim3 grid = WALK ? dim3(walk_ctas()) : dim3(tiles, p.nkv, p.splits);
+  dim3 grid(tiles, p.nkv, p.splits);
   // Decode steps of up to 32 requests are launched overlapped with the preceding kernel:
   // the CTAs request their old key/value tiles while q is still being written.  Larger
   // grids are launched WITHOUT overlap: CTAs that start while the small kernel before them
   // still occupies the SMs are placed unevenly, and a bandwidth-bound grid's time is set by
   // its most loaded SM (measured: batch 64 decode lost 9% with an overlapped launch).
-  tl::launch_kernel_opt(ROWS16 && (WALK || tiles <= p.overlap_max_tiles || p.late_wait), attention_mma_kernel<D, ROWS16, TMA, STAGES, EXTRAS, WALK>, grid, THREADS,
+  tl::launch_kernel_opt(ROWS16 && (tiles <= p.overlap_max_tiles || p.late_wait), attention_mma_kernel<D, ROWS16, TMA, STAGES, EXTRAS>, grid, THREADS,
                         SMEM, stream, map_kv, p);
   return TL_LAUNCH_CHECK();
 }
@@ -969,14 +847,20 @@ int launch_for(const Params& p, long long num_pages, int tiles, bool rows16, cud
   const bool tma = decode_tma_enabled() && num_pages > 0 && p.page_size >= 8 && p.page_size % 8 == 0 &&
                    BLOCK_N % p.page_size == 0 &&
                    cached_map(&map_kv, p.pages, (uint64_t)num_pages * 2 * p.nkv * p.page_size, D, (uint32_t)p.page_size);
-  if (p.splits == 0) return tma ? launch<D, true, true, 2, EXTRAS, true>(map_kv, p, tiles, stream) : TL_ERR_UNSUPPORTED;
   if (!tma) return launch<D, true, false, 2, EXTRAS>(map_kv, p, tiles, stream);
   // Without key splits (large batches) every CTA walks its request's whole context, and a third
   // stage keeps more of it requested (batch 128 at 2,048 tokens: 7.15 -> 6.68 ms a decode step;
   // batch 64: equal).  With splits the grid is sized for three CTAs an SM, which three stages do
   // not leave room for (batch 8 to 32: 5-14 % slower).
   // A grid of at most two CTAs an SM (batch 1 and 2) has the room as well: batch 1 -0.8 %.
-  const bool roomy = p.splits == 1 || (long long)tiles * p.nkv * p.splits <= 2ll * sm_count();
+  static int sms = 0;
+  if (sms <= 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
+      sms = 148;
+  }
+  const bool roomy = p.splits == 1 || (long long)tiles * p.nkv * p.splits <= 2ll * sms;
   if (decode_stages() == 3 || (decode_stages() == 0 && roomy)) return launch<D, true, true, 3, EXTRAS>(map_kv, p, tiles, stream);
   return launch<D, true, true, 2, EXTRAS>(map_kv, p, tiles, stream);
 }
@@ -989,7 +873,6 @@ extern "C" {
 
 // Bytes of float32 workspace for ``splits`` key splits of ``tiles`` decode tiles.
 long long tl_attention_mma_workspace(int tiles, int nh, int d, int splits) {
-  if (splits == 0) return (long long)walk_ctas() * 2 * 16 * (d + 2) * 4;
   return splits > 1 ? (long long)tiles * nh * splits * (d + 2) * 4 : 0;
 }
 
@@ -1006,8 +889,7 @@ int tl_attention_mma_error() {
 // With splits > 1 every tile is a request that brings ONE token (tile_row null, at most 16
 // query heads a KV head); the workspace holds tiles * nh * splits * (d + 2) floats, and only
 // the output rows of those tokens are written.  ``splits`` is what the grid provides; a request
-// uses as many of them as its length warrants; 0: the CTAs of a one-wave grid share all requests' key tiles evenly (TMA page sizes,
-// at most 384 requests, ``arrivals`` needed).  ``arrivals``: tiles * nkv ints, zero before the
+// uses as many of them as its length warrants.  ``arrivals``: tiles * nkv ints, zero before the
 // call and zero again after it: the split that finishes last merges (one kernel); null: a second
 // kernel merges.
 // late_wait != 0 (16-row tiles only): the kernel launched just before on this stream is the prompt
@@ -1029,9 +911,8 @@ int tl_attention_mma_ex(const void* q, long long q_stride, const void* pages, lo
   if (tiles <= 0 || tokens <= 0) return 0;
   if ((d != 64 && d != 128) || nkv <= 0 || nh % nkv || page_size <= 0 || q_stride % 8 || out_stride % 4)
     return TL_ERR_UNSUPPORTED;
-  if (splits < 0 || (!rows16 && splits != 1) || nkv > 65535 || splits > 64) return TL_ERR_UNSUPPORTED;
-  if (splits != 1 && (tile_row || nh / nkv > 16)) return TL_ERR_UNSUPPORTED;
-  if (splits == 0 && (tiles > WALK_MAX || !arrivals)) return TL_ERR_UNSUPPORTED;
+  if (splits < 1 || (!rows16 && splits != 1) || nkv > 65535 || splits > 64) return TL_ERR_UNSUPPORTED;
+  if (splits > 1 && (tile_row || nh / nkv > 16)) return TL_ERR_UNSUPPORTED;
   if (tl_attention_mma_workspace(tiles, nh, d, splits) > workspace_bytes) return TL_ERR_UNSUPPORTED;
   Params p;
   p.q = (const __nv_bfloat16*)q;
@@ -1046,9 +927,8 @@ int tl_attention_mma_ex(const void* q, long long q_stride, const void* pages, lo
   p.out = (__nv_bfloat16*)out;
   p.out_stride = out_stride;
   p.part_acc = (float*)workspace;
-  p.part_ml = p.part_acc + (splits == 0 ? (size_t)walk_ctas() * 2 * 16 * d : (size_t)tiles * nh * splits * d);
-  p.arrivals = splits != 1 ? arrivals : nullptr;
-  p.tiles = tiles;
+  p.part_ml = p.part_acc + (size_t)tiles * nh * splits * d;
+  p.arrivals = splits > 1 ? arrivals : nullptr;
   p.nh = nh;
   p.nkv = nkv;
   p.page_size = page_size;

@@ -8,7 +8,6 @@ a kernel refuses, or a missing library is an error here.
 from __future__ import annotations
 
 import ctypes
-import functools
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
@@ -1512,12 +1511,6 @@ def _arrivals(device, count: int) -> torch.Tensor:
 
 # TORCHLET_B200_DECODE_MERGE=kernel: a second kernel merges the key splits (for measurements)
 _merge_in_kernel = os.environ.get("TORCHLET_B200_DECODE_MERGE", "") != "kernel"
-_decode_tma = os.environ.get("TORCHLET_B200_DECODE_TMA", "1") not in ("0", "")  # as csrc/attention_mma.cu reads it
-
-
-@functools.lru_cache(maxsize=None)
-def _sm_count(index: int) -> int:
-    return torch.cuda.get_device_properties(index).multi_processor_count
 
 
 def attention_mma(qkv, pages, block_table, req_indptr, kv_before, tile_req, tile_row, tiles, out, tokens, nh, nkv,
@@ -1527,7 +1520,7 @@ def attention_mma(qkv, pages, block_table, req_indptr, kv_before, tile_req, tile
     tile i is request i from its first packed row.  With ``splits`` > 1 every tile is a request
     that brings one token; only those tokens' rows of ``out`` are written.  ``splits`` is the
     number of CTAs the grid holds for a request's keys; the kernel uses as many as the request's
-    own length warrants (0: the CTAs of one wave share all requests' key tiles evenly, ``decode_walk_supported``).  ``late_wait`` (16-row tiles): the launch just before this one on the
+    own length warrants.  ``late_wait`` (16-row tiles): the launch just before this one on the
     stream was ``attention_tc`` for the other requests of the same step; this grid starts beside
     it and waits for it at its end instead of at its start.  ``softcap``: scores become
     softcap * tanh(score / softcap); ``sink``: one is added to the softmax's denominator (True), or
@@ -1540,8 +1533,6 @@ def attention_mma(qkv, pages, block_table, req_indptr, kv_before, tile_req, tile
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
     # key splits: float32 partial results of every (decode tile, head, split); the split that finishes last merges
     need = tiles * nh * splits * (d + 2) * 4 if splits > 1 else 0
-    if splits == 0:  # two entries of up to 16 rows for each of the three CTAs an SM
-        need = 3 * _sm_count(qkv.device.index) * 2 * 16 * (d + 2) * 4
     ws = _workspace(("attention", qkv.device), need) if need else None
     # up to 16 splits the last split to finish merges them inside the kernel (one round of loads;
     # measured -1 % of a decode step at batch 8 to 32); more are merged by a second kernel, whose
@@ -1556,13 +1547,6 @@ def attention_mma(qkv, pages, block_table, req_indptr, kv_before, tile_req, tile
         float(softcap or 0.0), *_sink(sink, nh), _ptr(gate), gate.stride(0) if gate is not None else 0,
         _ptr(prior_ml), _ptr(prior_acc), _stream())
     _check(code, "attention_mma", 2 if splits > 1 and arrivals is None else 1)
-
-
-def decode_walk_supported(requests: int, page_size: int) -> bool:
-    """Whether ``attention_mma`` takes ``splits`` 0: pages that its TMA boxes take, the merge inside the kernel, a bounded number
-    of requests."""
-    return (_merge_in_kernel and _decode_tma and requests <= 384 and page_size >= 8 and page_size % 8 == 0
-            and 64 % page_size == 0)
 
 
 def _prior(prior, tokens: int, nh: int, d: int):

@@ -145,10 +145,7 @@ def forward(mixer, ctx, qkv, cache, out, gate=None, prior=None) -> bool:
             softcap=softcap, sink=sink, gate=gate, prior=prior)
     if plan["decode"] is not None:
         tile_req, count = plan["decode"]
-        if count * nkv > _sm_count(qkv.device.index) and ops.decode_walk_supported(count, cache.page_size):
-            splits = 0  # more (request, KV head) pairs than SMs: one wave shares all their key tiles (see the kernel)
-        else:
-            splits = decode_splits(count, nkv, ctx.max_kv_len, qkv.device)
+        splits = decode_splits(count, nkv, ctx.max_kv_len, qkv.device)
         ops.attention_mma(qkv, cache.pages, cache.block_table, ctx.req_indptr, ctx.kv_before, tile_req, None,
                           count, rows16=True, splits=splits, late_wait=beside, **common)
     if merge_portions is not None:
