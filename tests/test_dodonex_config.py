@@ -131,3 +131,26 @@ def test_plain_rotation_and_group_norm():
     assert abs(r[0, 0] - (1 * math.cos(a0) - 3 * math.sin(a0))) < 1e-12
     assert abs(r[0, 3] - (4 * math.cos(a1) + 2 * math.sin(a1))) < 1e-12
     assert torch.allclose(plain.rotate_half_pairs(v, torch.tensor([0]), 100.0, 4), v)
+
+
+@pytest.mark.parametrize("window", [None, 300])
+def test_row_tiles_of_the_latent_attention_start_with_those_that_see_the_most_keys(window):
+    """Single tokens behind long contexts and portions behind cached prefixes beside a fresh portion: the kernel's tiles are
+    handed out in descending numbers of visible keys, each once."""
+    from types import SimpleNamespace
+
+    import numpy as np
+
+    from torchlet_b200.parts.latent_attention import ROWS, row_tiles
+
+    heads, before, new = 16, np.array([4000, 0, 2500, 90, 0, 7]), [1, 70, 9, 1, 200, 33]
+    indptr = np.concatenate([[0], np.cumsum(new)])
+    ctx = SimpleNamespace(plans={}, decode_only=False, num_requests=len(new), req_indptr_host=indptr, kv_before_host=before,
+                          upload=torch.from_numpy)
+    req, row, count, splits = row_tiles(ctx, heads, window)
+    assert splits == 1 and count == len(req) == len(row)
+    pairs = list(zip(req.tolist(), row.tolist()))
+    assert sorted(pairs) == [(r, start) for r, n in enumerate(new) for start in range(0, n * heads, ROWS)]
+    seen = [min(before[r] + start // heads + 1, window or 10 ** 9) for r, start in pairs]
+    assert seen == sorted(seen, reverse=True)
+    assert pairs[0][0] == (0 if window is None else min(r for r, n in enumerate(new) if before[r] + n >= 300))

@@ -70,10 +70,13 @@ def row_tiles(ctx, heads: int, window=None):
                 for row in range(0, rows, ROWS):
                     tile_req.append(r)
                     tile_row.append(row)
-            # the later tiles of a portion see more keys and come first: the last CTAs to start are the short ones
+            # tiles that see the most keys first, as in attention_bf16._plan: the last CTAs to start are the short ones
             # (a 2,048-token prompt at 16 heads: 583 us against 712)
             req, row = np.asarray(tile_req, dtype=np.int32), np.asarray(tile_row, dtype=np.int32)
-            order = np.argsort(-row, kind="stable")
+            keys_seen = ctx.kv_before_host[req] + row // heads + 1
+            if (window or 0) > 0:
+                keys_seen = np.minimum(keys_seen, window)
+            order = np.argsort(-keys_seen, kind="stable")
             both = ctx.upload(np.concatenate([req[order], row[order]]))
             plan = (both[:len(tile_req)], both[len(tile_req):], len(tile_req), 1)
         ctx.plans[key] = plan
