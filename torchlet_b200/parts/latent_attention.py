@@ -73,7 +73,9 @@ def row_tiles(ctx, heads: int, window=None):
             # tiles that see the most keys first, as in attention_bf16._plan: the last CTAs to start are the short ones
             # (a 2,048-token prompt at 16 heads: 583 us against 712)
             req, row = np.asarray(tile_req, dtype=np.int32), np.asarray(tile_row, dtype=np.int32)
-            keys_seen = ctx.kv_before_host[req] + row // heads + 1
+            keys_seen = row // heads + 1
+            if ctx.num_requests > 1:
+                keys_seen = keys_seen + ctx.kv_before_host[req]
             if (window or 0) > 0:
                 keys_seen = np.minimum(keys_seen, window)
             order = np.argsort(-keys_seen, kind="stable")
