@@ -824,3 +824,24 @@ def test_finish_accum_norm_adds_the_splits_in_order(hidden, splits):
             x = want.double()
             normed = x / torch.sqrt(x.pow(2).mean(-1, keepdim=True) + eps) * weight.double()
             assert ((out.double() - normed).abs() <= 2.0 ** -8 * normed.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("hidden, splits", [(4, 2), (896, 19), (1020, 7), (1024, 1), (1028, 8), (2048, 3), (2052, 9), (3584, 7), (4096, 16),
+                                            (4100, 5), (8192, 4)])
+def test_finish_accum_norm_gives_the_same_bits_on_and_off_the_16_byte_boundaries(hidden, splits):
+    """The squares of a row are added in one order, whichever kernel takes it: rows on 16-byte boundaries and the same rows four
+    bytes beside them are normed to the same bits (600 rows: a root that is one bit off turns some bfloat16 roundings)."""
+    ops = _ops()
+    T = 600
+    made = [randn(*shape, seed=i) for i, shape in enumerate(((splits, T, hidden), (hidden,), (T, hidden), (hidden,)))]
+
+    def run(part, bias, acc, weight):
+        out = torch.empty(T, hidden, device=DEV, dtype=torch.bfloat16)
+        ops.finish_accum_norm(part, splits, bias, acc, weight, 1e-6, out)
+        return acc, out
+
+    def beside(t):
+        return torch.empty(t.numel() + 1, device=DEV)[1:].view(t.shape).copy_(t)
+
+    for a, b in zip(run(*(t.clone() for t in made)), run(*map(beside, made))):
+        assert torch.equal(a, b)

@@ -79,17 +79,19 @@ __global__ void finish_qkv_rope_kernel(const float* __restrict__ partial, int sp
 }
 
 // One block per token row, rows of a multiple of 4 on 16-byte boundaries: a thread owns PER groups of four columns and asks for
-// AHEAD splits of them before it adds the first, so the kernel is bound by one or two trips to the L2 and the row's sum.  Two
-// splits a trip took 19 splits (896 columns, K 4864) ten trips: one row 3.6 us, now 2.9; 48 rows of 14 splits 3.2 and 2.3, 64
-// rows of 3,584 columns and 7 splits 3.9 and 2.8.
-template <int NT, int PER>
+// AHEAD splits of them before it adds the first, so the kernel is bound by one or two trips to the L2 and the row's sum.  With two
+// splits a trip, 19 splits (896 columns, K 4864) took ten: one row 3.5 us, now 3.0; 48 rows of 14 splits 3.2 and 2.4, 64 rows of
+// 3,584 columns and 7 splits 4.0 and 3.1.  The squares are added as in finish_accum_norm_kernel, thread i those of columns i,
+// i + NT, ..., so that the kernel that takes a row shows in no bit: the row goes through shared memory once for that (8 rows of
+// 3,584: 0.2 us).
+template <int NT, int PER, int AHEAD>
 __global__ void __launch_bounds__(NT)
 finish_accum_norm_wide_kernel(const float* __restrict__ partial, int splits, const float* __restrict__ bias,
                               float* __restrict__ acc, const float* __restrict__ weight, __nv_bfloat16* __restrict__ out,
                               int tokens, int hidden, float eps) {
   tl::pdl_launch_dependents();  // the next kernel may start its prologue (it waits for us before it reads our output)
-  constexpr int AHEAD = NT == 1024 ? 4 : (PER == 1 ? 16 : 8);
   __shared__ float scratch[32];
+  __shared__ __align__(16) float whole[4 * NT * PER];  // the row
   const int t = blockIdx.x, groups = hidden / 4;
   tl::pdl_wait();               // everything before us in the stream is complete and visible
 
@@ -112,31 +114,42 @@ finish_accum_norm_wide_kernel(const float* __restrict__ partial, int splits, con
       for (int k = 0; k < PER; ++k)
         part[s][k] = __ldcg(src + (size_t)min(s0 + s, splits - 1) * plane + min((int)threadIdx.x + k * NT, groups - 1));
 #pragma unroll
-    for (int s = 0; s < AHEAD; ++s) {  // ascending splits; past the last one zeros are added
+    for (int s = 0; s < AHEAD; ++s) {  // ascending splits; past the last one -0 is added, which changes nothing
       const bool live = s0 + s < splits;
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
-        sum[k].x += live ? part[s][k].x : 0.f;
-        sum[k].y += live ? part[s][k].y : 0.f;
-        sum[k].z += live ? part[s][k].z : 0.f;
-        sum[k].w += live ? part[s][k].w : 0.f;
+        sum[k].x += live ? part[s][k].x : -0.f;
+        sum[k].y += live ? part[s][k].y : -0.f;
+        sum[k].z += live ? part[s][k].z : -0.f;
+        sum[k].w += live ? part[s][k].w : -0.f;
       }
     }
   }
-  float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
     const int j = threadIdx.x + k * NT;
-    if (j >= groups) continue;
-    v[k].x += sum[k].x;
-    v[k].y += sum[k].y;
-    v[k].z += sum[k].z;
-    v[k].w += sum[k].w;
-    row[j] = v[k];
-    ss = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, ss))));
+    if (j < groups) {
+      v[k].x += sum[k].x;
+      v[k].y += sum[k].y;
+      v[k].z += sum[k].z;
+      v[k].w += sum[k].w;
+      row[j] = v[k];
+    }
+    reinterpret_cast<float4*>(whole)[j] = v[k];  // (zeros past the row's end)
   }
   if (!out) return;
-  ss = block_sum<NT>(ss, scratch);
+  __syncthreads();
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4 * PER; ++k) {
+    const float x = whole[threadIdx.x + k * NT];
+    ss = fmaf(x, x, ss);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // (block_sum without its first barrier: scratch is untouched)
+  ss = warp_sum(ss);
+  if (lane == 0) scratch[warp] = ss;
+  __syncthreads();
+  ss = warp_sum(lane < NT / 32 ? scratch[lane] : 0.f);
   const float inv = rsqrtf(ss / (float)hidden + eps);
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
@@ -152,7 +165,7 @@ finish_accum_norm_wide_kernel(const float* __restrict__ partial, int splits, con
   }
 }
 
-// The same for any row.  PER = elements of the row each thread keeps in registers.
+// The same for any row.  PER = elements of the row each thread keeps in registers; NT follows from the width alone, here and above.
 template <int NT, int PER>
 __global__ void __launch_bounds__(NT)
 finish_accum_norm_kernel(const float* __restrict__ partial, int splits, const float* __restrict__ bias,
@@ -247,17 +260,24 @@ int tl_finish_accum_norm(const float* partial, int splits, const float* bias, fl
   const bool wide = hidden % 4 == 0 && ((reinterpret_cast<uintptr_t>(partial) | reinterpret_cast<uintptr_t>(bias) |
                                          reinterpret_cast<uintptr_t>(acc) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0 &&
                     (reinterpret_cast<uintptr_t>(out) & 7) == 0;
-#define TL_FINISH(NT, PER)                                                                                              \
-  tl::launch_kernel(finish_accum_norm_wide_kernel<NT, PER>, tokens, NT, 0, stream, partial, splits, bias, acc, weight, o, \
-                    tokens, hidden, eps)
-  if (wide && hidden <= 1024) TL_FINISH(256, 1);
-  else if (wide && hidden <= 2048) TL_FINISH(512, 1);
-  else if (wide && hidden <= 4096) TL_FINISH(512, 2);
-  else if (wide && hidden <= 8192) TL_FINISH(1024, 2);
-  else if (hidden <= 16384)
-    tl::launch_kernel(finish_accum_norm_kernel<1024, 16>, tokens, 1024, 0, stream, partial, splits, bias, acc, weight, o, tokens, hidden, eps);
-  else
-    return TL_ERR_UNSUPPORTED;
+#define TL_FINISH(KERNEL, NT) \
+  tl::launch_kernel(KERNEL, tokens, NT, 0, stream, partial, splits, bias, acc, weight, o, tokens, hidden, eps)
+// as many splits asked for at once as there are, up to MOST (registers); asking for 16 where there are 2 costs more than the sum
+// (one row of 896: 2.0 us against 1.4)
+#define TL_FINISH_WIDE(NT, PER, MOST)                                                                            \
+  if (splits <= 2) TL_FINISH((finish_accum_norm_wide_kernel<NT, PER, 2>), NT);                                   \
+  else if (splits <= 4 || MOST == 4) TL_FINISH((finish_accum_norm_wide_kernel<NT, PER, 4>), NT);                 \
+  else if (splits <= 8 || MOST == 8) TL_FINISH((finish_accum_norm_wide_kernel<NT, PER, MOST < 8 ? MOST : 8>), NT); \
+  else TL_FINISH((finish_accum_norm_wide_kernel<NT, PER, MOST>), NT)
+  if (wide && hidden <= 1024) { TL_FINISH_WIDE(256, 1, 16); }
+  else if (wide && hidden <= 2048) { TL_FINISH_WIDE(512, 1, 16); }
+  else if (wide && hidden <= 4096) { TL_FINISH_WIDE(512, 2, 8); }
+  else if (wide && hidden <= 8192) { TL_FINISH_WIDE(1024, 2, 4); }
+  else if (hidden <= 1024) TL_FINISH((finish_accum_norm_kernel<256, 4>), 256);
+  else if (hidden <= 4096) TL_FINISH((finish_accum_norm_kernel<512, 8>), 512);
+  else if (hidden <= 16384) TL_FINISH((finish_accum_norm_kernel<1024, 16>), 1024);
+  else return TL_ERR_UNSUPPORTED;
+#undef TL_FINISH_WIDE
 #undef TL_FINISH
   return TL_LAUNCH_CHECK();
 }
