@@ -11,11 +11,11 @@
 // of the NCW warps of a row block meet in shared memory, P goes to shared memory in bfloat16, and
 // for O every warp reads all of P and the value columns [cw DVW, (cw + 1) DVW) that it accumulates
 // (DVW <= 128: 64 float registers a thread).  NCW = 1, 2, 4 for dv up to 128, 256, 512.
-// With room for two tiles of keys (all sizes up to dk 576) the next one is copied while this one is multiplied: P is swizzled
-// instead of padded and the row maxima and sums lie in the 16 padding bytes of the query and key rows, which makes the 227 KB
-// suffice at dk 576.  A warp copies whole rows and looks their pages up a tile ahead.  2,048 tokens at 16 heads, dk 576: 435 us,
-// with one tile at a time 583 (712 with the tiles of few keys first).  What is left is the shared-memory reads of the fragments
-// (885 KB a tile: 3.7 of 7.6 us).
+// A warp copies whole rows of a key tile, 32 pieces of 16 bytes at a time, and looks its rows' pages up a tile ahead.  2,048
+// tokens at 16 heads, dk 576: 420 us, 580 with pages looked up and divisions made for every piece (and 710 with the tiles of few
+// keys first); 4 heads, dk 112: 116 and 170.  A second stage for the next key tile takes the room of a second block: equal at dk
+// 288 and up, 4 to 14 % slower below.  What is left is the shared-memory reads of the fragments (885 KB a tile at dk 576: 3.7 of
+// 7.4 us).
 //
 // Rows of keys outside what the tile's rows see (past the last row's own, before the first row's first under a window
 // or a chunked mask) are zero-filled (0 x stale NaN would be NaN).
@@ -42,8 +42,6 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool valid)
   const int bytes = valid ? 16 : 0;  // 0: the 16 bytes are zero-filled
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 __device__ __forceinline__ void copies_done() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
 }
@@ -85,7 +83,7 @@ __device__ __forceinline__ __nv_bfloat16* p_at(__nv_bfloat16* Ps, int row, int c
   return Ps + row * KEYS + ((((col >> 3) ^ row) & 7) << 3) + (col & 7);
 }
 
-template <int NCW, int STAGES>
+template <int NCW>
 __global__ void __launch_bounds__(128 * NCW)
 latent_attention_mma_kernel(const Args a) {
   tl::pdl_wait();
@@ -95,11 +93,11 @@ latent_attention_mma_kernel(const Args a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int stride = a.dk + PAD;
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-  __nv_bfloat16* stages = Qs + (size_t)ROWS * stride;
-  __nv_bfloat16* Ps = stages + (size_t)STAGES * KEYS * stride;
-  // the maxima and sums of the NCW <= 4 warps of a row: four floats in the padding of the row of Qs and of the first stage
+  __nv_bfloat16* Ks = Qs + (size_t)ROWS * stride;
+  __nv_bfloat16* Ps = Ks + (size_t)KEYS * stride;
+  // the maxima and sums of the NCW <= 4 warps of a row: four floats in the padding of the rows of Qs and Ks
   auto red_max = [&](int c, int r) -> float& { return reinterpret_cast<float*>(Qs + (size_t)r * stride + a.dk)[c]; };
-  auto red_sum = [&](int c, int r) -> float& { return reinterpret_cast<float*>(stages + (size_t)r * stride + a.dk)[c]; };
+  auto red_sum = [&](int c, int r) -> float& { return reinterpret_cast<float*>(Ks + (size_t)r * stride + a.dk)[c]; };
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rw = warp & 3, cw = warp >> 2;
@@ -146,44 +144,41 @@ latent_attention_mma_kernel(const Args a) {
   const bool on_lo = r_lo < nrows, on_hi = r_hi < nrows;
   const bool warp_has_rows = rw * 16 < nrows;  // a tile of few rows (single tokens, few heads): the other warps only load
 
-  // A warp copies RW rows of a key tile; lane i < RW knows the page of row i (-1: the key is not seen, zeros)
+  // A warp copies RW rows of a key tile, 32 pieces of 16 bytes at a time whatever the row's length (a row at a time left 22 of
+  // 32 lanes idle at dk 80); lane i < RW knows where row i lies in the pages (-1: the key is not seen, zeros)
   constexpr int RW = KEYS / (4 * NCW);
-  auto page_of = [&](int kt) {
+  auto row_of = [&](int kt) -> long long {
     const int key = kt * KEYS + warp * RW + lane;
     if (lane >= RW || kt >= tile_hi || key < kv_lo || key >= kv_end) return -1;
     int page = 0;
     if (TL_DEBUG_OK(key / a.page_size < a.table_width, TL_DEBUG_POSITION, key)) page = table[key / a.page_size];
     if (!TL_DEBUG_OK(page >= 0 && page < a.num_pages, TL_DEBUG_PAGE, page)) page = 0;
-    return page;
+    return (long long)page * a.page_size + key % a.page_size;
   };
-  auto copy_tile = [&](int kt, int my_page) {
-    __nv_bfloat16* dst = stages + (size_t)((kt - tile_lo) % STAGES) * KEYS * stride + (size_t)warp * RW * stride;
-#pragma unroll
-    for (int i = 0; i < RW; ++i) {
-      const int page = __shfl_sync(0xffffffffu, my_page, i);
-      const int slot = (kt * KEYS + warp * RW + i) % a.page_size;
-      const __nv_bfloat16* src = a.pages + ((size_t)(page < 0 ? 0 : page) * a.page_size + (page < 0 ? 0 : slot)) * a.dk;
-      for (int c = lane; c < chunks; c += 32) copy16(dst + (size_t)i * stride + c * 8, src + c * 8, page >= 0);
+  const int first_row = lane / chunks, first_chunk = lane % chunks, more_rows = 32 / chunks, more_chunks = 32 % chunks;
+  auto copy_rows = [&](long long my_row) {
+    __nv_bfloat16* dst = Ks + (size_t)warp * RW * stride;
+    int r = first_row, c = first_chunk;
+#pragma unroll 4
+    for (int n = 0; n < RW * chunks; n += 32) {
+      const long long from = __shfl_sync(0xffffffffu, my_row, r & 31);
+      if (r < RW) copy16(dst + (size_t)r * stride + c * 8, a.pages + (from < 0 ? 0 : from) * a.dk + c * 8, from >= 0);
+      c += more_chunks;
+      r += more_rows;
+      if (c >= chunks) {
+        c -= chunks;
+        ++r;
+      }
     }
-    copies_commit();
   };
-  int next_page = page_of(tile_lo);
-  if (STAGES > 1 && tile_lo < tile_hi) {
-    copy_tile(tile_lo, next_page);
-    next_page = page_of(tile_lo + 1);
-  }
+  long long next_row = row_of(tile_lo);
 
   for (int kt = tile_lo; kt < tile_hi; ++kt) {
     const int key0 = kt * KEYS;
-    const __nv_bfloat16* Ks = stages + (size_t)((kt - tile_lo) % STAGES) * KEYS * stride;
-    __syncthreads();  // everyone is done with the tile before, with its stage and with Ps
-    if (STAGES == 1 || kt + 1 < tile_hi) {
-      copy_tile(kt + STAGES - 1, next_page);
-      next_page = page_of(kt + STAGES);
-      copies_wait<STAGES - 1>();
-    } else {
-      copies_wait<0>();
-    }
+    __syncthreads();  // everyone is done with Ks and Ps of the tile before
+    copy_rows(next_row);
+    next_row = row_of(kt + 1);
+    copies_done();
     __syncthreads();
 
     // S for rows of rw and keys [cw KW, (cw + 1) KW)
@@ -366,10 +361,7 @@ latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ 
   }
 }
 
-constexpr size_t SMEM_LIMIT = 227 * 1024;
-size_t smem_bytes(int dk, int stages) {
-  return (size_t)(ROWS + stages * KEYS) * (dk + PAD) * 2 + (size_t)ROWS * KEYS * 2;
-}
+size_t smem_bytes(int dk) { return (size_t)(ROWS + KEYS) * (dk + PAD) * 2 + (size_t)ROWS * KEYS * 2; }
 
 }  // namespace
 
@@ -414,20 +406,16 @@ int tl_latent_attention_mma(const void* q, const void* pages, const int* block_t
   a.scale = scale;
   a.window = window;
   const int ncw = dv <= 128 ? 1 : (dv <= 256 ? 2 : 4);
-  const int stages = smem_bytes(dk, 2) <= SMEM_LIMIT ? 2 : 1;
-  const size_t smem = smem_bytes(dk, stages);
+  const size_t smem = smem_bytes(dk);
   dim3 grid(tiles, splits);
   cudaError_t err;
-#define TL_LAUNCH_NCW(N, S)                                                                                      \
-  err = cudaFuncSetAttribute(latent_attention_mma_kernel<N, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+#define TL_LAUNCH_NCW(N)                                                                                         \
+  err = cudaFuncSetAttribute(latent_attention_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
   if (err != cudaSuccess) return (int)err;                                                                       \
-  tl::launch_kernel(latent_attention_mma_kernel<N, S>, grid, 128 * N, smem, stream, a)
-  if (ncw == 1 && stages == 2) { TL_LAUNCH_NCW(1, 2); }
-  else if (ncw == 2 && stages == 2) { TL_LAUNCH_NCW(2, 2); }
-  else if (ncw == 4 && stages == 2) { TL_LAUNCH_NCW(4, 2); }
-  else if (ncw == 1) { TL_LAUNCH_NCW(1, 1); }
-  else if (ncw == 2) { TL_LAUNCH_NCW(2, 1); }
-  else { TL_LAUNCH_NCW(4, 1); }
+  tl::launch_kernel(latent_attention_mma_kernel<N>, grid, 128 * N, smem, stream, a)
+  if (ncw == 1) { TL_LAUNCH_NCW(1); }
+  else if (ncw == 2) { TL_LAUNCH_NCW(2); }
+  else { TL_LAUNCH_NCW(4); }
 #undef TL_LAUNCH_NCW
   int code = TL_LAUNCH_CHECK();
   if (code || splits == 1) return code;
