@@ -845,3 +845,15 @@ def test_finish_accum_norm_gives_the_same_bits_on_and_off_the_16_byte_boundaries
 
     for a, b in zip(run(*(t.clone() for t in made)), run(*map(beside, made))):
         assert torch.equal(a, b)
+
+
+def test_bfloat16_products_of_any_size_add_in_ascending_order():
+    """2^24 and then ones: every one is lost in the chain of ascending k; any other order of the sum shows."""
+    ops = _ops()
+    M, N, K = 3, 5, 67  # (no multiple of 8: the any-size kernel)
+    x = torch.ones(M, K, device=DEV, dtype=torch.bfloat16)
+    w = torch.ones(N, K, device=DEV, dtype=torch.bfloat16)
+    w[:, 0] = 2.0 ** 24
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm_simt(x, w, out)
+    assert (out == 2.0 ** 24).all()

@@ -4,7 +4,9 @@
 // cores, no reduced-precision mode) and the any-size path for bfloat16 operands
 // that the tensor-core kernels refuse.
 //
-// Every kernel here adds in the SAME order, which depends on K alone, so a row's result does not depend on
+// bfloat16 operands: each output element is the sum over k in ascending order.
+//
+// float32: every kernel here adds in the SAME order, which depends on K alone, so a row's result does not depend on
 // which other rows are in the batch, nor on which kernel took it: K is cut into at most 16 pieces of
 // piece_length(K) entries (a multiple of 32); a piece is an ascending chain of fused multiply-adds that starts
 // at zero; four consecutive pieces are added in ascending order to a quarter, the quarters in ascending order to
@@ -23,11 +25,13 @@
 //       reads an operand and k for 64 products.  Where the tiles leave SMs idle, the four blocks of a cluster take a quarter
 //       of K each.  509 tokens, K x N: 896 x 9728 245 us (36 TFLOP/s), 4864 x 896 148 us, 896 x 896 35 us; 42 TFLOP/s on the
 //       largest products.
-//   gemm_simt_kernel        any type, stride and alignment (the other two copy 16 bytes at a time).
+//   gemm_simt_kernel        any type, stride and alignment (the other two copy 16 bytes at a time, float32 alone).
 //
 // Reference counterparts: nn.Linear in v10_triton_paged_gqa/layer/gqa.py:122-124,84
 // and model/qwen2_5.py:83-87; down_kernel / swiglu_kernel GEMMs in
 // v10_triton_paged_gqa/kernel/ffn_swiglu.py:5-164.
+#include <limits.h>
+
 #include "common.cuh"
 
 namespace {
@@ -46,34 +50,44 @@ gemm_simt_kernel(const T* __restrict__ x, const T* __restrict__ w, const float* 
   tl::pdl_wait();               // everything before us in the stream is complete and visible
   tl::pdl_launch_dependents();  // the next kernel may start its own prologue
 
+  constexpr bool PIECES = sizeof(T) == 4;
   __shared__ float xs[BK][BM + 1];
   __shared__ float ws[BK][BN + 1];
+  __shared__ float totals[PIECES ? TM * TN : 1][256];  // of the quarters so far, a column a thread
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int tx = tid % 16, ty = tid / 16;  // 16 x 16 threads, each TM x TN outputs
-  const int piece = piece_length(K);
-  float acc[TM][TN], quarter[TM][TN], total[TM][TN];
+  float acc[TM][TN], quarter[PIECES ? TM : 1][TN];
+  auto clear = [](auto& v) {
+    for (auto& row : v)
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = quarter[i][j] = total[i][j] = 0.f;
-
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // 64 rows x 16 k-values per operand, 4 per thread
+      for (int j = 0; j < TN; ++j) row[j] = 0.f;
+  };
+  clear(acc);
+  clear(quarter);
+  // 64 rows x 16 k-values per operand, 4 per thread; the next step's are requested before this one's are multiplied
+  T xr[4], wr[4];
+  auto request = [&](int k0) {  // (past an edge the last entry; it is dropped below)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int e = tid + i * 256;
-      const int r = e / BK, c = e % BK;
-      const int k = k0 + c;
-      float xv = 0.f, wv = 0.f;
-      if (k < K) {
-        if (m0 + r < M) xv = to_float(x[(size_t)(m0 + r) * ldx + k]);
-        if (n0 + r < N) wv = to_float(w[(size_t)(n0 + r) * ldw + k]);
-      }
-      xs[c][r] = xv;
-      ws[c][r] = wv;
+      const int e = tid + i * 256, r = e / BK, k = min(k0 + e % BK, K - 1);
+      xr[i] = x[(size_t)min(m0 + r, M - 1) * ldx + k];
+      wr[i] = w[(size_t)min(n0 + r, N - 1) * ldw + k];
+    }
+  };
+  const int piece_steps = PIECES ? piece_length(K) / BK : INT_MAX;
+  int steps_left = piece_steps, pieces = 0;
+  bool first_quarter = true;
+  request(0);
+  for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = tid + i * 256, r = e / BK, c = e % BK;
+      xs[c][r] = k0 + c < K && m0 + r < M ? to_float(xr[i]) : 0.f;
+      ws[c][r] = k0 + c < K && n0 + r < N ? to_float(wr[i]) : 0.f;
     }
     __syncthreads();
+    if (k0 + BK < K) request(k0 + BK);
 #pragma unroll
     for (int c = 0; c < BK; ++c) {
       float xa[TM], wb[TN];
@@ -87,21 +101,29 @@ gemm_simt_kernel(const T* __restrict__ x, const T* __restrict__ w, const float* 
         for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(xa[i], wb[j], acc[i][j]);
     }
     __syncthreads();
-    const int done = k0 + BK;
-    const bool last = done >= K;
-    if (last || done % piece == 0) {
-      const bool quarter_ends = last || done % (4 * piece) == 0;
+    if constexpr (PIECES) {
+      const bool last = k0 + BK >= K;
+      if (--steps_left == 0 || last) {
+        const bool quarter_ends = ++pieces == 4 || last;
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          quarter[i][j] += acc[i][j];
-          acc[i][j] = 0.f;
-          if (quarter_ends) {
-            total[i][j] += quarter[i][j];
-            quarter[i][j] = 0.f;
+          for (int j = 0; j < TN; ++j) {
+            quarter[i][j] += acc[i][j];
+            acc[i][j] = 0.f;
+            if (quarter_ends) {
+              const float sum = first_quarter ? quarter[i][j] : totals[i * TN + j][tid] + quarter[i][j];
+              totals[i * TN + j][tid] = sum;
+              quarter[i][j] = 0.f;
+              if (last) acc[i][j] = sum;
+            }
           }
+        steps_left = piece_steps;
+        if (quarter_ends) {
+          first_quarter = false;
+          pieces = 0;
         }
+      }
     }
   }
 #pragma unroll
@@ -112,7 +134,7 @@ gemm_simt_kernel(const T* __restrict__ x, const T* __restrict__ w, const float* 
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tx * TN + j;
       if (n >= N) continue;
-      float v = total[i][j];
+      float v = acc[i][j];
       if (bias) v += bias[n];
       OutT* o = out + (size_t)m * ldo + n;
       if (ACCUM)
