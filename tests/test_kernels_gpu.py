@@ -85,7 +85,10 @@ def test_gemm_simt(dtype, out_dtype, M, N, K):
         assert torch.equal(alone[0], out[M - 1])
 
 
-@pytest.mark.parametrize("N, K", [(1, 4), (33, 36), (130, 512), (2048, 516), (9504, 68), (2080, 2052)])
+@pytest.mark.parametrize("N, K", [(1, 4), (33, 36), (130, 512), (2048, 516), (9504, 68), (2080, 2052),
+                                  # several quarters and a partial last piece in the kernels without clusters, then the
+                                  # sizes on both sides of the line between those and clusters
+                                  (9504, 900), (19008, 548), (2048, 384), (2049, 388), (3552, 700), (3556, 388)])
 def test_gemm_float32_kernels_add_in_one_order(N, K):
     """Stream, tile and any-alignment kernels: the same bits for a row, whatever rows stand beside it; in the error bound of
     their order (a piece of at most K / 16 + 32 terms, 4 pieces, 4 quarters, the bias: gamma_n with n that many roundings)."""

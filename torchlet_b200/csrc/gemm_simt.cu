@@ -528,35 +528,55 @@ int launch_clusters(Kernel kernel, bool& configured, dim3 grid, int threads, int
   return TL_LAUNCH_CHECK();
 }
 
-constexpr int SMS = 148;
-// Between 33 and 128 rows: up to this many columns the stream kernel, 32 rows a block, has the shorter chains (64 rows, K x N
-// 4864 x 896: 35 against 69 us; 896 x 1152: 11 against 17); on wider products the tiles read the weights less often (64 rows,
-// 896 x 9728: 52 us against two passes of 26).
-constexpr int NARROW = 2048;
+int sm_count() {
+  static int sms = 0;
+  if (sms <= 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
+      sms = 148;
+  }
+  return sms;
+}
+
+// The kernel, its tile and its split follow from the sizes; the bits depend on none of them.  Every form was measured at K 4 to
+// 4096, N 32 to 12288 and M 1 to 2048; the lines:
+// - Four blocks a cluster where all of them are resident at once, or K is long enough to pay for a second wave, and not at all
+//   where most quarters of K are empty (17 rows, K 4 x N 4096: 9.1 us as clusters, 2.4 in one block; 509 rows, 64 x 4096: 46 and 11;
+//   2 rows, 512 x 4096: 6.0 and 3.6, 4096 x 4096: 18.6 and 22.5).
+// - 17 to 32 rows, and up to 128 of narrow products: the stream kernel, 32 rows a block, has the shorter chains (64 rows, K x N
+//   4864 x 896: 35 against 69 us; 896 x 1152: 11 against 17); on wider products the tiles read the weights less often (64 rows,
+//   896 x 9728: 52 us against two passes of 26), on short K they start faster (17 rows, 32 x 2048: 2.8 us against 4.6).
+// - Small tiles for up to 128 rows, and for short K until they take two waves (509 rows, 256 x 2048: 13 us, 21 with large ones).
+constexpr int SHORT_K = 64, NARROW = 2048;
 
 template <int MT>
 int launch_stream(const float* x, const float* w, const float* bias, float* out, int accum, int M, int N, int K, int ldx,
                   int ldw, int ldo, cudaStream_t stream) {
   const int tiles = (N + 31) / 32, down = (M + MT - 1) / MT;
   static bool configured[2] = {false, false};
-  // a block that walks whole rows needs no exchange; where such blocks do not fill the SMs twice, four of them share the rows
-  if (tiles >= 2 * SMS)
-    return launch_clusters<1>(gemm_f32_stream_kernel<MT, 1>, configured[0], dim3(tiles, down), STREAM_WARPS * 32, STREAM_SMEM<MT>,
-                              stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
-  return launch_clusters<4>(gemm_f32_stream_kernel<MT, 4>, configured[1], dim3(4 * tiles, down), STREAM_WARPS * 32,
-                            STREAM_SMEM<MT>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
+  const bool together = 4ll * tiles * down <= 3 * sm_count();
+  if (K > SHORT_K && (together || (K >= (MT <= 16 ? 1024 : 512) && tiles < 2 * sm_count())))
+    return launch_clusters<4>(gemm_f32_stream_kernel<MT, 4>, configured[1], dim3(4 * tiles, down), STREAM_WARPS * 32,
+                              STREAM_SMEM<MT>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
+  return launch_clusters<1>(gemm_f32_stream_kernel<MT, 1>, configured[0], dim3(tiles, down), STREAM_WARPS * 32, STREAM_SMEM<MT>,
+                            stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
 }
+
+// Blocks of a tile size that are resident at once.
+template <int TILE_M, int TILE_N, int TC> int resident() { return sm_count() * ((TC == 8 ? 256 : 512) / TILE_THREADS<TILE_M, TILE_N, TC>); }
 
 template <int TILE_M, int TILE_N, int TC>
 int launch_tiles(const float* x, const float* w, const float* bias, float* out, int accum, int M, int N, int K, int ldx,
                  int ldw, int ldo, cudaStream_t stream) {
   const int across = (N + TILE_N - 1) / TILE_N, down = (M + TILE_M - 1) / TILE_M;
+  const long long blocks = (long long)across * down, room = resident<TILE_M, TILE_N, TC>();
   constexpr int NT = TILE_THREADS<TILE_M, TILE_N, TC>;
   static bool configured[2] = {false, false};
-  if ((long long)across * down >= SMS * ((TC == 8 ? 256 : 512) / NT))
-    return launch_clusters<1>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 1>, configured[0], dim3(across, down), NT,
+  if ((K > 160 && 4 * blocks <= room) || (K >= 512 && blocks < room))
+    return launch_clusters<4>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 4>, configured[1], dim3(4 * across, down), NT,
                               TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
-  return launch_clusters<4>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 4>, configured[1], dim3(4 * across, down), NT,
+  return launch_clusters<1>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 1>, configured[0], dim3(across, down), NT,
                             TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
 }
 
@@ -566,8 +586,11 @@ int launch_f32(const float* x, const float* w, const float* bias, float* out, in
   if (M <= 4) return launch_stream<4>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
   if (M <= 8) return launch_stream<8>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
   if (M <= 16) return launch_stream<16>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
-  if (M <= 32 || (M <= 128 && N <= NARROW)) return launch_stream<32>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
-  if (M <= 128) return launch_tiles<64, 64, 4>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
+  if (K > SHORT_K && (M <= 32 || (M <= 128 && N <= NARROW)))
+    return launch_stream<32>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
+  const long long small = (long long)((N + 63) / 64) * ((M + 63) / 64);
+  if (K <= 512 ? small < 2 * resident<64, 64, 4>() : M <= 128)
+    return launch_tiles<64, 64, 4>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
   return launch_tiles<128, 64, 8>(x, w, bias, out, accum, M, N, K, ldx, ldw, ldo, stream);
 }
 
