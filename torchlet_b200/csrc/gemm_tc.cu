@@ -82,7 +82,7 @@ struct Params {
   int stack_rows;
   // one product a head (persistent kernel): head h takes columns [h K, (h + 1) K) of the row operand, rows [h group_rows,
   // (h + 1) group_rows) of the column operand and writes (bf16) from column h head_out on; 0: not by heads
-  int heads = 0, head_out = 0;
+  int heads, head_out;
 };
 
 __device__ __forceinline__ float silu(float g) { return g / (1.f + __expf(-g)); }
@@ -100,8 +100,9 @@ __device__ __forceinline__ float gated(float g, float u, float limit, float alph
   return silu(g) * u;
 }
 
-// 32 accumulator values of output row m, columns n0 .. n0+31 (normal orientation).
-__device__ __forceinline__ void epilogue_chunk(const Params& p, int m, int n0, const float (&v)[32], int cols = 32) {
+// 32 accumulator values of output row m, columns n0 .. n0+31 (normal orientation).  ``bf16_shift``: a bf16 output row starts that
+// many columns on.
+__device__ __forceinline__ void epilogue_chunk(const Params& p, int m, int n0, const float (&v)[32], int cols = 32, int bf16_shift = 0) {
   const int N = p.cols;
   if (p.epilogue == EPI_SWIGLU_BF16) {
     // columns n0..n0+15 are gate j..j+15, n0+16..n0+31 the matching up values
@@ -157,7 +158,7 @@ __device__ __forceinline__ void epilogue_chunk(const Params& p, int m, int n0, c
     if (stores_bf16(p.epilogue)) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) r[j] = activated(p.epilogue, r[j]);
-      __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)m * p.ldo + n;
+      __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)m * p.ldo + bf16_shift + n;
       if (full && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
         uint32_t packed[4];
 #pragma unroll
@@ -428,8 +429,8 @@ gemm_tc_swapped_kernel(const __grid_constant__ CUtensorMap map_row, const __grid
 
 // The group of a tile of the persistent kernel (0 without a plan); negative: the tile is skipped.  Every
 // role of the CTA asks with the same arguments, so all of them skip the same tiles.
-__device__ __forceinline__ int tile_group(const Params& p, int tile) {
-  if (p.heads) return tile / (p.num_tiles / p.heads);
+template <bool HEADS> __device__ __forceinline__ int tile_group(const Params& p, int tile) {
+  if constexpr (HEADS) return tile / (p.num_tiles / p.heads);
   if (!p.plan) return 0;
   const int row_tile = tile / (p.num_tiles / p.row_tiles);
   return row_tile < p.plan[0] ? p.plan[1 + row_tile] : -1;
@@ -437,12 +438,12 @@ __device__ __forceinline__ int tile_group(const Params& p, int tile) {
 // Row and column tile of a tile index.  One group: row tiles fastest, so that the CTAs that run together share
 // weight tiles.  With a plan: column tiles fastest, so that the CTAs that run together work on the few row tiles
 // of one or two groups and need those groups' weights only.
-__device__ __forceinline__ void tile_coords(const Params& p, int tile, int* row_tile, int* col_tile) {
+template <bool HEADS> __device__ __forceinline__ void tile_coords(const Params& p, int tile, int* row_tile, int* col_tile) {
   if (p.plan) {
     const int col_tiles = p.num_tiles / p.row_tiles;
     *row_tile = tile / col_tiles;
     *col_tile = tile - *row_tile * col_tiles;
-  } else if (p.heads) {  // a head after the other
+  } else if constexpr (HEADS) {  // a head after the other
     const int within = tile % (p.num_tiles / p.heads);
     *row_tile = within % p.row_tiles;
     *col_tile = within / p.row_tiles;
@@ -458,6 +459,9 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int* row_
 // waves.  The accumulator is double-buffered in tensor memory (2 x 256 columns): while the
 // four epilogue warps drain tile i, the MMA thread already accumulates tile i + 1, and the
 // TMA producer never stops between tiles.
+// HEADS: one product a head (an instance of its own: the few operations it adds cost the smallest products 5 %, 4.8 -> 5.1 us for
+// 257 rows of 256 x 512).
+template <bool HEADS>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_row, const __grid_constant__ CUtensorMap map_col,
                           const Params p) {
@@ -505,12 +509,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_row, const __g
       int s = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) {
-        const int group = tile_group(p, tile);
+        const int group = tile_group<HEADS>(p, tile);
         if (group < 0) continue;
         int row_tile, col_tile;
-        tile_coords(p, tile, &row_tile, &col_tile);
+        tile_coords<HEADS>(p, tile, &row_tile, &col_tile);
         const int row0 = row_tile * BLOCK_P, col0 = col_tile * p.block_q;
-        const int wrow0 = group * p.group_rows + col0, x_block0 = p.heads ? group * num_kb : 0;
+        const int wrow0 = group * p.group_rows + col0, x_block0 = HEADS ? group * num_kb : 0;
         for (int kb = 0; kb < num_kb; ++kb) {
           mbar_wait(&empty[s], phase ^ 1, abort_flag, &g_error_word, 1);
           mbar_expect_tx(&full[s], stage_bytes);
@@ -537,7 +541,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_row, const __g
     uint32_t phase = 0;
     uint64_t a_desc = a_desc0, b_desc = b_desc0;
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) {
-      if (tile_group(p, tile) < 0) continue;
+      if (tile_group<HEADS>(p, tile) < 0) continue;
       const int a = local & 1;
       mbar_wait(&tmem_empty[a], ((local >> 1) & 1) ^ 1, abort_flag, &g_error_word, 4);
       const uint32_t acc = tmem_base + a * ACC_COLS;
@@ -565,22 +569,20 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_row, const __g
   } else {
     const int quarter = warp & 3;
     int local = 0;
-    Params e = p;  // (by heads: the output of the tile's head)
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) {
-      const int group = tile_group(p, tile);
+      const int group = tile_group<HEADS>(p, tile);
       if (group < 0) continue;
-      if (p.heads) e.out = (__nv_bfloat16*)p.out + (size_t)group * p.head_out;
       const int a = local & 1;
       int row_tile, col_tile;
-      tile_coords(p, tile, &row_tile, &col_tile);
-      const int row0 = row_tile * BLOCK_P, col0 = col_tile * p.block_q;
+      tile_coords<HEADS>(p, tile, &row_tile, &col_tile);
+      const int row0 = row_tile * BLOCK_P, col0 = col_tile * p.block_q, shift = HEADS ? group * p.head_out : 0;
       mbar_wait(&tmem_full[a], (local >> 1) & 1, abort_flag, &g_error_word, 3);
       fence_after_sync();
       const int row = row0 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + a * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
       const bool live = row < p.rows;
-      const bool whole = accumulate_row_serves(e, col0, p.block_q);
-      if (whole) accumulate_row(e, row, col0, p.block_q, taddr, live);
+      const bool whole = accumulate_row_serves(p, col0, p.block_q);
+      if (whole) accumulate_row(p, row, col0, p.block_q, taddr, live);
 #pragma unroll 1
       for (int c = whole ? p.block_q : 0; c < p.block_q; c += 32) {
         float v[32];
@@ -600,7 +602,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_row, const __g
 #pragma unroll
           for (int j = 16; j < 32; ++j) v[j] = 0.f;
         }
-        if (live) epilogue_chunk(e, row, col0 + c, v, cols);
+        if (live) epilogue_chunk(p, row, col0 + c, v, cols, shift);
       }
       // the accumulator may be overwritten once all four warps have read it
       fence_before_sync();
@@ -1228,13 +1230,13 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* o
   const int smem = p.stages * stage_bytes + 1024 + 512;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tc_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            SMEM_LIMIT);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
   const int ctas = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  tl::launch_kernel(gemm_tc_persistent_kernel, dim3(ctas), THREADS, smem, stream, map_row, map_col, p);
+  tl::launch_kernel(gemm_tc_persistent_kernel<false>, dim3(ctas), THREADS, smem, stream, map_row, map_col, p);
   return TL_LAUNCH_CHECK();
 }
 
@@ -1319,13 +1321,13 @@ int tl_gemm_tc_heads(const void* x, const void* w, void* out, long long ldo, int
   const int smem = p.stages * stage_bytes + 1024 + 512;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tc_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            SMEM_LIMIT);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
   const int ctas = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  tl::launch_kernel(gemm_tc_persistent_kernel, dim3(ctas), THREADS, smem, stream, map_row, map_col, p);
+  tl::launch_kernel(gemm_tc_persistent_kernel<true>, dim3(ctas), THREADS, smem, stream, map_row, map_col, p);
   return TL_LAUNCH_CHECK();
 }
 
@@ -1406,13 +1408,13 @@ int tl_gemm_tc_grouped(const void* x, const void* w, void* out, long long ldo, i
   const int smem = p.stages * stage_bytes + 1024 + 512;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tc_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            SMEM_LIMIT);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
   const int ctas = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  tl::launch_kernel(gemm_tc_persistent_kernel, dim3(ctas), THREADS, smem, stream, map_row, map_col, p);
+  tl::launch_kernel(gemm_tc_persistent_kernel<false>, dim3(ctas), THREADS, smem, stream, map_row, map_col, p);
   return TL_LAUNCH_CHECK();
 }
 
