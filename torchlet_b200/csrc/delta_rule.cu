@@ -117,7 +117,7 @@ template <int N> __device__ __forceinline__ void copies_wait() {
 constexpr int KS = 4;
 constexpr int SPLIT_COLS = 16;
 
-template <int DK, bool VEC, int COLS>
+template <int DK, bool VEC, int COLS, bool LONG>
 __global__ void __launch_bounds__(COLS * KS / (COLS == DK ? 2 : 1))
 delta_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ gates,
                   const int* __restrict__ req_indptr, const int* __restrict__ slots, float* __restrict__ state,
@@ -154,11 +154,13 @@ delta_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* 
     for (int e = tid; e < 2 * CHUNK * 6 * DK; e += NT) (&stage[0][0][0][0])[e] = 0.f;
     __syncthreads();
   }
-  // 16-byte copies: a thread's entries of a chunk are the same in every chunk, so their sources are worked out once and move on
-  // by a chunk (with the divisions in the loop a block of 64 threads spent more on them than on the recurrence)
+  // 16-byte copies: a thread's entries of a chunk are the same in every chunk, so for whole chunks (LONG) their sources are worked
+  // out once and move on by a chunk (with the divisions in the loop a block of 64 threads spent more on them than on the
+  // recurrence); for a token or a few, whose kernel is as long as its start, that is the longer way (32 heads of 64, one
+  // token: 2.8 us against 2.3)
   constexpr int QUADS = DK / 4, COPIES = (CHUNK * 6 * QUADS + NT - 1) / NT;
-  const float* source[VEC ? COPIES : 1];
-  if constexpr (VEC) {
+  const float* source[LONG ? COPIES : 1];
+  if constexpr (LONG) {
 #pragma unroll
     for (int i = 0; i < COPIES; ++i) {
       const int e = tid + i * NT, tt = e / (6 * QUADS), what = e / QUADS % 6, q = e % QUADS;
@@ -169,13 +171,22 @@ delta_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* 
   }
   auto fetch = [&](int base, int buf) {
     const int count = last - base < CHUNK ? last - base : CHUNK;
-    if constexpr (VEC) {
+    if constexpr (LONG) {
       const int quads = dim >> 2;
 #pragma unroll
       for (int i = 0; i < COPIES; ++i) {
         const int e = tid + i * NT, tt = e / (6 * QUADS), what = e / QUADS % 6, q = e % QUADS;
         if (tt < count && q < quads) copy16(&stage[buf][tt][what][4 * q], source[i]);
         source[i] += (size_t)CHUNK * (what < 3 ? proj_stride : heads * 3 * dim);
+      }
+    } else if constexpr (VEC) {
+      const int quads = dim >> 2;
+      for (int e = tid; e < count * 6 * quads; e += NT) {
+        const int tt = e / (6 * quads), rest = e - tt * 6 * quads, what = rest / quads, q = rest - what * quads;
+        const int t = base + tt;
+        const float* src = what < 3 ? proj + (size_t)t * proj_stride + what * hd + h * dim
+                                    : gates + (((size_t)t * heads + h) * 3 + (what - 3)) * dim;
+        copy16(&stage[buf][tt][what][4 * q], src + 4 * q);
       }
     } else {
       for (int e = tid; e < count * 6 * dim; e += NT) {
@@ -315,6 +326,33 @@ delta_finish_kernel(const float* __restrict__ o, const float* __restrict__ proj,
     out[(size_t)t * hd + h * dim + i] = from_float<T>(row[i] * inv * weight[h * dim + i] * sigmoidf_(gate[i]));
 }
 
+int sm_count() {
+  static int sms = 0;
+  if (sms <= 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
+      sms = 148;
+  }
+  return sms;
+}
+
+// Whether a head's columns go to several blocks (the bits are the same).  Measured at head sizes 36 to 256, 1 to 384 (request,
+// head) pairs and 1 to 512 tokens a request:
+// - up to 64: a block of 16 columns is faster (128 tokens: 40 -> 25 us) only where at most two lie
+//   on an SM (64 pairs of 64: 40 -> 34; 80 pairs: 40 -> 51), and its longer start has to be won back (64 pairs: 1 token 3.1 -> 4.2 us,
+//   16 tokens 6.7 -> 10; 16 pairs: 16 tokens 6.5 -> 5.3);
+// - up to 128: where at most four lie on an SM (64 pairs of 128: 1 token 5.3 -> 4.2 us, 128 tokens 111 -> 100; 80 pairs:
+//   5.7 -> 6.3 and 112 -> 196);
+// - beyond: the block of all columns is the slower one everywhere (148 pairs of 256: 1 token 48 -> 22 us, 512 tokens equal).
+bool split_columns(int requests, int heads, int dim, int tokens) {
+  const long long pairs = (long long)requests * heads, blocks = pairs * ((dim + SPLIT_COLS - 1) / SPLIT_COLS);
+  if (dim <= 32) return false;
+  if (dim <= 64) return blocks <= 2 * sm_count() && tokens >= (blocks <= sm_count() ? 16ll : 64ll) * requests;
+  if (dim <= 128) return blocks <= 4 * sm_count();
+  return pairs <= sm_count();
+}
+
 }  // namespace
 
 TL_DEBUG_READER(tl_delta_rule_debug_error)
@@ -340,23 +378,24 @@ int tl_delta_prepare(const float* proj, int proj_stride, const float* w2t, const
   return TL_LAUNCH_CHECK();
 }
 
-// state: float32 [max_slots, heads, dim, dim]; out: float32 [tokens, heads * dim].
+// state: float32 [max_slots, heads, dim, dim]; out: float32 [tokens, heads * dim]; tokens: of all requests.
 int tl_delta_scan(const float* proj, int proj_stride, const float* gates, const int* req_indptr, const int* slots,
-                  float* state, float* out, int requests, int heads, int dim, int max_slots, cudaStream_t stream) {
+                  float* state, float* out, int requests, int heads, int dim, int tokens, int max_slots, cudaStream_t stream) {
   if (requests <= 0) return 0;
   if (dim <= 0 || dim > 256 || heads > 65535) return TL_ERR_UNSUPPORTED;
   dim3 grid(requests, heads);
   const bool vec = dim % 4 == 0 && proj_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(proj) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(gates) & 15) == 0;
-  // fewer blocks than SMs: several blocks a head (148 pairs at 16 columns a block are four to sixteen blocks an SM at most)
-  const bool split = dim > 32 && (long long)requests * heads <= 148;
-#define TL_SCAN_COLS(DK, COLS)                                                                                     \
-  if (vec)                                                                                                         \
-    tl::launch_kernel(delta_scan_kernel<DK, true, COLS>, grid, COLS * KS / (COLS == DK ? 2 : 1), 0, stream, proj,  \
-                      proj_stride, gates, req_indptr, slots, state, out, heads, dim, max_slots);                   \
-  else                                                                                                             \
-    tl::launch_kernel(delta_scan_kernel<DK, false, COLS>, grid, COLS * KS / (COLS == DK ? 2 : 1), 0, stream, proj, \
-                      proj_stride, gates, req_indptr, slots, state, out, heads, dim, max_slots)
+  const bool split = split_columns(requests, heads, dim, tokens);
+  // (head sizes up to 64: a chunk of 8 tokens; up to 128: 4 tokens 8.2 -> 7.6 us, 2 equal; beyond: 1 token 20 us against 22)
+  const bool long_portions = vec && (dim > 128 || tokens >= (dim > 64 ? 4ll : 8ll) * requests);
+#define TL_SCAN_INSTANCE(DK, VEC, COLS, LONG)                                                                       \
+  tl::launch_kernel(delta_scan_kernel<DK, VEC, COLS, LONG>, grid, COLS * KS / (COLS == DK ? 2 : 1), 0, stream, proj, \
+                    proj_stride, gates, req_indptr, slots, state, out, heads, dim, max_slots)
+#define TL_SCAN_COLS(DK, COLS)                          \
+  if (long_portions) TL_SCAN_INSTANCE(DK, true, COLS, true);    \
+  else if (vec) TL_SCAN_INSTANCE(DK, true, COLS, (DK > 128)); \
+  else TL_SCAN_INSTANCE(DK, false, COLS, false)
 #define TL_SCAN(DK)                                     \
   if (split) {                                          \
     grid.z = (dim + SPLIT_COLS - 1) / SPLIT_COLS;       \
@@ -371,6 +410,7 @@ int tl_delta_scan(const float* proj, int proj_stride, const float* gates, const 
   else { TL_SCAN(256); }
 #undef TL_SCAN
 #undef TL_SCAN_COLS
+#undef TL_SCAN_INSTANCE
   return TL_LAUNCH_CHECK();
 }
 

@@ -132,7 +132,7 @@ _SIGNATURES = {
         "tl_delta_prepare": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_void_p],
         "tl_delta_scan": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                          c_int, c_void_p],
+                          c_int, c_int, c_void_p],
         "tl_delta_finish": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
                             c_void_p],
         "tl_delta_rule_debug_error": [c_void_p],
@@ -533,7 +533,7 @@ def delta_scan(proj, gates, req_indptr, slots, state, out, requests: int, heads:
     assert state.shape[1:] == (heads, dim, dim) and req_indptr.dtype == slots.dtype == torch.int32
     code = _fn("delta_rule", "tl_delta_scan")(proj.data_ptr(), proj.stride(0), gates.data_ptr(), req_indptr.data_ptr(),
                                               slots.data_ptr(), state.data_ptr(), out.data_ptr(), requests, heads, dim,
-                                              state.shape[0], _stream())
+                                              out.shape[0], state.shape[0], _stream())
     _check(code, "delta_scan")
 
 
