@@ -284,6 +284,9 @@ def test_float32_attention_by_chunks(case):
         assert torch.equal(run(0, T, all_alone=True), whole)
     if min(q_lens) > 1:
         assert torch.equal(run(0, T, some_alone=False), whole)
+    last = max((i + 1 for i, n in enumerate(q_lens) if n <= 8), default=0)
+    assert torch.equal(run(0, T, portions=sum(n > 1 for n in q_lens), least_tokens=min(q_lens), most_tokens=max(q_lens),
+                           few_rows=sum(q_lens[:last])), whole)
 
 
 @pytest.mark.parametrize("case", [c for c in ATTENTION_CASES if c[4] in (64, 128)] + [

@@ -17,8 +17,8 @@
 //
 // Two more kernels take the 32-bit rows of head_dim up to 128 (a multiple of 4) whose keys lie in one window and whose heads
 // read one KV head each (``in_chunks`` below; a rule on the layer alone, so a request never changes between the orders):
-//   attention_f32_single_kernel   a token alone in its step: a block a (token, head), eight warps, each a chunk of keys;
-//   attention_f32_rows_kernel     tokens that stand beside others of their request: 32 packed (token, head) rows of a KV
+//   attention_f32_single_kernel   requests that bring one token, or few: a block a (token, head), eight warps, each a chunk of keys;
+//   attention_f32_rows_kernel     tokens that stand beside many others of their request: 32 packed (token, head) rows of a KV
 //                                 head share the key and value tiles in shared memory.
 // Both cut the keys into CHUNKS of 64 absolute positions: a chunk is an online softmax of its own over its tiles of 32 keys,
 // and the chunks are merged in ascending order.  So the order of every sum still depends on the position and window
@@ -197,7 +197,7 @@ struct ChunkArgs {
   float* out;
   const float* sink_values;
   const float* gate;
-  int q_stride, table_width, out_stride, tokens, nh, nkv, d, page_size, window, num_pages, sink, gate_stride, v_cols, all_alone;
+  int q_stride, table_width, out_stride, tokens, nh, nkv, d, page_size, window, num_pages, sink, gate_stride, v_cols, all_few, pack;
   float scale, softcap;
 };
 
@@ -207,10 +207,15 @@ __device__ __forceinline__ size_t key_row(const ChunkArgs& p, const int* table, 
   if (!TL_DEBUG_OK(page >= 0 && page < p.num_pages, TL_DEBUG_PAGE, page)) page = 0;
   return (((size_t)page * 2 * p.nkv + kvh) * p.page_size + key % p.page_size) * p.d;
 }
-// Whether no neighbouring row belongs to the token's request.
-__device__ __forceinline__ bool alone(const ChunkArgs& p, int t) {
-  const int req = p.token_req[t];
-  return (t == 0 || p.token_req[t - 1] != req) && (t + 1 >= p.tokens || p.token_req[t + 1] != req);
+// Requests that bring up to this many tokens go token by token.
+__host__ __device__ __forceinline__ int few_tokens(int group) { return 1; }
+// Whether the request of token t brings at most ``few`` <= 8 tokens to the step (asked by all lanes of a warp).
+__device__ __forceinline__ bool among_few(const ChunkArgs& p, int t, int few) {
+  const int u = t + (int)(threadIdx.x & 31) - 15;  // the neighbours; lane 15 has t itself
+  const bool there = u >= 0 && u < p.tokens;
+  const int req = there ? p.token_req[u] : 0, mine = __shfl_sync(0xffffffffu, req, 15);
+  const unsigned same = __ballot_sync(0xffffffffu, there && req == mine);
+  return __ffs(~(same >> 15)) - 1 + __clz(~(same << 17)) <= few;  // the ones from bit 15 up and those right below it
 }
 __device__ __forceinline__ void write_out(const ChunkArgs& p, int t, int h, int i, float acc, float inv) {
   if (i >= p.v_cols) return;
@@ -222,7 +227,9 @@ __device__ __forceinline__ void write_out(const ChunkArgs& p, int t, int h, int 
 // Bound by the latency of its walk: table entry, key and value rows, weights.  Eight warps take a chunk of 64 keys each, so
 // 700 keys are two rounds and not 22 tiles in a row, and a tile's values are requested with its keys: a step of 8 requests of up
 // to 700 keys at 14 heads of 64 takes 17 us a layer, 47 with the values requested behind the scores, eight keys at a
-// time (one warp a (token, head): 440).
+// time (one warp a (token, head): 440).  Up to 4 chunks leave warps of such a block idle: in a grid of
+// more than two waves (``pack``) it then takes 2, 4 or 8 heads and the blocks of the others leave at once.  64 requests of 40 keys at
+// 28 heads of 128: 27 us, a head a block 46; one such request 14 and 7.4.
 constexpr int SINGLE_WARPS = 8;
 
 template <int DP>
@@ -230,28 +237,46 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
   tl::pdl_wait();
   tl::pdl_launch_dependents();
   constexpr int VE = DP / 32, BATCH = 64 / VE;  // keys whose values are requested together
-  __shared__ __align__(16) float qs[DP];
-  __shared__ float parts[2][SINGLE_WARPS][DP + 2];  // a chunk's acc, m, l; two rounds
+  __shared__ __align__(16) float qs[SINGLE_WARPS][DP];  // of the block's heads
+  __shared__ float parts[2][SINGLE_WARPS][DP + 2];      // a chunk's acc, m, l; two rounds
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x / p.nh, h = blockIdx.x % p.nh;
-  if (!p.all_alone && !alone(p, t)) return;
-  const int kvh = h / (p.nh / p.nkv), d = p.d;
-  const int pos = p.positions[t], lo = first_key(pos, p.window);
-  const int* table = p.block_table + (size_t)p.token_req[t] * p.table_width;
-  for (int i = threadIdx.x; i < DP; i += SINGLE_WARPS * 32) qs[i] = i < d ? p.q[(size_t)t * p.q_stride + (size_t)h * d + i] : 0.f;
-  __syncthreads();
-  const size_t values = (size_t)p.nkv * p.page_size * d;  // from a key to its value
-  const int i = threadIdx.x;                              // the entry this thread merges
-  Softmax<1> total;
-  total.clear();
-  if (p.sink) {
-    total.m = p.sink_values ? p.sink_values[h] : 0.f;
-    total.l = 1.f;
+  const int t = blockIdx.x / p.nh, h0 = blockIdx.x % p.nh, d = p.d;
+  if (!p.all_few && !among_few(p, t, few_tokens(p.nh / p.nkv))) return;
+  // what does not hang on the position is requested before it
+  const int pos = p.positions[t], req = p.token_req[t];
+  const float* q_rows = p.q + (size_t)t * p.q_stride;
+  const float first_q = threadIdx.x < d ? q_rows[(size_t)h0 * d + threadIdx.x] : 0.f;
+  if (threadIdx.x < DP) qs[0][threadIdx.x] = first_q;
+  const int lo = first_key(pos, p.window);
+  const int chunks = pos / CHUNK_KEYS - lo / CHUNK_KEYS + 1;
+  // warps a head, a power of two: with fewer than eight one round is all
+  const int per_log2 = !p.pack || chunks > 4 ? 3 : (chunks > 2 ? 2 : chunks - 1), per = 1 << per_log2, heads = SINGLE_WARPS >> per_log2;
+  if (h0 & (heads - 1)) return;
+  const int h = h0 + (warp >> per_log2);
+  const int kvh = h / (p.nh / p.nkv);
+  const int* table = p.block_table + (size_t)req * p.table_width;
+  for (int e = DP + threadIdx.x; e < heads * DP; e += SINGLE_WARPS * 32) {
+    const int head = h0 + e / DP, i = e % DP;
+    qs[e / DP][i] = i < d && head < p.nh ? q_rows[(size_t)head * d + i] : 0.f;
   }
+  __syncthreads();
+  const float* my_q = qs[warp >> per_log2];
+  const size_t values = (size_t)p.nkv * p.page_size * d;  // from a key to its value
+  auto nothing_yet = [&](int head) {
+    Softmax<1> s;
+    s.clear();
+    if (p.sink) {
+      s.m = p.sink_values ? p.sink_values[head] : 0.f;
+      s.l = 1.f;
+    }
+    return s;
+  };
+  const int i = threadIdx.x;  // the entry this thread merges where the block has one head
+  Softmax<1> total = nothing_yet(h0);
   int buf = 0;
-  for (int first = lo / CHUNK_KEYS; first <= pos / CHUNK_KEYS; first += SINGLE_WARPS, buf ^= 1) {
-    const int chunk = first + warp;
-    if (chunk <= pos / CHUNK_KEYS) {
+  for (int first = lo / CHUNK_KEYS; first <= pos / CHUNK_KEYS; first += per, buf ^= 1) {
+    const int chunk = first + (warp & (per - 1));
+    if (chunk <= pos / CHUNK_KEYS && h < p.nh) {
       Softmax<VE> part;
       part.clear();
       for (int start = chunk * CHUNK_KEYS; start < (chunk + 1) * CHUNK_KEYS && start <= pos; start += 32) {
@@ -281,7 +306,7 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
               k[c] = base + 4 * c < d ? *reinterpret_cast<const float4*>(p.pages + row + base + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
-              const float4 qv = *reinterpret_cast<const float4*>(qs + base + 4 * c);
+              const float4 qv = *reinterpret_cast<const float4*>(my_q + base + 4 * c);
               dot = fmaf(qv.x, k[c].x, dot);
               dot = fmaf(qv.y, k[c].y, dot);
               dot = fmaf(qv.z, k[c].z, dot);
@@ -295,6 +320,7 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
         const int begin = lo > start ? lo - start : 0, end = pos - start < 31 ? pos - start : 31;
 #pragma unroll
         for (int j0 = 0; j0 < 32; j0 += BATCH) {
+          if (j0 > end) break;
           if (j0) values_from(j0);
 #pragma unroll
           for (int j = 0; j < BATCH; ++j) {
@@ -314,13 +340,27 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
       }
     }
     __syncthreads();  // (the round after the next overwrites this buffer, behind another barrier)
-    if (i < DP)
+    if (heads == 1 && i < DP)
       for (int w = 0; w < SINGLE_WARPS && first + w <= pos / CHUNK_KEYS; ++w) {
         const float acc[1] = {parts[buf][w][i]};
         total.merge(parts[buf][w][DP], parts[buf][w][DP + 1], acc);
       }
   }
-  if (i < DP) write_out(p, t, h, i, total.acc[0], 1.f / total.l);
+  if (heads == 1) {
+    if (i < DP) write_out(p, t, h0, i, total.acc[0], 1.f / total.l);
+    return;
+  }
+  for (int e = threadIdx.x; e < heads * DP; e += SINGLE_WARPS * 32) {
+    const int head = h0 + e / DP;
+    if (head >= p.nh) continue;
+    total = nothing_yet(head);
+    for (int w = 0; w < chunks; ++w) {
+      const float* part = parts[0][e / DP * per + w];
+      const float acc[1] = {part[e % DP]};
+      total.merge(part[DP], part[DP + 1], acc);
+    }
+    write_out(p, t, head, e % DP, total.acc[0], 1.f / total.l);
+  }
 }
 
 // Bound by shared-memory reads and the softmax's shuffles; the tile's keys and values, one 16-byte read a lane instead of a row
@@ -332,7 +372,7 @@ template <int DP> constexpr int ROWS_SMEM = (PACKED * DP + 32 * (DP + 4) + 32 * 
 // A block takes PACKED / group consecutive tokens at one KV head; row r is token r / group, head r % group of the group.  The
 // tokens may belong to several requests, which are taken one after the other.
 template <int DP>
-__global__ void __launch_bounds__(ROWS_WARPS * 32) attention_f32_rows_kernel(const ChunkArgs p) {
+__global__ void __launch_bounds__(ROWS_WARPS * 32, DP == 64 ? 2 : 1) attention_f32_rows_kernel(const ChunkArgs p) {
   tl::pdl_wait();
   tl::pdl_launch_dependents();
   constexpr int VE = DP / 32, NT = ROWS_WARPS * 32, COPIES = 32 * DP / 4 / NT, R = ROWS_A_WARP;
@@ -345,20 +385,27 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) attention_f32_rows_kernel(con
   const int group = p.nh / p.nkv, span = PACKED / group;
   const int kvh = blockIdx.y, t0 = (int)(gridDim.x - 1 - blockIdx.x) * span;  // the last tokens see the most keys: first
   const int count = p.tokens - t0 < span ? p.tokens - t0 : span;
-  for (int e = tid; e < PACKED * DP; e += NT) {
-    const int r = e / DP, i = e % DP, token = r / group;
-    qs[e] = (token < count && i < d) ? p.q[(size_t)(t0 + token) * p.q_stride + (size_t)(kvh * group + r % group) * d + i] : 0.f;
-  }
   const size_t values = (size_t)p.nkv * p.page_size * d;
+  const int my_req = lane < count ? p.token_req[t0 + lane] : 0, my_pos = lane < count ? p.positions[t0 + lane] : 0;  // (span <= 32)
+  bool queries_here = false;
+  const int few = few_tokens(group);
   for (int a = 0, b; a < count; a = b) {  // tokens [a, b) of one request
-    const int req = p.token_req[t0 + a];
-    int least = INT_MAX, most = -1;
-    for (b = a; b < count && p.token_req[t0 + b] == req; ++b) {
-      const int pos = p.positions[t0 + b];
-      least = min(least, first_key(pos, p.window));
-      most = max(most, pos);
+    const int req = __shfl_sync(0xffffffffu, my_req, a);
+    const unsigned others = ~__ballot_sync(0xffffffffu, lane < count && my_req == req) >> a;
+    b = others ? a + __ffs(others) - 1 : count;
+    // the other kernel's (the run may go on in the blocks beside this one)
+    const bool all_here = (a > 0 || t0 == 0) && (b < count || t0 + count == p.tokens);
+    if (b - a <= few && (all_here || among_few(p, t0 + a, few))) continue;
+    const bool here = lane >= a && lane < b;
+    const int least = __reduce_min_sync(0xffffffffu, here ? first_key(my_pos, p.window) : INT_MAX);
+    const int most = __reduce_max_sync(0xffffffffu, here ? my_pos : -1);
+    if (!queries_here) {  // (read behind the first tile's barriers)
+      for (int e = tid; e < PACKED * DP; e += NT) {
+        const int r = e / DP, i = e % DP, token = r / group;
+        qs[e] = (token < count && i < d) ? p.q[(size_t)(t0 + token) * p.q_stride + (size_t)(kvh * group + r % group) * d + i] : 0.f;
+      }
+      queries_here = true;
     }
-    if (b - a == 1 && alone(p, t0 + a)) continue;  // the other kernel's
     const int* table = p.block_table + (size_t)req * p.table_width;
     float4 kr[COPIES], vr[COPIES];
     auto fetch = [&](int start) {
@@ -380,7 +427,8 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) attention_f32_rows_kernel(con
     for (int r = 0; r < R; ++r) {
       const int row = warp * R + r, token = row / group;
       live[r] = row < span * group && token >= a && token < b;
-      pos[r] = live[r] ? p.positions[t0 + token] : -1;
+      pos[r] = __shfl_sync(0xffffffffu, my_pos, token & 31);
+      if (!live[r]) pos[r] = -1;
       lo[r] = live[r] ? first_key(pos[r], p.window) : 0;
       seen[r] = false;
       total[r].clear();
@@ -449,6 +497,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) attention_f32_rows_kernel(con
         __syncwarp();
 #pragma unroll 2
         for (int j = 0; j < 32; j += 4) {
+          if (start + j > most) break;
           float4 w[R];
 #pragma unroll
           for (int r = 0; r < R; ++r) w[r] = *reinterpret_cast<const float4*>(ws + (warp * R + r) * 32 + j);
@@ -492,26 +541,43 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) attention_f32_rows_kernel(con
   }
 }
 
+int sm_count() {
+  static int sms = 0;
+  if (sms <= 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
+      sms = 148;
+  }
+  return sms;
+}
+
 // The layers whose 32-bit rows go by chunks.  Nothing here depends on the step.
 bool in_chunks(int nh, int nkv, int d, int keep, int chunks) {
   return d <= 128 && d % 4 == 0 && nh / nkv <= PACKED && keep == 0 && chunks == 1 && nkv <= 65535;
 }
 
+// ``portions`` requests bring more than one token; none brings fewer than ``least`` or more than ``most``; those of up to 8 lie in
+// the first few_rows rows.
 template <int DP>
-int launch_chunks(const ChunkArgs& p, bool some_alone, cudaStream_t stream) {
-  if (!p.all_alone) {
+int launch_chunks(ChunkArgs p, int portions, int least, int most, int few_rows, cudaStream_t stream) {
+  const int group = p.nh / p.nkv, span = PACKED / group, few = few_tokens(group);
+  p.all_few = most <= few;
+  if (p.all_few) few_rows = p.tokens;
+  else if (least > few) few_rows = 0;
+  if (!p.all_few) {
     static bool configured = false;
     if (!configured && ROWS_SMEM<DP> > 48 * 1024) {
       const cudaError_t err = cudaFuncSetAttribute(attention_f32_rows_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM<DP>);
       if (err != cudaSuccess) return (int)err;
       configured = true;
     }
-    const int span = PACKED / (p.nh / p.nkv);
     tl::launch_kernel(attention_f32_rows_kernel<DP>, dim3((p.tokens + span - 1) / span, p.nkv), ROWS_WARPS * 32, ROWS_SMEM<DP>, stream, p);
     const int rc = TL_LAUNCH_CHECK();
-    if (rc || !some_alone) return rc;
+    if (rc || few_rows == 0) return rc;
   }
-  tl::launch_kernel(attention_f32_single_kernel<DP>, dim3((unsigned)p.tokens * p.nh), SINGLE_WARPS * 32, 0, stream, p);
+  p.pack = (long long)few_rows * p.nh > 4 * sm_count();
+  tl::launch_kernel(attention_f32_single_kernel<DP>, dim3((unsigned)few_rows * p.nh), SINGLE_WARPS * 32, 0, stream, p);
   return TL_LAUNCH_CHECK();
 }
 
@@ -519,13 +585,15 @@ int launch_chunks(const ChunkArgs& p, bool some_alone, cudaStream_t stream) {
 
 TL_DEBUG_READER(tl_attention_generic_debug_error)
 
-// alone: 2: every token is the only one of its request in this step, 0: none is, 1: the kernels find out which are.
+// Hints about the step (1, 1, ``tokens`` and ``tokens`` where nothing is known): how many requests bring more than one token, the fewest and
+// the most tokens that one brings, and the row behind the last of a request of up to 8 tokens.
 extern "C" int tl_attention_generic(const void* q, int q_stride, const void* pages, int dtype,
                                     const int* block_table, int table_width, const int* token_req,
                                     const int* positions, void* out, int out_stride, int tokens,
                                     int nh, int nkv, int d, int page_size, int window, float scale,
                                     int num_pages, float softcap, int sink, const float* sink_values,
-                                    const float* gate, int gate_stride, int keep, int chunks, int v_cols, int alone,
+                                    const float* gate, int gate_stride, int keep, int chunks, int v_cols, int portions, int least,
+                                    int most, int few_rows,
                                     cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (d <= 0 || d > MAX_D || nkv <= 0 || nh % nkv || page_size <= 0) return TL_ERR_UNSUPPORTED;
@@ -533,8 +601,10 @@ extern "C" int tl_attention_generic(const void* q, int q_stride, const void* pag
   if (dtype == TL_DTYPE_F32 && in_chunks(nh, nkv, d, keep, chunks) && (reinterpret_cast<uintptr_t>(pages) & 15) == 0) {
     const ChunkArgs p{(const float*)q, (const float*)pages, block_table, token_req, positions, (float*)out, sink_values, gate,
                       q_stride, table_width, out_stride, tokens, nh, nkv, d, page_size, window, num_pages, sink, gate_stride,
-                      v_cols, alone == 2 || tokens == 1, scale, softcap};
-    return d <= 64 ? launch_chunks<64>(p, alone != 0, stream) : launch_chunks<128>(p, alone != 0, stream);
+                      v_cols, 0, 0, scale, softcap};
+    few_rows = few_rows < tokens ? few_rows : tokens;
+    return d <= 64 ? launch_chunks<64>(p, portions, least, most, few_rows, stream)
+                   : launch_chunks<128>(p, portions, least, most, few_rows, stream);
   }
   const size_t smem = (size_t)WARPS * chunks * d * sizeof(float);
   if (smem > 200 * 1024) return TL_ERR_UNSUPPORTED;

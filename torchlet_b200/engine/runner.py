@@ -93,9 +93,9 @@ class StepContext:
         self.num_tokens = 0
         self.num_requests = 0
         self.max_q_len = 0
+        self.lengths = {}  # how many tokens the requests bring, as ops.attention_generic takes it
         self.max_kv_len = 0
         self.decode_only = False
-        self.some_alone = True  # False: no request brings a single token
         # device int32 tensors
         self.tokens = self.positions = self.token_req = None
         self.req_indptr = self.kv_before = self.slots = self.logit_rows = None
@@ -428,7 +428,7 @@ class ModelRunner:
         view = lambda name: dev[layout[name][0]:layout[name][0] + layout[name][1]]
         ctx = StepContext(self)
         ctx.num_tokens = ctx.num_requests = b
-        ctx.max_q_len, ctx.decode_only = 1, True
+        ctx.max_q_len, ctx.decode_only, ctx.lengths = 1, True, {"all_alone": True}
         ctx.max_kv_len = self.config.max_seq_len
         ctx.tokens, ctx.positions, ctx.token_req = view("tok"), view("pos"), view("req")
         ctx.req_indptr, ctx.kv_before, ctx.slots = view("ind"), view("kvb"), view("slot")
@@ -677,9 +677,15 @@ class ModelRunner:
         ctx = StepContext(self)
         ctx.num_tokens, ctx.num_requests = T, n
         ctx.max_q_len = max(lens)
+        few_rows = T  # without the last requests of many tokens
+        for length in reversed(lens):
+            if length <= 8:
+                break
+            few_rows -= length
+        ctx.lengths = {"portions": sum(length > 1 for length in lens), "least_tokens": min(lens), "most_tokens": ctx.max_q_len,
+                       "few_rows": few_rows}
         ctx.max_kv_len = max(b + q for b, q in zip(kv_before, lens))
         ctx.decode_only = ctx.max_q_len == 1
-        ctx.some_alone = min(lens) == 1
         ctx.tokens, ctx.positions, ctx.token_req = tok_d, pos_d, req_d
         ctx.req_indptr, ctx.kv_before, ctx.slots = ind_d, kvb_d, slot_d
         ctx.logit_rows = row_d if m else None

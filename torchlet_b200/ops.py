@@ -47,7 +47,7 @@ _SIGNATURES = {
     "attention_generic": {
         "tl_attention_generic": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_float, c_int,
-                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "tl_attention_generic_debug_error": [c_void_p],
     },
     "gemm_tc": {
@@ -394,11 +394,14 @@ def _sink(sink, nh: int) -> tuple:
 
 def attention_generic(q, q_stride, pages, block_table, token_req, positions, out, tokens, nh, nkv, d,
                       page_size, window, scale, softcap=None, sink=False, gate=None, keep: int = 0, spread: bool = False,
-                      v_cols=None, all_alone: bool = False, some_alone: bool = True) -> None:
+                      v_cols=None, all_alone: bool = False, some_alone: bool = True, portions: int = 1,
+                      least_tokens: int = 1, most_tokens=None, few_rows=None) -> None:
     """Paged causal GQA attention of any sizes; q may be a view into qkv.  ``keep``: the first that many
     positions stay visible beside the window; ``spread``: query rows span all KV heads, [nh][nkv][d] (``qkv_prepare``);
     ``v_cols``: value entries a head writes (default d); ``all_alone``: every token is its request's only one in
-    this step; ``some_alone`` False: none is (the default lets the kernels find out).
+    this step; ``some_alone`` False: none is; ``portions``, ``least_tokens``, ``most_tokens``, ``few_rows``: how many
+    requests bring more than one token, the fewest and the most that one brings, and the row behind the last request of up to 8 tokens
+    (hints for the launch of float32 rows).
     ``softcap``: scores become softcap * tanh(score / softcap); ``sink``: one is added to the softmax's
     denominator (True), or exp(sink[head]) (a float32 tensor [nh]); ``gate`` (float32 [tokens, >= nh * d] rows): the output is multiplied by sigmoid(gate)."""
     _need_cuda(q, pages, block_table, token_req, positions, out, gate)
@@ -409,7 +412,8 @@ def attention_generic(q, q_stride, pages, block_table, token_req, positions, out
         block_table.shape[1], token_req.data_ptr(), positions.data_ptr(), out.data_ptr(), out.stride(0),
         tokens, nh, nkv, d, page_size, int(window or 0), float(scale), pages.shape[0], float(softcap or 0.0),
         *_sink(sink, nh), _ptr(gate), gate.stride(0) if gate is not None else 0, int(keep), nkv if spread else 1,
-        int(v_cols or d), 2 if all_alone else int(some_alone), _stream())
+        int(v_cols or d), portions, max(least_tokens, 1 if some_alone or all_alone else 2), 1 if all_alone else most_tokens or tokens,
+        tokens if few_rows is None else few_rows, _stream())
     _check(code, "attention_generic")
 
 

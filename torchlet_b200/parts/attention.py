@@ -107,7 +107,7 @@ class AttentionMixer(Mixer):
         if not (ctx.dtype == torch.bfloat16 and attention_bf16.forward(self, ctx, qkv, cache, out)):
             ops.attention_generic(qkv, qkv.stride(0), cache.pages, cache.block_table, ctx.token_req,
                                   ctx.positions, out, tokens, self.num_heads, self.num_kv_heads,
-                                  self.head_dim, cache.page_size, self.window, self.scale, all_alone=ctx.decode_only,
-                                  some_alone=getattr(ctx, "some_alone", True))
+                                  self.head_dim, cache.page_size, self.window, self.scale,
+                                  **getattr(ctx, "lengths", {}))
         if not self.o_proj.accumulate_later(ctx, out, acc):
             self.o_proj.forward(out, acc, accumulate=True)

@@ -305,8 +305,8 @@ class GatedAttentionMixer(Mixer):
         if not (ctx.dtype == torch.bfloat16 and attention_bf16.forward(self, ctx, q, cache, out, gate=gate)):
             ops.attention_generic(q, q.stride(0), cache.pages, cache.block_table, ctx.token_req, ctx.positions, out, tokens,
                                   self.num_heads, self.num_kv_heads, self.head_dim, cache.page_size, self.window, self.scale,
-                                  softcap=self.softcap, sink=self.sink, gate=gate, all_alone=ctx.decode_only,
-                                  some_alone=getattr(ctx, "some_alone", True))
+                                  softcap=self.softcap, sink=self.sink, gate=gate,
+                                  **getattr(ctx, "lengths", {}))
         if self.value_rotation is not None or self.gate == "head_sigmoid":
             ops.head_finish(out, ctx.positions, self.value_rotation.inv_freq if self.value_rotation is not None else None,
                             proj[:, self.gate_offset:] if self.gate == "head_sigmoid" else None, self.num_heads, self.head_dim)
