@@ -250,6 +250,11 @@ def test_attention_generic(case, dtype):
     ([100, 0], [40, 130], 6, 3, 36, 16, 33),
     ([90, 64, 3], [1, 5, 1], 4, 4, 100, 16, 1),
     ([700], [3], 33, 1, 64, 16, None),  # more heads a KV head than packed rows: one warp a (token, head)
+    # requests of so few tokens that they go token by token, and of just more; contexts of one to nine chunks
+    ([0, 63, 64, 128, 255, 256, 520, 3], [8, 9, 1, 2, 7, 3, 5, 8], 5, 5, 64, 16, None),
+    ([300, 0, 100, 60], [2, 3, 1, 4], 15, 5, 128, 16, 70),
+    ([10, 0, 200], [5, 4, 3], 6, 3, 100, 8, None),
+    ([5] * 9, [9, 12, 20, 10, 9, 33, 11, 40, 17], 3, 3, 64, 16, None),  # several requests a block of packed rows
 ])
 def test_float32_attention_by_chunks(case):
     """Rows that share a step, rows alone and any cut between give the same bits (the order of the sums depends on position

@@ -207,8 +207,10 @@ __device__ __forceinline__ size_t key_row(const ChunkArgs& p, const int* table, 
   if (!TL_DEBUG_OK(page >= 0 && page < p.num_pages, TL_DEBUG_PAGE, page)) page = 0;
   return (((size_t)page * 2 * p.nkv + kvh) * p.page_size + key % p.page_size) * p.d;
 }
-// Requests that bring up to this many tokens go token by token.
-__host__ __device__ __forceinline__ int few_tokens(int group) { return 1; }
+// Requests that bring up to this many tokens go token by token: they fill too little of the packed rows of a block, which takes
+// its requests one after the other.  32 requests of 2 tokens behind 1,000 at 8 heads of 64 with a KV head each: 59 us, packed 938
+// (one warp a (token, head): 670).
+__host__ __device__ __forceinline__ int few_tokens(int group) { return group < 8 ? 8 / group : 1; }
 // Whether the request of token t brings at most ``few`` <= 8 tokens to the step (asked by all lanes of a warp).
 __device__ __forceinline__ bool among_few(const ChunkArgs& p, int t, int few) {
   const int u = t + (int)(threadIdx.x & 31) - 15;  // the neighbours; lane 15 has t itself
@@ -370,7 +372,8 @@ constexpr int ROWS_WARPS = 16, ROWS_A_WARP = 2, PACKED = ROWS_WARPS * ROWS_A_WAR
 template <int DP> constexpr int ROWS_SMEM = (PACKED * DP + 32 * (DP + 4) + 32 * DP + PACKED * 32) * 4;
 
 // A block takes PACKED / group consecutive tokens at one KV head; row r is token r / group, head r % group of the group.  The
-// tokens may belong to several requests, which are taken one after the other.
+// tokens may belong to several requests: gridDim.z blocks take them in turn (requests one after the other in a block: 32 of 5
+// tokens at 28 heads of 128, KV heads of 7, 23 us, side by side 15.7).
 template <int DP>
 __global__ void __launch_bounds__(ROWS_WARPS * 32, DP == 64 ? 2 : 1) attention_f32_rows_kernel(const ChunkArgs p) {
   tl::pdl_wait();
@@ -389,13 +392,14 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32, DP == 64 ? 2 : 1) attention_f
   const int my_req = lane < count ? p.token_req[t0 + lane] : 0, my_pos = lane < count ? p.positions[t0 + lane] : 0;  // (span <= 32)
   bool queries_here = false;
   const int few = few_tokens(group);
-  for (int a = 0, b; a < count; a = b) {  // tokens [a, b) of one request
+  for (int a = 0, b, turn = 0; a < count; a = b) {  // tokens [a, b) of one request
     const int req = __shfl_sync(0xffffffffu, my_req, a);
     const unsigned others = ~__ballot_sync(0xffffffffu, lane < count && my_req == req) >> a;
     b = others ? a + __ffs(others) - 1 : count;
     // the other kernel's (the run may go on in the blocks beside this one)
     const bool all_here = (a > 0 || t0 == 0) && (b < count || t0 + count == p.tokens);
     if (b - a <= few && (all_here || among_few(p, t0 + a, few))) continue;
+    if (turn++ % gridDim.z != blockIdx.z) continue;  // another block's
     const bool here = lane >= a && lane < b;
     const int least = __reduce_min_sync(0xffffffffu, here ? first_key(my_pos, p.window) : INT_MAX);
     const int most = __reduce_max_sync(0xffffffffu, here ? my_pos : -1);
@@ -572,7 +576,9 @@ int launch_chunks(ChunkArgs p, int portions, int least, int most, int few_rows, 
       if (err != cudaSuccess) return (int)err;
       configured = true;
     }
-    tl::launch_kernel(attention_f32_rows_kernel<DP>, dim3((p.tokens + span - 1) / span, p.nkv), ROWS_WARPS * 32, ROWS_SMEM<DP>, stream, p);
+    // as many blocks for the same tokens as there are requests among them, up to four
+    const int turns = (int)min(4ll, 1 + ((long long)span * portions + p.tokens / 2) / p.tokens);
+    tl::launch_kernel(attention_f32_rows_kernel<DP>, dim3((p.tokens + span - 1) / span, p.nkv, turns), ROWS_WARPS * 32, ROWS_SMEM<DP>, stream, p);
     const int rc = TL_LAUNCH_CHECK();
     if (rc || few_rows == 0) return rc;
   }
