@@ -868,3 +868,27 @@ def test_bfloat16_products_of_any_size_add_in_ascending_order():
     out = torch.empty(M, N, device=DEV)
     ops.gemm_simt(x, w, out)
     assert (out == 2.0 ** 24).all()
+
+
+@pytest.mark.parametrize("n, q_len", [(300, 1), (300, 40)])
+def test_float32_attention_where_a_chunk_of_keys_is_out_of_reach(n, q_len):
+    """Scores of -inf over whole chunks of 64 keys (an element of these keys is -inf) weigh nothing; the other keys count as
+    without them."""
+    ops = _ops()
+    nh, nkv, d, page = 4, 2, 64, 16
+    x = paged_inputs([n], [q_len], nh, nkv, d, page, torch.float32, seed=3)
+    x["qkv"][:, :nh * d] = x["qkv"][:, :nh * d].abs() + 0.1
+    q, k, v = (t.double().clone() for t in x["dense"][0])
+    q = q.abs() + 0.1
+    gone = list(range(64, 192)) + list(range(256, 300))  # chunks 1 and 2, and the part of chunk 4 that is cached
+    table = x["table"][0].tolist()
+    for key in gone:
+        x["pages"][table[key // page], 0, :, key % page, 5] = -float("inf")
+    out = torch.full((q_len, nh * d), float("nan"), device=DEV)
+    ops.attention_generic(x["qkv"], x["qkv"].stride(0), x["pages"], x["table"], x["token_req"], x["positions"], out, q_len, nh,
+                          nkv, d, page, None, 0.1)
+    s = torch.einsum("thd,shd->hts", q, k.repeat_interleave(nh // nkv, 1)) * 0.1
+    hidden = torch.arange(n + q_len)[None, :] > torch.arange(n, n + q_len)[:, None]
+    hidden[:, gone] = True
+    want = torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(hidden, -float("inf")), -1), v.repeat_interleave(nh // nkv, 1))
+    assert (out.cpu().double() - want.reshape(q_len, -1)).abs().max() <= 1e-5 * v.abs().max()

@@ -156,6 +156,8 @@ constexpr int CHUNK_KEYS = 64;
 // An online softmax over some keys: largest score, weights' sum, and this lane's entries of the weighted sum of values.
 template <int VE> struct Softmax {
   float m, l, acc[VE];
+  // Of a chunk whose scores are all -inf nothing remains; the others' keys count as ever.
+  static __device__ __forceinline__ float finite(float top) { return top == -INFINITY ? 0.f : top; }
   __device__ __forceinline__ void clear() {
     m = -INFINITY;
     l = 0.f;
@@ -164,9 +166,9 @@ template <int VE> struct Softmax {
   }
   // A tile of 32 keys, one a lane, at least one of them valid, ``top`` their largest score: the lane's weight; then, with
   // the sum of the tile's weights, the state behind the tile.
-  __device__ __forceinline__ float weight(float s, float top, bool valid) const { return valid ? expf(s - fmaxf(m, top)) : 0.f; }
+  __device__ __forceinline__ float weight(float s, float top, bool valid) const { return valid ? expf(s - finite(fmaxf(m, top))) : 0.f; }
   __device__ __forceinline__ void rescale(float top, float sum) {
-    const float new_m = fmaxf(m, top), corr = expf(m - new_m);
+    const float new_m = fmaxf(m, top), corr = expf(m - finite(new_m));
     l = fmaf(l, corr, sum);
     m = new_m;
 #pragma unroll
@@ -174,7 +176,7 @@ template <int VE> struct Softmax {
   }
   // Takes the keys of a later chunk in.
   __device__ __forceinline__ void merge(float m2, float l2, const float (&acc2)[VE]) {
-    const float new_m = fmaxf(m, m2), a = expf(m - new_m), b = expf(m2 - new_m);
+    const float new_m = fmaxf(m, m2), a = expf(m - finite(new_m)), b = expf(m2 - finite(new_m));
     l = fmaf(l, a, __fmul_rn(l2, b));
 #pragma unroll
     for (int i = 0; i < VE; ++i) acc[i] = fmaf(acc[i], a, __fmul_rn(acc2[i], b));
