@@ -892,3 +892,18 @@ def test_float32_attention_where_a_chunk_of_keys_is_out_of_reach(n, q_len):
     hidden[:, gone] = True
     want = torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(hidden, -float("inf")), -1), v.repeat_interleave(nh // nkv, 1))
     assert (out.cpu().double() - want.reshape(q_len, -1)).abs().max() <= 1e-5 * v.abs().max()
+
+
+def test_float32_attention_counts_the_kernels_it_launches():
+    ops = _ops()
+    x = paged_inputs([100, 0, 90], [1, 40, 1], 6, 1, 64, 16, torch.float32, seed=3)  # six heads a KV head: one token alone is few
+
+    def launches(a, b, **hints):
+        out, before = torch.empty(b - a, 6 * 64, device=DEV), ops.launch_count
+        ops.attention_generic(x["qkv"][a:b], x["qkv"].stride(0), x["pages"], x["table"], x["token_req"][a:b].contiguous(),
+                              x["positions"][a:b].contiguous(), out, b - a, 6, 1, 64, 16, None, 0.1, **hints)
+        return ops.launch_count - before
+
+    assert launches(0, 42) == launches(0, 42, few_rows=42) == 2
+    assert launches(0, 1) == launches(0, 42, all_alone=True) == 1
+    assert launches(1, 41, some_alone=False) == launches(1, 41, few_rows=0) == 1

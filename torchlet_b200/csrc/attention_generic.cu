@@ -586,7 +586,8 @@ int launch_chunks(ChunkArgs p, int portions, int least, int most, int few_rows, 
   }
   p.pack = (long long)few_rows * p.nh > 4 * sm_count();
   tl::launch_kernel(attention_f32_single_kernel<DP>, dim3((unsigned)few_rows * p.nh), SINGLE_WARPS * 32, 0, stream, p);
-  return TL_LAUNCH_CHECK();
+  const int rc = TL_LAUNCH_CHECK();
+  return rc || p.all_few ? rc : -2;  // two kernels
 }
 
 }  // namespace
@@ -595,6 +596,7 @@ TL_DEBUG_READER(tl_attention_generic_debug_error)
 
 // Hints about the step (1, 1, ``tokens`` and ``tokens`` where nothing is known): how many requests bring more than one token, the fewest and
 // the most tokens that one brings, and the row behind the last of a request of up to 8 tokens.
+// Returns 0, an error code, or -2 where two kernels were launched.
 extern "C" int tl_attention_generic(const void* q, int q_stride, const void* pages, int dtype,
                                     const int* block_table, int table_width, const int* token_req,
                                     const int* positions, void* out, int out_stride, int tokens,

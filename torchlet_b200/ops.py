@@ -414,7 +414,7 @@ def attention_generic(q, q_stride, pages, block_table, token_req, positions, out
         *_sink(sink, nh), _ptr(gate), gate.stride(0) if gate is not None else 0, int(keep), nkv if spread else 1,
         int(v_cols or d), portions, max(least_tokens, 1 if some_alone or all_alone else 2), 1 if all_alone else most_tokens or tokens,
         tokens if few_rows is None else few_rows, _stream())
-    _check(code, "attention_generic")
+    _check(max(code, 0), "attention_generic", max(1, -code))
 
 
 def sample(logits, out, temperature=None, seed=None, counter=None) -> None:
