@@ -199,7 +199,7 @@ struct ChunkArgs {
   float* out;
   const float* sink_values;
   const float* gate;
-  int q_stride, table_width, out_stride, tokens, nh, nkv, d, page_size, window, num_pages, sink, gate_stride, v_cols, all_few, pack;
+  int q_stride, table_width, out_stride, tokens, nh, nkv, d, page_size, window, num_pages, sink, gate_stride, v_cols, all_few;
   float scale, softcap;
 };
 
@@ -232,16 +232,16 @@ __device__ __forceinline__ void write_out(const ChunkArgs& p, int t, int h, int 
 // 700 keys are two rounds and not 22 tiles in a row, and a tile's values are requested with its keys: a step of 8 requests of up
 // to 700 keys at 14 heads of 64 takes 17 us a layer, 47 with the values requested behind the scores, eight keys at a
 // time (one warp a (token, head): 440).  Up to 4 chunks leave warps of such a block idle: in a grid of
-// more than two waves (``pack``) it then takes 2, 4 or 8 heads and the blocks of the others leave at once.  64 requests of 40 keys at
+// more than two waves (PACK) it then takes 2, 4 or 8 heads and the blocks of the others leave at once.  64 requests of 40 keys at
 // 28 heads of 128: 27 us, a head a block 46; one such request 14 and 7.4.
 constexpr int SINGLE_WARPS = 8;
 
-template <int DP>
+template <int DP, bool PACK>
 __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_kernel(const ChunkArgs p) {
   tl::pdl_wait();
   tl::pdl_launch_dependents();
   constexpr int VE = DP / 32, BATCH = 64 / VE;  // keys whose values are requested together
-  __shared__ __align__(16) float qs[SINGLE_WARPS][DP];  // of the block's heads
+  __shared__ __align__(16) float qs[PACK ? SINGLE_WARPS : 1][DP];  // of the block's heads
   __shared__ float parts[2][SINGLE_WARPS][DP + 2];      // a chunk's acc, m, l; two rounds
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x / p.nh, h0 = blockIdx.x % p.nh, d = p.d;
@@ -254,9 +254,9 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
   const int lo = first_key(pos, p.window);
   const int chunks = pos / CHUNK_KEYS - lo / CHUNK_KEYS + 1;
   // warps a head, a power of two: with fewer than eight one round is all
-  const int per_log2 = !p.pack || chunks > 4 ? 3 : (chunks > 2 ? 2 : chunks - 1), per = 1 << per_log2, heads = SINGLE_WARPS >> per_log2;
+  const int per_log2 = !PACK || chunks > 4 ? 3 : (chunks > 2 ? 2 : chunks - 1), per = 1 << per_log2, heads = SINGLE_WARPS >> per_log2;
   if (h0 & (heads - 1)) return;
-  const int h = h0 + (warp >> per_log2);
+  const int local = PACK ? warp >> per_log2 : 0, h = h0 + local;  // this warp's head of the block's
   const int kvh = h / (p.nh / p.nkv);
   const int* table = p.block_table + (size_t)req * p.table_width;
   for (int e = DP + threadIdx.x; e < heads * DP; e += SINGLE_WARPS * 32) {
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
     qs[e / DP][i] = i < d && head < p.nh ? q_rows[(size_t)head * d + i] : 0.f;
   }
   __syncthreads();
-  const float* my_q = qs[warp >> per_log2];
+  const float* my_q = qs[local];
   const size_t values = (size_t)p.nkv * p.page_size * d;  // from a key to its value
   auto nothing_yet = [&](int head) {
     Softmax<1> s;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(SINGLE_WARPS * 32, 2) attention_f32_single_ker
   Softmax<1> total = nothing_yet(h0);
   int buf = 0;
   for (int first = lo / CHUNK_KEYS; first <= pos / CHUNK_KEYS; first += per, buf ^= 1) {
-    const int chunk = first + (warp & (per - 1));
+    const int chunk = first + (PACK ? warp & (per - 1) : warp);
     if (chunk <= pos / CHUNK_KEYS && h < p.nh) {
       Softmax<VE> part;
       part.clear();
@@ -584,8 +584,11 @@ int launch_chunks(ChunkArgs p, int portions, int least, int most, int few_rows, 
     const int rc = TL_LAUNCH_CHECK();
     if (rc || few_rows == 0) return rc;
   }
-  p.pack = (long long)few_rows * p.nh > 4 * sm_count();
-  tl::launch_kernel(attention_f32_single_kernel<DP>, dim3((unsigned)few_rows * p.nh), SINGLE_WARPS * 32, 0, stream, p);
+  const unsigned blocks = (unsigned)few_rows * p.nh;
+  if (blocks > 4u * sm_count())
+    tl::launch_kernel(attention_f32_single_kernel<DP, true>, dim3(blocks), SINGLE_WARPS * 32, 0, stream, p);
+  else
+    tl::launch_kernel(attention_f32_single_kernel<DP, false>, dim3(blocks), SINGLE_WARPS * 32, 0, stream, p);
   const int rc = TL_LAUNCH_CHECK();
   return rc || p.all_few ? rc : -2;  // two kernels
 }
@@ -611,7 +614,7 @@ extern "C" int tl_attention_generic(const void* q, int q_stride, const void* pag
   if (dtype == TL_DTYPE_F32 && in_chunks(nh, nkv, d, keep, chunks) && (reinterpret_cast<uintptr_t>(pages) & 15) == 0) {
     const ChunkArgs p{(const float*)q, (const float*)pages, block_table, token_req, positions, (float*)out, sink_values, gate,
                       q_stride, table_width, out_stride, tokens, nh, nkv, d, page_size, window, num_pages, sink, gate_stride,
-                      v_cols, 0, 0, scale, softcap};
+                      v_cols, 0, scale, softcap};
     few_rows = few_rows < tokens ? few_rows : tokens;
     return d <= 64 ? launch_chunks<64>(p, portions, least, most, few_rows, stream)
                    : launch_chunks<128>(p, portions, least, most, few_rows, stream);
