@@ -183,7 +183,8 @@ template <int MT> constexpr int STREAM_STAGE = 32 * W_STRIDE + MT * W_STRIDE;  /
 // (token group + j TG).  Every staged value then serves several products: one lane a row would read 9 times 16 bytes for 32
 // products at 8 tokens and 33 for 128 at 32, this takes 6 and 12.
 template <int MT> constexpr int TG = MT >= 8 ? 4 : (MT >= 4 ? 2 : 1);
-// few stages and many warps: the more tokens, the longer a chunk's products hide the next chunk's copies
+// From 16 tokens on two stages, for more warps an SM: a warp requests its next chunk behind the products of this one and waits for
+// it, the other warps' products cover the trip.  Three stages keep one more chunk on its way during the products.
 template <int MT> constexpr int STREAM_STAGES = MT >= 16 ? 2 : 3;
 template <int MT> constexpr int STREAM_SMEM = STREAM_WARPS * STREAM_STAGES<MT> * STREAM_STAGE<MT> * 4;
 
