@@ -175,6 +175,32 @@ def test_delta_scan_gives_the_same_bits_from_few_and_from_many_blocks(H, D, stri
         assert torch.equal(out, many[sum(lens[:r]):sum(lens[:r + 1])]) and torch.equal(alone[r], state[r])
 
 
+@pytest.mark.parametrize("H,D,requests", [(4, 64, 1), (40, 64, 2), (5, 128, 8), (75, 32, 4)])
+def test_delta_scan_blocks_kept_apart(H, D, requests):
+    """Portions of 64 tokens and more take shared memory by how many blocks an SM has: one, two, three, more; the bits are
+    those of the same tokens in portions of fewer."""
+    from torchlet_b200 import ops
+
+    n, size = 66, H * D
+    T = n * requests
+    proj = rand(T, 5 * size, seed=3).to(DEV)
+    gates = torch.rand(T, H, 3, D, generator=torch.Generator().manual_seed(4)) / D
+    gates[:, :, 0] = gates[:, :, 0] * D * 0.4 + 0.55
+    gates = gates.view(T, -1).to(DEV)
+    state, out = torch.zeros(requests, H, D, D, device=DEV), torch.empty(T, size, device=DEV)
+    slots = torch.arange(requests, dtype=torch.int32, device=DEV)
+    indptr = torch.arange(0, T + 1, n, dtype=torch.int32, device=DEV)
+    ops.delta_scan(proj, gates, indptr, slots, state, out, requests, H, D)
+    for r in range(requests):
+        again = torch.zeros_like(state)
+        for first, last in ((0, 40), (40, n)):
+            rows = slice(r * n + first, r * n + last)
+            part = torch.empty(last - first, size, device=DEV)
+            ops.delta_scan(proj[rows], gates[rows], torch.tensor([0, last - first], dtype=torch.int32, device=DEV), slots[r:r + 1], again, part, 1, H, D)
+            assert torch.equal(part, out[rows])
+        assert torch.equal(again[r], state[r])
+
+
 @pytest.mark.parametrize("T,H,N,K,gap", [(1, 1, 8, 64, 0), (129, 3, 72, 64, 8), (300, 4, 256, 192, 0), (257, 5, 520, 128, 24)])
 def test_products_by_heads_in_one_launch(T, H, N, K, gap):
     """Against float64 within the rounding of the bfloat16 result; columns between the heads' stay as they were."""

@@ -117,6 +117,30 @@ def test_gla_kernels_carry_the_state(H, D, V, rank, tau):
         close(fin, plain_finish(plain_run(0, 9), slice(0, 9)), tol, "finish")
 
 
+@pytest.mark.parametrize("H,D,V,requests", [(4, 64, 32, 1), (40, 64, 72, 2), (30, 128, 64, 8), (75, 32, 40, 4)])
+def test_gla_scan_blocks_kept_apart(H, D, V, requests):
+    """Portions of 64 tokens and more take shared memory by how many blocks an SM has: one, two, four, more; the bits are
+    those of the same tokens in portions of fewer."""
+    from torchlet_b200 import ops
+
+    n = 66
+    T = n * requests
+    proj = rand(T, 2 * H * D + H * V, seed=4, scale=0.7).to(DEV)
+    decay = (torch.rand(T, H * D, generator=torch.Generator().manual_seed(5)) * 0.3 + 0.7).to(DEV)
+    state, out = torch.zeros(requests, H, D, V, device=DEV), torch.empty(T, H * V, device=DEV)
+    slots = torch.arange(requests, dtype=torch.int32, device=DEV)
+    ops.gla_scan(proj, decay, torch.arange(0, T + 1, n, dtype=torch.int32, device=DEV), slots, state, out, requests, H, D, V, 0.5)
+    for r in range(requests):
+        again = torch.zeros_like(state)
+        for first, last in ((0, 40), (40, n)):
+            rows = slice(r * n + first, r * n + last)
+            part = torch.empty(last - first, H * V, device=DEV)
+            ops.gla_scan(proj[rows], decay[rows], torch.tensor([0, last - first], dtype=torch.int32, device=DEV), slots[r:r + 1], again, part,
+                         1, H, D, V, 0.5)
+            assert torch.equal(part, out[rows])
+        assert torch.equal(again[r], state[r])
+
+
 def test_gla_state_remembers_a_token_far_back():
     """Decay close to one in one channel: a key written 600 tokens earlier still answers its query."""
     from torchlet_b200 import ops

@@ -115,6 +115,19 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
 }
 
+// Dynamic shared memory that keeps the blocks of a LONG kernel apart.  Such a grid, launched while its predecessor
+// still runs, starts wherever room appears first: several blocks land on SMs that have emptied early, others stay
+// idle, and the kernel takes as long as the fullest SM.  With this much more shared memory a block, no SM takes more
+// than its even share, ceil(blocks / SMs).  ``used``: shared memory the block has anyway.  0 from five blocks an SM on,
+// where chance evens them out.
+inline size_t spread_smem(long long blocks, int sms, size_t used) {
+  constexpr size_t SM_BYTES = 228 * 1024, RESERVED = 1024;  // sm_100a: an SM's shared memory, what a block costs beside its own
+  const long long share = (blocks + sms - 1) / sms;
+  if (share < 1 || share > 4) return 0;
+  const size_t least = SM_BYTES / (share + 1) + 16 - RESERVED;  // share + 1 blocks of this size no longer fit
+  return least > used ? (least - used + 15) / 16 * 16 : 0;
+}
+
 // The first key position a query at position ``pos`` sees, by the mask code all paged attention kernels share:
 // window > 0: the last ``window`` positions, the query's own included; window < 0: the positions of the query's own
 // chunk of -window positions (chunks are counted from position 0 of the sequence); 0: every position before it.

@@ -116,6 +116,7 @@ template <int N> __device__ __forceinline__ void copies_wait() {
 // heads of 64: 342 us against 812.
 constexpr int KS = 4;
 constexpr int SPLIT_COLS = 16;
+__host__ __device__ constexpr int scan_chunk(int dk) { return dk <= 64 ? 8 : (dk <= 128 ? 4 : 2); }
 
 template <int DK, bool VEC, int COLS, bool LONG>
 __global__ void __launch_bounds__(COLS * KS / (COLS == DK ? 2 : 1))
@@ -127,7 +128,7 @@ delta_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* 
   constexpr int CPL = COLS == DK ? 2 : 1;  // columns a lane serves
   constexpr int NT = COLS * KS / CPL;
   constexpr int PER = DK / KS;  // key channels a lane keeps of each of its columns
-  constexpr int CHUNK = DK <= 64 ? 8 : (DK <= 128 ? 4 : 2);
+  constexpr int CHUNK = scan_chunk(DK);
   __shared__ __align__(16) float stage[2][CHUNK][6][DK];  // r, k, v, w, u, a*u
   const int req = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int part = tid % KS;
@@ -353,6 +354,14 @@ bool split_columns(int requests, int heads, int dim, int tokens) {
   return pairs <= sm_count();
 }
 
+// ``apart``: the blocks walk long enough (64 tokens) that their places matter more than the larger shared memory's carve-out.
+template <typename... KArgs, typename... Args>
+void scan_launch(void (*kernel)(KArgs...), dim3 grid, int threads, bool apart, size_t used, cudaStream_t stream, Args... args) {
+  size_t smem = apart ? tl::spread_smem((long long)grid.x * grid.y * grid.z, sm_count(), used) : 0;
+  if (smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) smem = 0;
+  tl::launch_kernel(kernel, grid, threads, smem, stream, args...);
+}
+
 }  // namespace
 
 TL_DEBUG_READER(tl_delta_rule_debug_error)
@@ -388,10 +397,11 @@ int tl_delta_scan(const float* proj, int proj_stride, const float* gates, const 
                    (reinterpret_cast<uintptr_t>(gates) & 15) == 0;
   const bool split = split_columns(requests, heads, dim, tokens);
   // (head sizes up to 64: a chunk of 8 tokens; up to 128: 4 tokens 8.2 -> 7.6 us, 2 equal; beyond: 1 token 20 us against 22)
+  const bool long_walk = tokens >= 64ll * requests;
   const bool long_portions = vec && (dim > 128 || tokens >= (dim > 64 ? 4ll : 8ll) * requests);
 #define TL_SCAN_INSTANCE(DK, VEC, COLS, LONG)                                                                       \
-  tl::launch_kernel(delta_scan_kernel<DK, VEC, COLS, LONG>, grid, COLS * KS / (COLS == DK ? 2 : 1), 0, stream, proj, \
-                    proj_stride, gates, req_indptr, slots, state, out, heads, dim, max_slots)
+  scan_launch(delta_scan_kernel<DK, VEC, COLS, LONG>, grid, COLS * KS / (COLS == DK ? 2 : 1), long_walk,             \
+              sizeof(float) * 2 * scan_chunk(DK) * 6 * DK, stream, proj, proj_stride, gates, req_indptr, slots, state, out, heads, dim, max_slots)
 #define TL_SCAN_COLS(DK, COLS)                          \
   if (long_portions) TL_SCAN_INSTANCE(DK, true, COLS, true);    \
   else if (vec) TL_SCAN_INSTANCE(DK, true, COLS, (DK > 128)); \

@@ -145,6 +145,12 @@ constexpr int STAGES = 4;
 // DECAY_BONUS: rows like DECAY_ROWS, and ``bonus`` [heads * dim] weighs the current token's k v^T in its own output.
 // k stands ``k_offset`` numbers behind q, v ``v_offset``.
 constexpr int DECAY_ROWS = 0, DECAY_HEAD = 1, DECAY_TOKEN = 2, DECAY_BONUS = 3;
+__host__ __device__ constexpr bool no_decay_row(int mode) { return mode == DECAY_HEAD || mode == DECAY_TOKEN; }
+__host__ __device__ constexpr int scan_chunk(int dk, int mode) {  // tokens a stage
+  return no_decay_row(mode) ? (dk <= 128 ? 8 : 4) : (dk <= 64 ? 8 : (dk <= 128 ? 4 : 2));
+}
+__host__ __device__ constexpr int scan_row(int dk, int mode, int cols) { return (no_decay_row(mode) ? 2 : 3) * dk + cols + 4; }
+
 template <int DK, bool VEC, int MODE, int COLS>
 __global__ void __launch_bounds__(lanes_a_column(DK) * COLS)
 gla_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ decay,
@@ -153,14 +159,14 @@ gla_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* __
                 const float* __restrict__ bonus, long long k_offset, long long v_offset) {
   tl::pdl_launch_dependents();
   tl::pdl_wait();
-  constexpr bool FIXED = MODE == DECAY_HEAD || MODE == DECAY_TOKEN;  // no decay row is staged
+  constexpr bool FIXED = no_decay_row(MODE);  // no decay row is staged
   constexpr int KS = lanes_a_column(DK);
   constexpr int PER = DK / KS;
   // a staged token: q, k, (a: only where the decay is a row a token), v, the token's decay number.  Without the a
   // row a stage holds twice as many tokens of the larger key sizes, and the walk meets half as many barriers.
   constexpr int VOFF = (FIXED ? 2 : 3) * DK;
-  constexpr int CHUNK = FIXED ? (DK <= 128 ? 8 : 4) : (DK <= 64 ? 8 : (DK <= 128 ? 4 : 2));
-  constexpr int row = VOFF + COLS + 4;
+  constexpr int CHUNK = scan_chunk(DK, MODE);
+  constexpr int row = scan_row(DK, MODE, COLS);
   __shared__ __align__(16) float stage[STAGES * CHUNK * row];  // [STAGES][CHUNK]
   constexpr int NT = KS * COLS;
   const int req = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -504,6 +510,14 @@ __global__ void rotate_heads_kernel(float* __restrict__ rows, int stride, const 
   head[i + half] = v * c + u * s;
 }
 
+// ``apart``: the blocks walk long enough (64 tokens) that their places matter more than the larger shared memory's carve-out.
+template <typename... KArgs, typename... Args>
+void scan_launch(void (*kernel)(KArgs...), dim3 grid, int threads, bool apart, int sms, size_t used, cudaStream_t stream, Args... args) {
+  size_t smem = apart ? tl::spread_smem((long long)grid.x * grid.y * grid.z, sms, used) : 0;
+  if (smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) smem = 0;
+  tl::launch_kernel(kernel, grid, threads, smem, stream, args...);
+}
+
 }  // namespace
 
 TL_DEBUG_READER(tl_gla_debug_error)
@@ -534,11 +548,11 @@ int tl_gla_decay(const float* proj, int proj_stride, int low_offset, const float
 }
 
 // state: float32 [max_slots, heads, dim, vdim]; out: float32 [tokens, heads * vdim].
-// decay_mode: 0 ``decay`` holds [tokens, heads * dim] rows, 1 one constant per head, 2 [tokens, heads] (one number per
+// tokens: of all requests.  decay_mode: 0 ``decay`` holds [tokens, heads * dim] rows, 1 one constant per head, 2 [tokens, heads] (one number per
 // token and head), 3 rows and ``bonus`` [heads * dim].  k_offset, v_offset: how far k and v stand behind q.  qk_heads: how many heads q and k have (divides heads).
 int tl_gla_scan(const float* proj, int proj_stride, const float* decay, const int* req_indptr, const int* slots,
-                float* state, float* out, int requests, int heads, int qk_heads, int dim, int vdim, int max_slots,
-                float qscale, int decay_mode, const float* bonus, long long k_offset, long long v_offset,
+                float* state, float* out, int requests, int heads, int qk_heads, int dim, int vdim, int tokens,
+                int max_slots, float qscale, int decay_mode, const float* bonus, long long k_offset, long long v_offset,
                 cudaStream_t stream) {
   if (requests <= 0) return 0;
   if (dim <= 0 || dim > 256 || vdim <= 0 || vdim > 256 || heads > 65535) return TL_ERR_UNSUPPORTED;
@@ -555,10 +569,12 @@ int tl_gla_scan(const float* proj, int proj_stride, const float* decay, const in
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   }
   const bool narrow = vec && (long long)requests * heads * ((vdim + COLS_NARROW - 1) / COLS_NARROW) <= sms;
+  const bool long_walk = tokens >= 64ll * requests;
 #define TL_SCAN_ONE(DK, VEC, MODE, COLS)                                                                                   \
-  tl::launch_kernel(gla_scan_kernel<DK, VEC, MODE, COLS>, dim3(requests, heads, (vdim + COLS - 1) / COLS),                 \
-                    lanes_a_column(DK) * COLS, 0, stream, proj, proj_stride, decay, req_indptr, slots, state, out, heads,  \
-                    qk_heads, dim, vdim, max_slots, qscale, bonus, k_offset, v_offset)
+  scan_launch(gla_scan_kernel<DK, VEC, MODE, COLS>, dim3(requests, heads, (vdim + COLS - 1) / COLS),                       \
+              lanes_a_column(DK) * COLS, long_walk, sms, sizeof(float) * STAGES * scan_chunk(DK, MODE) * scan_row(DK, MODE, COLS), \
+              stream, proj, proj_stride, decay, req_indptr, slots, state, out, heads, qk_heads, dim, vdim, max_slots,      \
+              qscale, bonus, k_offset, v_offset)
 #define TL_SCAN_MODE(DK, MODE)                                    \
   {                                                               \
     if (narrow) TL_SCAN_ONE(DK, true, MODE, COLS_NARROW);         \

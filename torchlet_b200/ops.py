@@ -158,7 +158,7 @@ _SIGNATURES = {
     "gla": {
         "tl_gla_decay": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
         "tl_gla_scan": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                        c_int, c_int, c_float, c_int, c_void_p, c_longlong, c_longlong, c_void_p],
+                        c_int, c_int, c_int, c_float, c_int, c_void_p, c_longlong, c_longlong, c_void_p],
         "tl_rotate_heads_f32": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "tl_gla_finish": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float,
                           c_void_p],
@@ -589,7 +589,7 @@ def gla_scan(proj, decay, req_indptr, slots, state, out, requests: int, heads: i
     assert state.shape[1:] == (heads, dim, vdim) and req_indptr.dtype == slots.dtype == torch.int32
     code = _fn("gla", "tl_gla_scan")(proj.data_ptr(), proj.stride(0), decay.data_ptr(), req_indptr.data_ptr(),
                                      slots.data_ptr(), state.data_ptr(), out.data_ptr(), requests, heads, qk_heads, dim,
-                                     vdim, state.shape[0], float(qscale), 1 if fixed_decay else (2 if token_decay else (3 if bonus is not None else 0)),
+                                     vdim, out.shape[0], state.shape[0], float(qscale), 1 if fixed_decay else (2 if token_decay else (3 if bonus is not None else 0)),
                                      _ptr(bonus), qk_heads * dim if k_offset is None else int(k_offset),
                                      2 * qk_heads * dim if v_offset is None else int(v_offset), _stream())
     _check(code, "gla_scan")
