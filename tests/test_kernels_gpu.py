@@ -907,3 +907,39 @@ def test_float32_attention_counts_the_kernels_it_launches():
     assert launches(0, 42) == launches(0, 42, few_rows=42) == 2
     assert launches(0, 1) == launches(0, 42, all_alone=True) == 1
     assert launches(1, 41, some_alone=False) == launches(1, 41, few_rows=0) == 1
+
+
+@pytest.mark.parametrize("nh,nkv,d,page", [(28, 4, 128, 16), (14, 2, 64, 8), (16, 1, 128, 64), (5, 5, 64, 32)])
+@pytest.mark.parametrize("splits", [1, 2, 5])
+@pytest.mark.parametrize("window", [None, 70])
+def test_decode_attention_around_the_depth_of_its_rings(nh, nkv, d, page, splits, window):
+    """Contexts of one to seven key tiles and their edges, against float64 over the same bfloat16 rows: the output is rounded
+    once and the weights once (2^-9 each, of a weighted mean of values up to a few units)."""
+    from torchlet_b200 import ops
+
+    g = torch.Generator().manual_seed(nh + page)
+    lens = [1, 2, 63, 64, 65, 128, 191, 192, 193, 256, 257, 320, 400]  # keys, the new token's among them
+    need = [-(-n // page) for n in lens]
+    order = torch.randperm(sum(need), generator=g) + 1
+    pages = torch.full((sum(need) + 1, 2, nkv, page, d), float("nan"), dtype=torch.bfloat16)
+    table = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    rows, at = [], 0
+    for r, n in enumerate(lens):
+        table[r, :need[r]] = order[at:at + need[r]]
+        at += need[r]
+        kv = torch.randn(2, nkv, n, d, generator=g).bfloat16()
+        rows.append(kv.double())
+        for t in range(n):
+            pages[table[r, t // page], :, :, t % page] = kv[:, :, t]
+    qkv = torch.randn(len(lens), (nh + 2 * nkv) * d, generator=g).bfloat16()
+    out = torch.full((len(lens), nh * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    ops.attention_mma(qkv.to(DEV), pages.to(DEV), table.to(DEV), torch.arange(len(lens) + 1, dtype=torch.int32, device=DEV),
+                      torch.tensor(lens, dtype=torch.int32, device=DEV) - 1, None, None, len(lens), out, len(lens), nh, nkv, d, page,
+                      window, d ** -0.5, rows16=True, splits=splits)
+    assert ops.attention_mma_error() == 0
+    for r, n in enumerate(lens):
+        first = max(0, n - window) if window else 0
+        q = qkv[r, :nh * d].double().view(nkv, nh // nkv, d)
+        weight = torch.softmax(q @ rows[r][0][:, first:].transpose(1, 2) * d ** -0.5, -1)
+        want = (weight @ rows[r][1][:, first:]).reshape(nh * d)
+        assert (out[r].cpu().double() - want).abs().max() <= 1e-2 * max(1.0, want.abs().max().item()), n

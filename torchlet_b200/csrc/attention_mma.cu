@@ -18,12 +18,11 @@
 //           blockIdx.z; each split then writes its (max, sum, accumulator) to a workspace
 //           and a second kernel merges the splits.
 //
-// Decode tiles (ROWS16) with a page size that is a multiple of 8 and divides 64 get their keys
-// and values by TMA instead: one box of page_size x 64 elements per page, K or V and half of the
-// head, one lane of warp 0 a box, into the 128-byte-swizzled layout that ldmatrix reads without
-// bank conflicts; the warps wait on an mbarrier per stage (bounded; a wait that gives up leaves a
-// code that tl_attention_mma_error() returns).  The gather with cp.async costs every thread some
-// hundred instructions a tile, which is what the 16-row tiles spent most of their time on.
+// Decode tiles (ROWS16) with a page size that is a multiple of 8 and divides 64 run on a kernel of
+// their own (attention_decode_kernel) and get their keys and values by TMA: one box per page, K or V, one lane
+// of a fifth warp a box, into the 128-byte-swizzled layout that ldmatrix reads without bank
+// conflicts; the warps wait on mbarriers (bounded; a wait that gives up leaves a code that
+// tl_attention_mma_error() returns).
 //
 // Reference counterparts: forward_ragged_attention_kernel and
 // forward_slot_attention_decode_kernel (v10_triton_paged_gqa/kernel/gqa.py:5-228), which
@@ -141,8 +140,25 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], const void* 
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(s));
 }
+// The same at an address in shared memory's own window: the decode kernel's warps run one to a scheduler, where every
+// instruction of an address counts.
+__device__ __forceinline__ void ldmatrix_x4_at(unsigned (&r)[4], unsigned s) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(s));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans_at(unsigned (&r)[4], unsigned s) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(s));
+}
+__device__ __forceinline__ float exp2_fast(float x) {  // (results below 2^-126 are zero)
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ void mma_16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
       "{%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -157,36 +173,6 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 // the row, so that the 8 rows of an ldmatrix fall into different banks.
 template <int D> __device__ __forceinline__ __nv_bfloat16* tile_at(__nv_bfloat16* tile, int row, int chunk) {
   return tile + row * D + ((chunk ^ (row & 7)) << 3);
-}
-
-// The same for a [64][D] key or value tile: with TMA the tile is D / 64 slabs of [64 rows][64
-// elements], each row 128 bytes with its 16-byte chunks xor-ed by the row (the 128-byte swizzle
-// of the copy); for D = 64 the two layouts are one.
-template <int D, bool TMA> __device__ __forceinline__ __nv_bfloat16* kv_at(__nv_bfloat16* tile, int row, int chunk) {
-  if constexpr (TMA) return tile + (chunk >> 3) * (BLOCK_N * 64) + row * 64 + (((chunk & 7) ^ (row & 7)) << 3);
-  return tile_at<D>(tile, row, chunk);
-}
-
-// Requests the K and V pages of keys [tile * 64, tile * 64 + 64) of one KV head by TMA into a
-// stage (warp 0, one lane a box).  Pages past the request's last key or past the table are
-// read from page 0 (always there; their keys are masked and their value rows are cleared in
-// shared memory before use).
-template <int D>
-__device__ __forceinline__ void tma_kv_tile(const CUtensorMap* map, const Params& p, const int* table, int kvh, int tile,
-                                            int hi_key, __nv_bfloat16* stage, uint64_t* full, int lane) {
-  constexpr int SLABS = D / 64;
-  const int pages_per_tile = BLOCK_N / p.page_size;
-  const int boxes = pages_per_tile * 2 * SLABS;  // at most 8 * 2 * 2 = 32
-  if (lane == 0) tc::mbar_expect_tx(full, 2 * BLOCK_N * D * 2);
-  __syncwarp();
-  if (lane < boxes) {
-    const int slab = lane % SLABS, is_v = (lane / SLABS) & 1, page_i = lane / (2 * SLABS);
-    const int index = tile * pages_per_tile + page_i;
-    const bool wanted = index < p.table_width && index * p.page_size <= hi_key;
-    const int page = wanted ? table[index] : 0;
-    __nv_bfloat16* dst = stage + is_v * (BLOCK_N * D) + slab * (BLOCK_N * 64) + page_i * p.page_size * 64;
-    tc::tma_load_2d(dst, map, full, slab * 64, ((page * 2 + is_v) * p.nkv + kvh) * p.page_size);
-  }
 }
 
 // Gathers the K and V rows of keys [key0, key0 + 64) of one KV head into shared memory.
@@ -240,13 +226,147 @@ __device__ __forceinline__ int effective_splits(int splits, int key_tiles) {
   return min(splits, max(1, (key_tiles + MIN_TILES_A_SPLIT - 1) / MIN_TILES_A_SPLIT));
 }
 
-// STAGES: key/value tiles in shared memory; 2, or 3 with the TMA loader where the grid leaves
-// room for only two CTAs an SM anyway.
-template <int D, bool ROWS16, bool TMA, int STAGES, bool EXTRAS>
-__global__ void __launch_bounds__(THREADS, STAGES == 2 ? 3 : 2)
-attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
-  static_assert(!TMA || ROWS16, "the TMA loader serves the 16-row tiles");
-  static_assert(STAGES == 2 || TMA, "more than two stages need the TMA loader");
+// A barrier of the four multiplying warps (the decode kernel has a fifth, which does not take part).
+__device__ __forceinline__ void rows_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// The end of a 16-row tile: merges the four warps' states through ``merge`` (shared memory that nothing else uses any
+// more), then writes the output or this split's partial result.
+template <int D, bool EXTRAS>
+__device__ __forceinline__ void finish_rows16(const Params& p, const float (&o_acc)[D / 8][4], const float (&m_run)[2],
+                                              const float (&l_run)[2], float* merge, int warp, int lane, int row_start,
+                                              int row_end, int tok0, int g, int kvh, int split, int my_splits) {
+  constexpr int DTILES = D / 8;
+  rows_barrier();
+  // merge[w][row][D + 2]: acc, then max and sum
+  constexpr int STRIDE = D + 2;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = (lane >> 2) + 8 * h;
+    float* dst = merge + ((size_t)warp * 16 + r) * STRIDE;
+#pragma unroll
+    for (int i = 0; i < DTILES; ++i) {
+      dst[i * 8 + (lane & 3) * 2] = o_acc[i][2 * h];
+      dst[i * 8 + (lane & 3) * 2 + 1] = o_acc[i][2 * h + 1];
+    }
+    if ((lane & 3) == 0) {
+      dst[D] = m_run[h];
+      dst[D + 1] = l_run[h];
+    }
+  }
+  rows_barrier();
+  const int rows_here = row_end - row_start;
+  for (int i = threadIdx.x; i < rows_here * D; i += THREADS) {
+    const int r = i / D, c = i % D;
+    float m_all = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) m_all = fmaxf(m_all, merge[((size_t)w * 16 + r) * STRIDE + D]);
+    const float m_ref = m_all == -INFINITY ? 0.f : m_all;
+    float acc = 0.f, l = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float* src = merge + ((size_t)w * 16 + r) * STRIDE;
+      const float f = exp2f(src[D] - m_ref);
+      acc += src[c] * f;
+      l += src[D + 1] * f;
+    }
+    const int row = row_start + r;
+    const int token = tok0 + row / g, head = kvh * g + row % g;
+    if (p.splits > 1) {
+      // key splits serve tiles of ONE token: the partial sums are indexed by (tile, head)
+      if (row >= g) continue;
+      const size_t item = ((size_t)blockIdx.x * p.nh + head) * p.splits + split;
+      p.part_acc[item * D + c] = acc;
+      if (c == 0) {
+        p.part_ml[item * 2] = m_all;
+        p.part_ml[item * 2 + 1] = l;
+      }
+    } else {
+      const PriorFactors pf = prior_of<EXTRAS>(p, token, head, m_all);
+      acc = acc * pf.own + prior_value<EXTRAS>(p, pf, token, head, D, c);
+      l = l * pf.own + pf.sum;
+      p.out[(size_t)token * p.out_stride + (size_t)head * D + c] =
+          __float2bfloat16_rn(acc / with_sink<EXTRAS>(p, head, l, m_all) * gate_of<EXTRAS>(p, token, head, D, c));
+    }
+  }
+  if (p.splits > 1 && p.arrivals) {
+    // The split that writes last merges all of them: no second kernel.  The last CTA reads the
+    // others' partial results from the L2.
+    __shared__ int last_to_arrive;
+    rows_barrier();  // every thread's partial results are written ...
+    int* counter = p.arrivals + (size_t)blockIdx.x * p.nkv + kvh;
+    if (threadIdx.x == 0) {
+      int ticket;  // ... and released to the GPU by the arrival itself; the last one acquires the others'
+      asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
+      last_to_arrive = ticket == my_splits - 1;
+      if (last_to_arrive) *counter = 0;  // zero again for the next launch
+    }
+    rows_barrier();
+    if (last_to_arrive) {
+      // Four output elements a thread and pass.  A thread asks for every split's (max, sum) of its
+      // head and for every split's four sums at once (one round trip to the L2), then weighs them.
+      for (int i = threadIdx.x; i < g * (D / 4); i += THREADS) {
+        const int r = i / (D / 4), c = (i % (D / 4)) * 4;
+        const size_t item = ((size_t)blockIdx.x * p.nh + kvh * g + r) * p.splits;
+        const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + item;
+        const float4* src = reinterpret_cast<const float4*>(p.part_acc + item * D + c);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float m_ref = -INFINITY, l = 0.f;
+        for (int sp = 0; sp < my_splits; sp += 16) {
+          float4 v[16];
+          float2 w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const bool used = sp + j < my_splits;
+            w[j] = used ? __ldcg(ml + sp + j) : make_float2(-INFINITY, 0.f);
+            v[j] = used ? __ldcg(src + (size_t)(sp + j) * (D / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+          float m_new = m_ref;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) m_new = fmaxf(m_new, w[j].x);
+          const float m_use = m_new == -INFINITY ? 0.f : m_new;
+          const float corr = exp2f(m_ref - m_use);  // 0 in the first round
+          acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
+          l *= corr;
+          m_ref = m_new;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float f = exp2f(w[j].x - m_use);  // exp2(-inf) = 0 for the unused ones
+            l = fmaf(w[j].y, f, l);
+            acc.x = fmaf(v[j].x, f, acc.x);
+            acc.y = fmaf(v[j].y, f, acc.y);
+            acc.z = fmaf(v[j].z, f, acc.z);
+            acc.w = fmaf(v[j].w, f, acc.w);
+          }
+        }
+        {
+          const PriorFactors pf = prior_of<EXTRAS>(p, tok0, kvh * g + r, m_ref);
+          l = l * pf.own + pf.sum;
+          acc.x = acc.x * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c);
+          acc.y = acc.y * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c + 1);
+          acc.z = acc.z * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c + 2);
+          acc.w = acc.w * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c + 3);
+        }
+        const float inv = 1.f / with_sink<EXTRAS>(p, kvh * g + r, l, m_ref);
+        if (EXTRAS && p.gate) {
+          const int head = kvh * g + r;
+          acc.x *= gate_of<EXTRAS>(p, tok0, head, D, c);
+          acc.y *= gate_of<EXTRAS>(p, tok0, head, D, c + 1);
+          acc.z *= gate_of<EXTRAS>(p, tok0, head, D, c + 2);
+          acc.w *= gate_of<EXTRAS>(p, tok0, head, D, c + 3);
+        }
+        uint2 packed;
+        packed.x = pack_bf16(acc.x * inv, acc.y * inv);
+        packed.y = pack_bf16(acc.z * inv, acc.w * inv);
+        *reinterpret_cast<uint2*>(p.out + (size_t)tok0 * p.out_stride + (size_t)(kvh * g + r) * D + c) = packed;
+      }
+    }
+  }
+}
+
+// Tiles of 64 packed rows, and of 16 where the page size does not suit the decode kernel's TMA boxes.
+template <int D, bool ROWS16, bool EXTRAS>
+__global__ void __launch_bounds__(THREADS, 3)
+attention_mma_kernel(const Params p) {
   // The wait on the preceding kernel comes further down: the step's metadata is written
   // by a host copy before any kernel of the step, and key/value tiles that lie wholly
   // before the step's own tokens were written by earlier steps, so both may be read first.
@@ -261,16 +381,10 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   // second stage's space; once every warp holds its Q fragments in registers that space
   // is free for the key/value tiles, so three CTAs fit an SM.
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  // the swizzle of the TMA copies works on address bits: the stages start on a 1024-byte boundary
-  uint8_t* smem_base = TMA ? reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023)
-                           : smem_raw;
-  __nv_bfloat16* kv = reinterpret_cast<__nv_bfloat16*>(smem_base);
+  __nv_bfloat16* kv = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   // 64-row tiles: Q [64][D] inside stage 1.  16-row tiles (decode): Q [16][D] after the
   // stages, so that both stages can be filled before the wait on the preceding kernel.
-  __nv_bfloat16* qs = ROWS16 ? kv + STAGES * 2 * BLOCK_N * D : kv + 2 * BLOCK_N * D;
-  // TMA: one "tile has landed" barrier a stage and the block's "a wait gave up" word, after Q
-  uint64_t* full = reinterpret_cast<uint64_t*>(qs + BLOCK_M * D);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(full + STAGES);
+  __nv_bfloat16* qs = ROWS16 ? kv + 2 * 2 * BLOCK_N * D : kv + 2 * BLOCK_N * D;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int req = p.tile_req ? p.tile_req[blockIdx.x] : blockIdx.x;
@@ -307,29 +421,16 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
     tile_begin = tile_begin + split * per;
     tile_end = min(tile_end, tile_begin + per);
   }
-  if constexpr (TMA) {
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < STAGES; ++i) tc::mbar_init(&full[i], 1);
-      *abort_flag = 0;
-      tc::mbar_fence_init();
-      tc::prefetch_tensormap(&map_kv);
-    }
-    __syncthreads();
-  }
 
   // ---- key/value tiles that earlier steps wrote may be requested before the wait
   constexpr int STAGE_ELEMS = 2 * BLOCK_N * D;
   const int num_tiles = max(0, tile_end - tile_begin);
   int issued = 0;  // tiles requested so far, counted from tile_begin
   if constexpr (ROWS16) {
-    while (issued < min(STAGES, num_tiles) && (tile_begin + issued) * BLOCK_N + BLOCK_N - 1 < before) {
+    while (issued < min(2, num_tiles) && (tile_begin + issued) * BLOCK_N + BLOCK_N - 1 < before) {
       __nv_bfloat16* stage = kv + issued * STAGE_ELEMS;
-      if constexpr (TMA) {
-        if (warp == 0) tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin + issued, hi_key, stage, &full[issued], lane);
-      } else {
-        load_kv_tile<D>(p, table, kvh, (tile_begin + issued) * BLOCK_N, lo_key, hi_key, stage, stage + BLOCK_N * D);
-        cp_async_commit();
-      }
+      load_kv_tile<D>(p, table, kvh, (tile_begin + issued) * BLOCK_N, lo_key, hi_key, stage, stage + BLOCK_N * D);
+      cp_async_commit();
       ++issued;
     }
   }
@@ -350,11 +451,7 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   }
   cp_async_commit();
   if (issued == 0 && num_tiles > 0) {
-    if constexpr (TMA) {
-      if (warp == 0) tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin, hi_key, kv, &full[0], lane);
-    } else {
-      load_kv_tile<D>(p, table, kvh, tile_begin * BLOCK_N, lo_key, hi_key, kv, kv + BLOCK_N * D);
-    }
+    load_kv_tile<D>(p, table, kvh, tile_begin * BLOCK_N, lo_key, hi_key, kv, kv + BLOCK_N * D);
     issued = 1;
   }
   cp_async_commit();
@@ -391,51 +488,18 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
   }
   __syncthreads();  // stage 1 may now be overwritten by key/value tiles
 
-  // the only tiles that can hold rows of keys outside [lo_key, hi_key]
-  const int edge_hi_tile = hi_key / BLOCK_N, edge_lo_tile = lo_key > 0 ? lo_key / BLOCK_N : -1;
-  // One key tile.  EDGE: the tile may hold rows of keys outside [lo_key, hi_key] (only the first
-  // and the last tile of a request can); the common tiles run a body without that code.
-  auto process_tile = [&](const int tile, auto edge_tag) {
-    constexpr bool EDGE = decltype(edge_tag)::value;
-    const int index = tile - tile_begin;
-    const int stage = index % STAGES;
+  for (int tile = tile_begin; tile < tile_end; ++tile) {
+    const int index = tile - tile_begin, stage = index & 1;
     __nv_bfloat16* ks_tile = kv + stage * STAGE_ELEMS;
     __nv_bfloat16* vs_tile = ks_tile + BLOCK_N * D;
-    if constexpr (TMA) {
-      // keep STAGES tiles requested: the stage of tile index - 1 is free since the barrier that ended it
-      while (issued < min(num_tiles, index + STAGES)) {
-        const int s_next = issued % STAGES;
-        if (warp == 0)
-          tma_kv_tile<D>(&map_kv, p, table, kvh, tile_begin + issued, hi_key, kv + s_next * STAGE_ELEMS, &full[s_next], lane);
-        ++issued;
-      }
-    } else if (issued == index + 1 && index + 1 < num_tiles) {  // request the next tile into the other stage
+    if (issued == index + 1 && index + 1 < num_tiles) {  // request the next tile into the other stage
       __nv_bfloat16* next = kv + (stage ^ 1) * STAGE_ELEMS;
       load_kv_tile<D>(p, table, kvh, (tile + 1) * BLOCK_N, lo_key, hi_key, next, next + BLOCK_N * D);
       ++issued;
     }
-    if constexpr (TMA) {
-      tc::mbar_wait(&full[stage], (index / STAGES) & 1, abort_flag, &g_error_word, 1);  // this tile is here
-      // Whole pages were copied: value rows of keys outside [lo_key, hi_key] hold whatever the page
-      // held before (another request's values, page 0).  Their weights are exactly 0, but 0 x NaN
-      // is NaN, so the warp clears those of its own 16 rows before it multiplies.
-      if constexpr (EDGE) {
-        const int key_first = tile * BLOCK_N + warp * 16;
-        if (key_first + 15 > hi_key || key_first < lo_key) {
-          for (int i = lane; i < 16 * (D / 8); i += 32) {
-            const int r = i / (D / 8), c = i % (D / 8);
-            if (key_first + r > hi_key || key_first + r < lo_key)
-              *reinterpret_cast<uint4*>(kv_at<D, true>(vs_tile, warp * 16 + r, c)) = make_uint4(0u, 0u, 0u, 0u);
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // a later TMA copy may refill the stage
-          __syncwarp();
-        }
-      }
-    } else {
-      cp_async_commit();
-      cp_async_wait<1>();  // everything but the request just made has landed: this tile is here
-      __syncthreads();
-    }
+    cp_async_commit();
+    cp_async_wait<1>();  // everything but the request just made has landed: this tile is here
+    __syncthreads();
 
     const int key_base = tile * BLOCK_N + (ROWS16 ? warp * 16 : 0);  // first key this warp multiplies
     const int key_row0 = ROWS16 ? warp * 16 : 0;                      // its row inside the tile
@@ -451,7 +515,7 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
         unsigned b[4];
         const int r = key_row0 + nb * 16 + (lane & 7) + (lane >> 4) * 8;
         const int c = 2 * ks + ((lane >> 3) & 1);
-        ldmatrix_x4(b, kv_at<D, TMA>(ks_tile, r, c));
+        ldmatrix_x4(b, tile_at<D>(ks_tile, r, c));
         mma_16816(s[2 * nb], q_frag[ks], b[0], b[1]);
         mma_16816(s[2 * nb + 1], q_frag[ks], b[2], b[3]);
       }
@@ -523,149 +587,19 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
         unsigned b[4];
         const int r = key_row0 + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
         const int c = 2 * nb + (lane >> 4);
-        ldmatrix_x4_trans(b, kv_at<D, TMA>(vs_tile, r, c));
+        ldmatrix_x4_trans(b, tile_at<D>(vs_tile, r, c));
         mma_16816(o_acc[2 * nb], p_frag[kk], b[0], b[1]);
         mma_16816(o_acc[2 * nb + 1], p_frag[kk], b[2], b[3]);
       }
     }
     __syncthreads();  // the stage may be overwritten by the load after next
-  };
-  for (int tile = tile_begin; tile < tile_end; ++tile) {
-    if (TMA && (tile == edge_hi_tile || tile == edge_lo_tile))
-      process_tile(tile, std::true_type{});
-    else
-      process_tile(tile, std::false_type{});
   }
   cp_async_wait<0>();
 
   // ---- finish: merge the warps (ROWS16), then write output or split partials
-  float* merge = reinterpret_cast<float*>(kv);  // reuse the K/V stages
   if constexpr (ROWS16) {
-    __syncthreads();
-    // merge[w][row][D + 2]: acc, then max and sum
-    constexpr int STRIDE = D + 2;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = (lane >> 2) + 8 * h;
-      float* dst = merge + ((size_t)warp * 16 + r) * STRIDE;
-#pragma unroll
-      for (int i = 0; i < DTILES; ++i) {
-        dst[i * 8 + (lane & 3) * 2] = o_acc[i][2 * h];
-        dst[i * 8 + (lane & 3) * 2 + 1] = o_acc[i][2 * h + 1];
-      }
-      if ((lane & 3) == 0) {
-        dst[D] = m_run[h];
-        dst[D + 1] = l_run[h];
-      }
-    }
-    __syncthreads();
-    const int rows_here = row_end - row_start;
-    for (int i = threadIdx.x; i < rows_here * D; i += THREADS) {
-      const int r = i / D, c = i % D;
-      float m_all = -INFINITY;
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) m_all = fmaxf(m_all, merge[((size_t)w * 16 + r) * STRIDE + D]);
-      const float m_ref = m_all == -INFINITY ? 0.f : m_all;
-      float acc = 0.f, l = 0.f;
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) {
-        const float* src = merge + ((size_t)w * 16 + r) * STRIDE;
-        const float f = exp2f(src[D] - m_ref);
-        acc += src[c] * f;
-        l += src[D + 1] * f;
-      }
-      const int row = row_start + r;
-      const int token = tok0 + row / g, head = kvh * g + row % g;
-      if (p.splits > 1) {
-        // key splits serve tiles of ONE token: the partial sums are indexed by (tile, head)
-        if (row >= g) continue;
-        const size_t item = ((size_t)blockIdx.x * p.nh + head) * p.splits + split;
-        p.part_acc[item * D + c] = acc;
-        if (c == 0) {
-          p.part_ml[item * 2] = m_all;
-          p.part_ml[item * 2 + 1] = l;
-        }
-      } else {
-        const PriorFactors pf = prior_of<EXTRAS>(p, token, head, m_all);
-        acc = acc * pf.own + prior_value<EXTRAS>(p, pf, token, head, D, c);
-        l = l * pf.own + pf.sum;
-        p.out[(size_t)token * p.out_stride + (size_t)head * D + c] =
-            __float2bfloat16_rn(acc / with_sink<EXTRAS>(p, head, l, m_all) * gate_of<EXTRAS>(p, token, head, D, c));
-      }
-    }
-    if (p.splits > 1 && p.arrivals) {
-      // The split that writes last merges all of them: no second kernel.  The last CTA reads the
-      // others' partial results from the L2.
-      __shared__ int last_to_arrive;
-      __syncthreads();  // every thread's partial results are written ...
-      int* counter = p.arrivals + (size_t)blockIdx.x * p.nkv + kvh;
-      if (threadIdx.x == 0) {
-        int ticket;  // ... and released to the GPU by the arrival itself; the last one acquires the others'
-        asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
-        last_to_arrive = ticket == my_splits - 1;
-        if (last_to_arrive) *counter = 0;  // zero again for the next launch
-      }
-      __syncthreads();
-      if (last_to_arrive) {
-        // Four output elements a thread and pass.  A thread asks for every split's (max, sum) of its
-        // head and for every split's four sums at once (one round trip to the L2), then weighs them.
-        for (int i = threadIdx.x; i < g * (D / 4); i += THREADS) {
-          const int r = i / (D / 4), c = (i % (D / 4)) * 4;
-          const size_t item = ((size_t)blockIdx.x * p.nh + kvh * g + r) * p.splits;
-          const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + item;
-          const float4* src = reinterpret_cast<const float4*>(p.part_acc + item * D + c);
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-          float m_ref = -INFINITY, l = 0.f;
-          for (int sp = 0; sp < my_splits; sp += 16) {
-            float4 v[16];
-            float2 w[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const bool used = sp + j < my_splits;
-              w[j] = used ? __ldcg(ml + sp + j) : make_float2(-INFINITY, 0.f);
-              v[j] = used ? __ldcg(src + (size_t)(sp + j) * (D / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            float m_new = m_ref;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) m_new = fmaxf(m_new, w[j].x);
-            const float m_use = m_new == -INFINITY ? 0.f : m_new;
-            const float corr = exp2f(m_ref - m_use);  // 0 in the first round
-            acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
-            l *= corr;
-            m_ref = m_new;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float f = exp2f(w[j].x - m_use);  // exp2(-inf) = 0 for the unused ones
-              l = fmaf(w[j].y, f, l);
-              acc.x = fmaf(v[j].x, f, acc.x);
-              acc.y = fmaf(v[j].y, f, acc.y);
-              acc.z = fmaf(v[j].z, f, acc.z);
-              acc.w = fmaf(v[j].w, f, acc.w);
-            }
-          }
-          {
-            const PriorFactors pf = prior_of<EXTRAS>(p, tok0, kvh * g + r, m_ref);
-            l = l * pf.own + pf.sum;
-            acc.x = acc.x * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c);
-            acc.y = acc.y * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c + 1);
-            acc.z = acc.z * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c + 2);
-            acc.w = acc.w * pf.own + prior_value<EXTRAS>(p, pf, tok0, kvh * g + r, D, c + 3);
-          }
-          const float inv = 1.f / with_sink<EXTRAS>(p, kvh * g + r, l, m_ref);
-          if (EXTRAS && p.gate) {
-            const int head = kvh * g + r;
-            acc.x *= gate_of<EXTRAS>(p, tok0, head, D, c);
-            acc.y *= gate_of<EXTRAS>(p, tok0, head, D, c + 1);
-            acc.z *= gate_of<EXTRAS>(p, tok0, head, D, c + 2);
-            acc.w *= gate_of<EXTRAS>(p, tok0, head, D, c + 3);
-          }
-          uint2 packed;
-          packed.x = pack_bf16(acc.x * inv, acc.y * inv);
-          packed.y = pack_bf16(acc.z * inv, acc.w * inv);
-          *reinterpret_cast<uint2*>(p.out + (size_t)tok0 * p.out_stride + (size_t)(kvh * g + r) * D + c) = packed;
-        }
-      }
-    }
+    finish_rows16<D, EXTRAS>(p, o_acc, m_run, l_run, reinterpret_cast<float*>(kv), warp, lane, row_start, row_end, tok0, g, kvh,
+                             split, my_splits);
   } else {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -686,6 +620,290 @@ attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p)
       }
     }
   }
+  // this grid is complete only when the one before it is: the next kernel waits for this one alone
+  if (p.late_wait) tl::pdl_wait();
+}
+
+// Decode: tiles of 16 packed rows whose keys and values arrive by TMA.  A fifth warp requests them, keys and values in
+// rings of their own (STAGES tiles each, a barrier for "landed" and one for "read by all four warps" a slot); the four
+// multiplying warps each take 16 of a tile's 64 keys and meet one another only at the end.  A warp multiplies the NEXT
+// tile's keys before this tile's softmax: the two chains (products; maximum, exponentials, sum) are independent, and
+// with one warp on a scheduler their latencies, and the instructions between them, are what a tile takes.  One CTA alone on an
+// SM: a tile of 64 keys of 128 in 0.77 us (pages of 16 tokens; 0.62 with pages of 64) against 1.28 with a block barrier a tile
+// and the request on a multiplying warp's path.  28 query heads on 4, 64 requests of 300 to 3,000 tokens: 72 -> 48 us (4.4 TB/s),
+// 64 of 4,096: 102 -> 89 (6.0 TB/s), 128 of 100 to 1,024: 52 -> 39, 24 of 210 to 2,100: 20.7 -> 16.2, 8 of 4,096: 18.5 -> 16.3;
+// 14 on 2 of 64, 128 of 200 to 2,048: 37 -> 28; one request of 300: 5.5 -> 5.7.
+constexpr int DECODE_THREADS = THREADS + 32;
+__host__ __device__ constexpr int decode_stages(int d) { return d == 128 ? 3 : 4; }
+__host__ __device__ constexpr int decode_ctas(int d) { return d == 128 ? 2 : 3; }  // resident an SM
+
+template <int D, bool EXTRAS>
+__global__ void __launch_bounds__(DECODE_THREADS, decode_ctas(D))
+attention_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
+  constexpr int STAGES = decode_stages(D);
+  constexpr int KSTEPS = D / 16, DTILES = D / 8, TILE = BLOCK_N * D;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  // the swizzle of the TMA copies works on address bits: the rings start on a 1024-byte boundary
+  __nv_bfloat16* k_ring = reinterpret_cast<__nv_bfloat16*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __nv_bfloat16* v_ring = k_ring + STAGES * TILE;
+  __nv_bfloat16* qs = v_ring + STAGES * TILE;  // [16][D]
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(qs + 16 * D);
+  uint64_t *v_full = k_full + STAGES, *k_read = k_full + 2 * STAGES, *v_read = k_full + 3 * STAGES;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(k_full + 4 * STAGES);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int req = p.tile_req ? p.tile_req[blockIdx.x] : blockIdx.x;
+  const int row_start = p.tile_row ? p.tile_row[blockIdx.x] : 0;
+  const int kvh = blockIdx.y, split = blockIdx.z;
+  const int g = p.nh / p.nkv;
+  const int tok0 = p.req_indptr[req];
+  const int q_len = p.req_indptr[req + 1] - tok0;
+  const int before = p.kv_before[req];
+  const int* table = p.block_table + (size_t)req * p.table_width;
+  const int row_end = min(q_len * g, row_start + 16);
+  if (row_start >= row_end) {
+    tl::pdl_wait();
+    return;
+  }
+  const int first_tok = row_start / g, last_tok = (row_end - 1) / g;
+  const int hi_key = before + last_tok;  // last key any row of the tile may see
+  const int lo_key = tl::first_key(before + first_tok, p.window);
+  int tile_begin = lo_key / BLOCK_N, tile_end = hi_key / BLOCK_N + 1;
+  int my_splits = 1;
+  if (p.splits > 1) {
+    my_splits = effective_splits(p.splits, tile_end - tile_begin);
+    if (split >= my_splits) {  // the request is too short to need this CTA
+      tl::pdl_wait();
+      return;
+    }
+    const int per = (tile_end - tile_begin + my_splits - 1) / my_splits;
+    tile_begin = tile_begin + split * per;
+    tile_end = min(tile_end, tile_begin + per);
+  }
+  const int num_tiles = max(0, tile_end - tile_begin);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2 * STAGES; ++i) tc::mbar_init(&k_full[i], 1);
+    for (int i = 0; i < 2 * STAGES; ++i) tc::mbar_init(&k_read[i], WARPS);
+    *abort_flag = 0;
+    tc::mbar_fence_init();
+  }
+  __syncthreads();
+
+  if (warp == WARPS) {
+    // ---- the requesting warp: one lane a page, whose keys (or values) of this head are one box [slab of 64][token].  Pages
+    // past the request's last key or past the table are read from page 0 (always there; their keys are masked and their
+    // value rows cleared before use).
+    const int pages_per_tile = BLOCK_N / p.page_size;
+    auto page_of = [&](const int t) {
+      const int index = (tile_begin + t) * pages_per_tile + lane;
+      return lane < pages_per_tile && t < num_tiles && index < p.table_width && index * p.page_size <= hi_key ? table[index] : 0;
+    };
+    // tiles that lie wholly before the step's own tokens were written by earlier steps and are requested before the wait.
+    // With late_wait the kernel before this one is the prompt portions' attention, which is independent of this one and
+    // whose every CTA had waited for this step's keys before this grid could start.
+    bool waited = p.late_wait;
+    auto request = [&](const int t, const int is_v, const int page) {
+      if (!waited && (tile_begin + t) * BLOCK_N + BLOCK_N - 1 >= before) {
+        tl::pdl_wait();
+        waited = true;
+      }
+      const int slot = t % STAGES;
+      uint64_t* full = (is_v ? v_full : k_full) + slot;
+      if (t >= STAGES) tc::mbar_wait((is_v ? v_read : k_read) + slot, (t / STAGES - 1) & 1, abort_flag, &g_error_word, 2);
+      if (lane == 0) tc::mbar_expect_tx(full, TILE * 2);
+      __syncwarp();
+      if (lane < pages_per_tile)
+        tc::tma_load_3d((is_v ? v_ring : k_ring) + slot * TILE + lane * p.page_size * D, &map_kv, full, 0,
+                        ((page * 2 + is_v) * p.nkv + kvh) * p.page_size, 0);
+      __syncwarp();
+    };
+    int page = page_of(0), page_next = page_of(1);
+    if (num_tiles > 0) request(0, 0, page);
+    for (int t = 0; t < num_tiles && !*abort_flag; ++t) {
+      const int page_after = page_of(t + 2);  // read a tile before it is needed
+      if (t + 1 < num_tiles) request(t + 1, 0, page_next);
+      request(t, 1, page);
+      page = page_next;
+      page_next = page_after;
+    }
+    if (!waited || p.late_wait) tl::pdl_wait();  // (no thread of the grid ends before the grids before it)
+    return;
+  }
+
+  // ---- q is written and visible after the wait
+  if (!p.late_wait) tl::pdl_wait();
+  tl::pdl_launch_dependents();  // the next kernel may start its own prologue
+  for (int i = threadIdx.x; i < 16 * (D / 8); i += THREADS) {  // zero for rows past the tile's end
+    const int r = i / (D / 8), c = i % (D / 8);
+    const int row = row_start + r;
+    const bool valid = row < row_end;
+    const __nv_bfloat16* src = p.q;
+    if (valid) src = p.q + (size_t)(tok0 + row / g) * p.q_stride + (size_t)(kvh * g + row % g) * D + c * 8;
+    cp_async_16(tile_at<D>(qs, r, c), src, valid);
+  }
+  cp_async_commit();
+  int row_pos[2], row_lo[2];  // the two rows this thread holds in accumulator fragments
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int row = row_start + (lane >> 2) + 8 * h;
+    row_pos[h] = row < row_end ? before + row / g : -1;  // -1: sees no key
+    row_lo[h] = row < row_end ? tl::first_key(row_pos[h], p.window) : 0;
+  }
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  float o_acc[DTILES][4];
+#pragma unroll
+  for (int i = 0; i < DTILES; ++i) o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f;
+  cp_async_wait<0>();
+  rows_barrier();
+  unsigned q_frag[KSTEPS][4];
+#pragma unroll
+  for (int ks = 0; ks < KSTEPS; ++ks)
+    ldmatrix_x4(q_frag[ks], tile_at<D>(qs, (lane & 7) + ((lane >> 3) & 1) * 8, 2 * ks + (lane >> 4)));
+
+  // A tile in a ring: page by page, slab by slab of 64 elements, rows of 128 bytes whose 16-byte pieces are xor-ed by the row.
+  const unsigned slab_bytes = p.page_size * 128;
+  auto row_at = [&](const int r) { return (unsigned)(r / p.page_size) * (p.page_size * D * 2) + (unsigned)(r % p.page_size) * 128; };
+  unsigned k_at[4], v_at[4];  // this lane's pieces of a tile's first slab, as ldmatrix wants them
+  {
+    const int kr = warp * 16 + (lane & 7) + (lane >> 4) * 8, vr = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      k_at[j] = tc::smem_addr(k_ring) + row_at(kr) + (((2 * j + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
+      v_at[j] = tc::smem_addr(v_ring) + row_at(vr) + (((2 * j + (lane >> 4)) ^ (lane & 7)) << 4);
+    }
+  }
+  // A slot of a ring and the parity of its "landed" barrier.
+  struct Turn {
+    int slot = 0;
+    unsigned parity = 0;
+    __device__ __forceinline__ void next() {
+      if (++slot == STAGES) slot = 0, parity ^= 1;
+    }
+  } kt, vt;
+
+  // S = Q K^T over this warp's 16 keys of the next tile; the odd k-steps add up on their own, which halves the chain
+  auto multiply_keys = [&](float (&s)[2][4]) {
+    tc::mbar_wait(&k_full[kt.slot], kt.parity, abort_flag, &g_error_word, 1);
+    const unsigned at = kt.slot * (TILE * 2);
+    float odd[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] = odd[i][e] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks) {
+      unsigned b[4];
+      ldmatrix_x4_at(b, k_at[ks & 3] + at + (ks >> 2) * slab_bytes);
+      mma_16816(ks & 1 ? odd[0] : s[0], q_frag[ks], b[0], b[1]);
+      mma_16816(ks & 1 ? odd[1] : s[1], q_frag[ks], b[2], b[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] += odd[i][e];
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&k_read[kt.slot]);
+    kt.next();
+  };
+
+  // keys below ``all_from`` or above ``all_to`` are not seen by every row of the tile
+  const int all_from = tl::first_key(hi_key, p.window), all_to = before + first_tok;
+  int key_first = tile_begin * BLOCK_N + warp * 16;  // first key this warp multiplies
+  // softmax and P V of one tile, whose scores are in s
+  auto finish_tile = [&](float (&s)[2][4]) {
+    // ---- mask, online softmax (float32)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (EXTRAS && p.cap_outer > 0.f) s[i][e] = capped_tanh(s[i][e] * p.cap_inner) * p.cap_outer;
+        else s[i][e] *= p.scale_log2;
+      }
+    if (key_first < all_from || key_first + 15 > all_to) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int key = key_first + i * 8 + (lane & 3) * 2 + (e & 1);
+          if (key > row_pos[e >> 1] || key < row_lo[e >> 1]) s[i][e] = -INFINITY;
+        }
+    }
+    float corr[2], m_use[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float top = fmaxf(fmaxf(s[0][2 * h], s[0][2 * h + 1]), fmaxf(s[1][2 * h], s[1][2 * h + 1]));
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+      const float m_new = fmaxf(m_run[h], top);
+      m_use[h] = m_new == -INFINITY ? 0.f : m_new;  // a row that has seen no key yet
+      corr[h] = exp2_fast(m_run[h] - m_use[h]);     // exp2(-inf) = 0 on the first tile
+      m_run[h] = m_new;
+    }
+    // (the sum stays this lane's own until the end: no shuffles in the loop)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] = exp2_fast(s[i][e] - m_use[e >> 1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      l_run[h] = fmaf(l_run[h], corr[h], (s[0][2 * h] + s[0][2 * h + 1]) + (s[1][2 * h] + s[1][2 * h + 1]));
+    const unsigned p_frag[4] = {pack_bf16(s[0][0], s[0][1]), pack_bf16(s[0][2], s[0][3]), pack_bf16(s[1][0], s[1][1]),
+                                pack_bf16(s[1][2], s[1][3])};
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {  // after the first tiles a new maximum is rare
+#pragma unroll
+      for (int i = 0; i < DTILES; ++i) {
+        o_acc[i][0] *= corr[0];
+        o_acc[i][1] *= corr[0];
+        o_acc[i][2] *= corr[1];
+        o_acc[i][3] *= corr[1];
+      }
+    }
+
+    // ---- O += P V over this warp's keys
+    tc::mbar_wait(&v_full[vt.slot], vt.parity, abort_flag, &g_error_word, 3);
+    const unsigned at = vt.slot * (TILE * 2);
+    // Whole pages were copied: value rows of keys outside [lo_key, hi_key] hold whatever the page held before (another
+    // request's values, page 0).  Their weights are exactly 0, but 0 x NaN is NaN, so the warp clears those of its own 16 rows.
+    if (key_first + 15 > hi_key || key_first < lo_key) {
+      for (int i = lane; i < 16 * (D / 8); i += 32) {
+        const int r = i / (D / 8), c = i % (D / 8);
+        if (key_first + r > hi_key || key_first + r < lo_key)
+          *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(v_ring) + at + row_at(warp * 16 + r) + (c >> 3) * slab_bytes +
+                                    (((c & 7) ^ (r & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // a later TMA copy may refill the slot
+      __syncwarp();
+    }
+#pragma unroll
+    for (int nb = 0; nb < DTILES / 2; ++nb) {
+      unsigned b[4];
+      ldmatrix_x4_trans_at(b, v_at[nb & 3] + at + (nb >> 2) * slab_bytes);
+      mma_16816(o_acc[2 * nb], p_frag, b[0], b[1]);
+      mma_16816(o_acc[2 * nb + 1], p_frag, b[2], b[3]);
+    }
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&v_read[vt.slot]);
+    vt.next();
+    key_first += BLOCK_N;
+  };
+  // two tiles a turn, so that the scores change places without copies
+  float s[2][4], s_next[2][4];
+  if (num_tiles > 0) multiply_keys(s);
+#pragma unroll 1
+  for (int t = 0; t < num_tiles; t += 2) {
+    if (t + 1 < num_tiles) multiply_keys(s_next);
+    finish_tile(s);
+    if (t + 1 >= num_tiles) break;
+    if (t + 2 < num_tiles) multiply_keys(s);
+    finish_tile(s_next);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
+    l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
+  }
+  finish_rows16<D, EXTRAS>(p, o_acc, m_run, l_run, reinterpret_cast<float*>(k_ring), warp, lane, row_start, row_end, tok0, g, kvh,
+                           split, my_splits);
   // this grid is complete only when the one before it is: the next kernel waits for this one alone
   if (p.late_wait) tl::pdl_wait();
 }
@@ -763,7 +981,7 @@ attention_combine_kernel(const float* __restrict__ part_acc, const float* __rest
   out[(size_t)token * out_stride + (size_t)head * D + c] = __float2bfloat16_rn(result);
 }
 
-// Tensor maps of cache layers [rows][D] with boxes of page_size x 64 elements, by base address.
+// Tensor maps of cache layers [rows][D] with boxes of D / 64 slabs x page_size rows x 64 elements, by base address.
 struct MapKey {
   const void* base;
   uint64_t rows;
@@ -783,7 +1001,7 @@ bool cached_map(CUtensorMap* out, const void* base, uint64_t rows, uint32_t cols
   auto it = cache.find(key);
   if (it == cache.end()) {
     CUtensorMap map;
-    if (!tc_host::make_map_bf16(&map, base, rows, cols, cols, box_rows)) return false;
+    if (!tc_host::make_map_bf16_slabs(&map, base, rows, cols, box_rows)) return false;
     if (cache.size() > 1024) cache.clear();
     it = cache.emplace(key, map).first;
   }
@@ -791,30 +1009,45 @@ bool cached_map(CUtensorMap* out, const void* base, uint64_t rows, uint32_t cols
   return true;
 }
 
-template <int D, bool ROWS16, bool TMA, int STAGES, bool EXTRAS>
-int launch(const CUtensorMap& map_kv, const Params& p, int tiles, cudaStream_t stream) {
+template <int D, bool ROWS16, bool EXTRAS>
+int launch(const Params& p, int tiles, cudaStream_t stream) {
   constexpr int BLOCK_M = ROWS16 ? 16 : 64;
-  // 16-row tiles: STAGES key/value stages and Q behind them; 64-row tiles: two stages, Q inside the second.
-  // TMA: room to start the stages on a 1024-byte boundary, the barriers and the abort word
-  constexpr int SMEM = ((ROWS16 ? STAGES : 2) * 2 * BLOCK_N * D + (ROWS16 ? BLOCK_M * D : 0)) * 2 + (TMA ? 1024 + 64 : 0);
+  // 16-row tiles: two key/value stages and Q behind them; 64-row tiles: Q inside the second
+  constexpr int SMEM = (2 * 2 * BLOCK_N * D + (ROWS16 ? BLOCK_M * D : 0)) * 2;
   static_assert(BLOCK_M * D <= 2 * BLOCK_N * D, "the Q rows fit one stage");
   static_assert(!ROWS16 || WARPS * 16 * (D + 2) * 4 <= 2 * 2 * BLOCK_N * D * 2, "merge buffer fits the stages");
-  static_assert((STAGES == 2 ? 3 : 2) * (SMEM + 1024) <= 227 * 1024, "three CTAs an SM with two stages, two with three");
+  static_assert(3 * (SMEM + 1024) <= 227 * 1024, "three CTAs an SM");
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(attention_mma_kernel<D, ROWS16, TMA, STAGES, EXTRAS>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t err = cudaFuncSetAttribute(attention_mma_kernel<D, ROWS16, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
-  dim3 grid(tiles, p.nkv, p.splits);
+  tl::launch_kernel_opt(ROWS16 && (tiles <= p.overlap_max_tiles || p.late_wait), attention_mma_kernel<D, ROWS16, EXTRAS>,
+                        dim3(tiles, p.nkv, p.splits), THREADS, SMEM, stream, p);
+  return TL_LAUNCH_CHECK();
+}
+
+template <int D, bool EXTRAS>
+int launch_decode(const CUtensorMap& map_kv, const Params& p, int tiles, cudaStream_t stream) {
+  constexpr int STAGES = decode_stages(D);
+  // the rings, Q, the barriers and the abort word, room to start on a 1024-byte boundary
+  constexpr int SMEM = (STAGES * 2 * BLOCK_N * D + 16 * D) * 2 + 4 * STAGES * 8 + 16 + 1024;
+  static_assert(WARPS * 16 * (D + 2) * 4 <= STAGES * 2 * BLOCK_N * D * 2, "merge buffer fits the rings");
+  static_assert(decode_ctas(D) * (SMEM + 1024) <= 228 * 1024, "the CTAs an SM is to hold");
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t err = cudaFuncSetAttribute(attention_decode_kernel<D, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (err != cudaSuccess) return (int)err;
+    configured = true;
+  }
   // Decode steps of up to 32 requests are launched overlapped with the preceding kernel:
   // the CTAs request their old key/value tiles while q is still being written.  Larger
   // grids are launched WITHOUT overlap: CTAs that start while the small kernel before them
   // still occupies the SMs are placed unevenly, and a bandwidth-bound grid's time is set by
   // its most loaded SM (measured: batch 64 decode lost 9% with an overlapped launch).
-  tl::launch_kernel_opt(ROWS16 && (tiles <= p.overlap_max_tiles || p.late_wait), attention_mma_kernel<D, ROWS16, TMA, STAGES, EXTRAS>, grid, THREADS,
-                        SMEM, stream, map_kv, p);
+  tl::launch_kernel_opt(tiles <= p.overlap_max_tiles || p.late_wait, attention_decode_kernel<D, EXTRAS>,
+                        dim3(tiles, p.nkv, p.splits), DECODE_THREADS, SMEM, stream, map_kv, p);
   return TL_LAUNCH_CHECK();
 }
 
@@ -828,41 +1061,15 @@ bool decode_tma_enabled() {
   return value == 1;
 }
 
-// TORCHLET_B200_DECODE_STAGES=2|3 forces the stage count of the TMA loader (for measurements).
-int decode_stages() {
-  static int value = -1;
-  if (value < 0) {
-    const char* v = getenv("TORCHLET_B200_DECODE_STAGES");
-    value = v ? atoi(v) : 0;
-    if (value != 2 && value != 3) value = 0;
-  }
-  return value;
-}
-
 template <int D, bool EXTRAS>
 int launch_for(const Params& p, long long num_pages, int tiles, bool rows16, cudaStream_t stream) {
+  if (!rows16) return launch<D, false, EXTRAS>(p, tiles, stream);
   CUtensorMap map_kv;
   memset(&map_kv, 0, sizeof(map_kv));
-  if (!rows16) return launch<D, false, false, 2, EXTRAS>(map_kv, p, tiles, stream);
   const bool tma = decode_tma_enabled() && num_pages > 0 && p.page_size >= 8 && p.page_size % 8 == 0 &&
                    BLOCK_N % p.page_size == 0 &&
                    cached_map(&map_kv, p.pages, (uint64_t)num_pages * 2 * p.nkv * p.page_size, D, (uint32_t)p.page_size);
-  if (!tma) return launch<D, true, false, 2, EXTRAS>(map_kv, p, tiles, stream);
-  // Without key splits (large batches) every CTA walks its request's whole context, and a third
-  // stage keeps more of it requested (batch 128 at 2,048 tokens: 7.15 -> 6.68 ms a decode step;
-  // batch 64: equal).  With splits the grid is sized for three CTAs an SM, which three stages do
-  // not leave room for (batch 8 to 32: 5-14 % slower).
-  // A grid of at most two CTAs an SM (batch 1 and 2) has the room as well: batch 1 -0.8 %.
-  static int sms = 0;
-  if (sms <= 0) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  const bool roomy = p.splits == 1 || (long long)tiles * p.nkv * p.splits <= 2ll * sms;
-  if (decode_stages() == 3 || (decode_stages() == 0 && roomy)) return launch<D, true, true, 3, EXTRAS>(map_kv, p, tiles, stream);
-  return launch<D, true, true, 2, EXTRAS>(map_kv, p, tiles, stream);
+  return tma ? launch_decode<D, EXTRAS>(map_kv, p, tiles, stream) : launch<D, true, EXTRAS>(p, tiles, stream);
 }
 
 }  // namespace
