@@ -117,6 +117,60 @@ def test_gla_kernels_carry_the_state(H, D, V, rank, tau):
         close(fin, plain_finish(plain_run(0, 9), slice(0, 9)), tol, "finish")
 
 
+@pytest.mark.parametrize("lens,H,D,V", [([64], 2, 64, 128), ([1], 1, 64, 128), ([130, 1, 64, 65, 15, 16, 17], 2, 64, 128),
+                                        ([100, 33], 2, 32, 64), ([77], 2, 60, 100), ([70, 9], 2, 12, 20), ([200], 1, 48, 256)])
+def test_gla_chunk_by_chunk(lens, H, D, V):
+    """Against the recurrence in float64, and no further from it than the scan (by a half at most: single sums of few terms
+    vary); requests below ``least`` and padding lanes leave state and output to the other kernel."""
+    from torchlet_b200 import ops
+
+    T, R, scale = sum(lens), len(lens), D ** -0.5
+    proj = rand(T, 2 * H * D + H * V + 4, seed=4).to(DEV)
+    decay = torch.sigmoid(rand(T, H * D, seed=5, scale=2.0)).pow(1 / 8.0).to(DEV)
+    start = rand(R + 1, H, D, V, seed=6).to(DEV)
+    indptr = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots = torch.arange(R, dtype=torch.int32, device=DEV)
+
+    def chunked(least, slots):
+        state, out = start.clone(), torch.full((T, H * V), float("nan"), device=DEV)
+        chunks = sum(-(-n // ops.gla_chunk_tokens()) for n in lens if n >= least)
+        workspace = torch.full((chunks * H * (D * V + 64),), float("nan"), device=DEV)
+        ops.gla_chunked(proj, decay, indptr, slots, state, out, workspace, R, chunks, least, H, D, V, scale)
+        return out, state
+
+    def scan(below):
+        state, out = start.clone(), torch.full((T, H * V), float("nan"), device=DEV)
+        ops.gla_scan(proj, decay, indptr, slots, state, out, R, H, D, V, scale, below=below)
+        return out, state
+
+    x, a = proj.double(), decay.double().view(T, H, D)
+    q, k, v = x[:, :H * D].view(T, H, D) * scale, x[:, H * D:2 * H * D].view(T, H, D), x[:, 2 * H * D:2 * H * D + H * V].view(T, H, V)
+    want, ends = [], []
+    for i in range(R):
+        S = start[i].double()
+        for t in range(int(indptr[i]), int(indptr[i + 1])):
+            S = a[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            want.append((q[t][:, None, :] @ S).reshape(1, H * V))
+        ends.append(S)
+    want, ends = torch.cat(want), torch.stack(ends)
+    error = lambda got, right: ((got.double() - right).norm() / right.norm()).item()
+    out, state = chunked(1, slots)
+    plain_out, plain_state = scan(None)
+    assert error(out, want) <= max(1.5 * error(plain_out, want), 1e-7)
+    assert error(state[:R], ends) <= max(1.5 * error(plain_state[:R], ends), 1e-7)
+    assert torch.equal(state[R], start[R])
+    # the two kernels side by side share the requests by length
+    some, some_state = chunked(33, slots)
+    rest, rest_state = scan(33)
+    for i, n in enumerate(lens):
+        rows = slice(int(indptr[i]), int(indptr[i + 1]))
+        mine, other = ((some, some_state), (rest, rest_state)) if n >= 33 else ((rest, rest_state), (some, some_state))
+        assert torch.equal(mine[0][rows], out[rows] if n >= 33 else plain_out[rows])
+        assert torch.isnan(other[0][rows]).all() and torch.equal(other[1][i], start[i])
+    padded, padded_state = chunked(1, torch.full_like(slots, -1))
+    assert (padded == 0).all() and torch.equal(padded_state, start)
+
+
 @pytest.mark.parametrize("H,D,V,requests", [(4, 64, 32, 1), (40, 64, 72, 2), (30, 128, 64, 8), (75, 32, 40, 4)])
 def test_gla_scan_blocks_kept_apart(H, D, V, requests):
     """Portions of 64 tokens and more take shared memory by how many blocks an SM has: one, two, four, more; the bits are

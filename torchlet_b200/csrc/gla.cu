@@ -155,7 +155,7 @@ template <int DK, bool VEC, int MODE, int COLS>
 __global__ void __launch_bounds__(lanes_a_column(DK) * COLS)
 gla_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ decay,
                 const int* __restrict__ req_indptr, const int* __restrict__ slots, float* __restrict__ state,
-                float* __restrict__ out, int heads, int qk_heads, int dim, int vdim, int max_slots, float qscale,
+                float* __restrict__ out, int heads, int qk_heads, int dim, int vdim, int below, int max_slots, float qscale,
                 const float* __restrict__ bonus, long long k_offset, long long v_offset) {
   tl::pdl_launch_dependents();
   tl::pdl_wait();
@@ -177,6 +177,7 @@ gla_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* __
   const int hv = heads * vdim;
   const int hq = h / (heads / qk_heads);  // the q/k head this head reads
   const int first = req_indptr[req], last = req_indptr[req + 1];
+  if (last - first >= below) return;  // its tokens are another kernel's
   const int slot = slots[req];
   const bool live = TL_DEBUG_OK(slot >= -1 && slot < max_slots, TL_DEBUG_SLOT, slot) && slot >= 0;
   if (!live) {  // a padding lane of a captured step: no state is touched
@@ -548,10 +549,10 @@ int tl_gla_decay(const float* proj, int proj_stride, int low_offset, const float
 }
 
 // state: float32 [max_slots, heads, dim, vdim]; out: float32 [tokens, heads * vdim].
-// tokens: of all requests.  decay_mode: 0 ``decay`` holds [tokens, heads * dim] rows, 1 one constant per head, 2 [tokens, heads] (one number per
+// tokens: of all requests; requests of ``below`` tokens and more are left out (gla_chunked.cu).  decay_mode: 0 ``decay`` holds [tokens, heads * dim] rows, 1 one constant per head, 2 [tokens, heads] (one number per
 // token and head), 3 rows and ``bonus`` [heads * dim].  k_offset, v_offset: how far k and v stand behind q.  qk_heads: how many heads q and k have (divides heads).
 int tl_gla_scan(const float* proj, int proj_stride, const float* decay, const int* req_indptr, const int* slots,
-                float* state, float* out, int requests, int heads, int qk_heads, int dim, int vdim, int tokens,
+                float* state, float* out, int requests, int heads, int qk_heads, int dim, int vdim, int tokens, int below,
                 int max_slots, float qscale, int decay_mode, const float* bonus, long long k_offset, long long v_offset,
                 cudaStream_t stream) {
   if (requests <= 0) return 0;
@@ -573,7 +574,7 @@ int tl_gla_scan(const float* proj, int proj_stride, const float* decay, const in
 #define TL_SCAN_ONE(DK, VEC, MODE, COLS)                                                                                   \
   scan_launch(gla_scan_kernel<DK, VEC, MODE, COLS>, dim3(requests, heads, (vdim + COLS - 1) / COLS),                       \
               lanes_a_column(DK) * COLS, long_walk, sms, sizeof(float) * STAGES * scan_chunk(DK, MODE) * scan_row(DK, MODE, COLS), \
-              stream, proj, proj_stride, decay, req_indptr, slots, state, out, heads, qk_heads, dim, vdim, max_slots,      \
+              stream, proj, proj_stride, decay, req_indptr, slots, state, out, heads, qk_heads, dim, vdim, below, max_slots, \
               qscale, bonus, k_offset, v_offset)
 #define TL_SCAN_MODE(DK, MODE)                                    \
   {                                                               \

@@ -155,10 +155,16 @@ _SIGNATURES = {
                                     c_void_p, c_int, c_void_p],
         "tl_latent_attention_mma_debug_error": [c_void_p],
     },
+    "gla_chunked": {
+        "tl_gla_chunk_tokens": [],
+        "tl_gla_chunked": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                           c_int, c_int, c_int, c_int, c_float, c_void_p],
+        "tl_gla_chunked_debug_error": [c_void_p],
+    },
     "gla": {
         "tl_gla_decay": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
         "tl_gla_scan": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                        c_int, c_int, c_int, c_float, c_int, c_void_p, c_longlong, c_longlong, c_void_p],
+                        c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_longlong, c_longlong, c_void_p],
         "tl_rotate_heads_f32": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "tl_gla_finish": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float,
                           c_void_p],
@@ -569,7 +575,7 @@ def gla_decay(proj, low_offset: int, w2t, bias, decay, rank: int, tau: float) ->
 
 def gla_scan(proj, decay, req_indptr, slots, state, out, requests: int, heads: int, dim: int, vdim: int,
              qscale: float, fixed_decay: bool = False, token_decay: bool = False, qk_heads: int | None = None,
-             bonus=None, k_offset: int | None = None, v_offset: int | None = None) -> None:
+             bonus=None, k_offset: int | None = None, v_offset: int | None = None, below: int | None = None) -> None:
     """Walks each request's tokens of the step through its slot's state [H, D, V] (float32):
     S = diag(decay) S + k v^T, out = S^T q * qscale; ``proj`` rows are [q (G D) | k (G D) | v (H V) | ...] with
     G = ``qk_heads`` (default H) heads of q and k, head h reading q/k head h // (H / G).
@@ -577,7 +583,7 @@ def gla_scan(proj, decay, req_indptr, slots, state, out, requests: int, heads: i
     (a retention), or with ``token_decay`` [tokens, H] (one number a token and head).  ``bonus`` (float32 [H, D], a decay
     per key channel only): out = (S_old + diag(bonus) k v^T)^T q instead.  ``k_offset``, ``v_offset``: where k and v stand
     behind q, in numbers (default: the row layout above), so that the three may lie in planes of their own.
-    A request whose slot is negative is padding."""
+    A request whose slot is negative is padding; requests of ``below`` tokens and more are left out."""
     _need_cuda(proj, decay, req_indptr, slots, state, out, bonus)
     assert bonus is None or (bonus.dtype == torch.float32 and bonus.is_contiguous() and bonus.numel() == heads * dim
                              and not fixed_decay and not token_decay)
@@ -589,10 +595,33 @@ def gla_scan(proj, decay, req_indptr, slots, state, out, requests: int, heads: i
     assert state.shape[1:] == (heads, dim, vdim) and req_indptr.dtype == slots.dtype == torch.int32
     code = _fn("gla", "tl_gla_scan")(proj.data_ptr(), proj.stride(0), decay.data_ptr(), req_indptr.data_ptr(),
                                      slots.data_ptr(), state.data_ptr(), out.data_ptr(), requests, heads, qk_heads, dim,
-                                     vdim, out.shape[0], state.shape[0], float(qscale), 1 if fixed_decay else (2 if token_decay else (3 if bonus is not None else 0)),
+                                     vdim, out.shape[0], (1 << 30) if below is None else int(below), state.shape[0],
+                                     float(qscale), 1 if fixed_decay else (2 if token_decay else (3 if bonus is not None else 0)),
                                      _ptr(bonus), qk_heads * dim if k_offset is None else int(k_offset),
                                      2 * qk_heads * dim if v_offset is None else int(v_offset), _stream())
     _check(code, "gla_scan")
+
+
+def gla_chunk_tokens() -> int:
+    """Tokens a chunk of ``gla_chunked`` has."""
+    return _fn("gla_chunked", "tl_gla_chunk_tokens")()
+
+
+def gla_chunked(proj, decay, req_indptr, slots, state, out, workspace, requests: int, chunks: int, least: int, heads: int,
+                dim: int, vdim: int, qscale: float) -> None:
+    """``gla_scan`` (a decay per key channel, rows [q | k | v | ...]) for the requests of at least ``least`` tokens, all chunks of
+    ``gla_chunk_tokens()`` tokens at once (csrc/gla_chunked.cu); the other requests' rows and states stay as they are.
+    ``chunks``: how many these requests have in all; ``workspace``: float32, chunks * heads * (dim * vdim + 64) numbers."""
+    _need_cuda(proj, decay, req_indptr, slots, state, out, workspace)
+    assert proj.dtype == decay.dtype == state.dtype == out.dtype == workspace.dtype == torch.float32
+    assert state.is_contiguous() and out.is_contiguous() and decay.is_contiguous() and workspace.is_contiguous()
+    assert proj.stride(1) == 1 and proj.shape[1] >= heads * (2 * dim + vdim) and decay.numel() == proj.shape[0] * heads * dim
+    assert out.numel() == proj.shape[0] * heads * vdim and workspace.numel() >= chunks * heads * (dim * vdim + 64)
+    assert state.shape[1:] == (heads, dim, vdim) and req_indptr.dtype == slots.dtype == torch.int32
+    code = _fn("gla_chunked", "tl_gla_chunked")(proj.data_ptr(), proj.stride(0), decay.data_ptr(), req_indptr.data_ptr(),
+                                                slots.data_ptr(), state.data_ptr(), out.data_ptr(), workspace.data_ptr(), requests,
+                                                chunks, least, heads, dim, vdim, state.shape[0], float(qscale), _stream())
+    _check(code, "gla_chunked", 3)
 
 
 def rotate_heads_f32(rows, positions, inv_freq, heads: int, dim: int, dims: int) -> None:
@@ -1705,7 +1734,7 @@ def debug_errors() -> list:
     in the ordinary build (``TORCHLET_B200_DEBUG`` unset), whose kernels carry no checks."""
     found = []
     for library in ("elementwise", "attention_generic", "attention_mma", "decode_fused", "slots", "stream_ops",
-                    "delta_rule", "latent_attention", "latent_attention_mma", "gla", "gated_attention", "hyper",
+                    "delta_rule", "latent_attention", "latent_attention_mma", "gla", "gla_chunked", "gated_attention", "hyper",
                     "pooled_attention", "ssm", "time_mixing", "token_shift", "qkv_prepare", "token_embed",
                     "attention_mixed_decode"):
         if any(name in _functions for name in _SIGNATURES[library]):

@@ -17,12 +17,20 @@ a2.b [H D]; norm [V]; o [hidden, H V].
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from .. import ops
 from ..config.spec import PartSpec
 from .base import MIXERS, Mixer, StateSpec, TensorSpec
 from .linear import Linear
+
+
+# Tokens from which on a request's portion goes chunk by chunk in the bfloat16 engine (csrc/gla_chunked.cu): few tokens are
+# through the scan before three kernels have ended (16 heads of 64 x 128, one request: 128 tokens 21 us against 33, 256 38
+# against 36, 2,048 275 against 76), many keep all SMs at work (4 x 128: 41 against 37; 32 x 64: 128 against 85; but 64 x 32:
+# 137 against 136, 128 x 16: 159 against 343).
+LEAST_ALONE, LEAST_OF_MANY, MANY = 192, 64, 1024
 
 
 @MIXERS.register("gated_linear_attention")
@@ -69,6 +77,20 @@ class GatedLinearAttention(Mixer):
         self.a2_bias, self.norm_weight = f32("a2.b"), f32("norm")
         self.a2 = f32("a2").t().contiguous()  # [rank, H D]: the threads of a block read consecutive entries
 
+    def _chunked(self, ctx, proj) -> tuple:
+        """(chunks of the requests whose portions go chunk by chunk, the fewest tokens of one, whether other requests are in
+        the step).  Only in the bfloat16 engine: the float32 engine's numbers do not depend on how a sequence is cut."""
+        if (ctx.decode_only or ctx.dtype != torch.bfloat16 or self.head_dim > 64 or self.head_dim % 4 or self.v_dim % 4
+                or proj.stride(0) % 4):
+            return 0, 0, True
+        plan = ctx.plans.get("gla_chunked")
+        if plan is None:
+            lengths = np.diff(ctx.req_indptr_host)
+            least = LEAST_OF_MANY if lengths[lengths >= LEAST_OF_MANY].sum() >= MANY else LEAST_ALONE
+            long = lengths[lengths >= least]
+            plan = ctx.plans["gla_chunked"] = (int((-(-long // ops.gla_chunk_tokens())).sum()), least, long.size < lengths.size)
+        return plan
+
     def forward(self, ctx, x, acc, cache) -> None:
         tokens, H, D, V = x.shape[0], self.num_heads, self.head_dim, self.v_dim
         proj = ctx.buffer("gla.proj", (tokens, 2 * self.k_size + 2 * self.v_size + self.rank), torch.float32)
@@ -76,7 +98,15 @@ class GatedLinearAttention(Mixer):
         decay = ctx.buffer("gla.decay", (tokens, self.k_size), torch.float32)
         ops.gla_decay(proj, 2 * self.k_size + 2 * self.v_size, self.a2, self.a2_bias, decay, self.rank, self.tau)
         o = ctx.buffer("gla.o", (tokens, self.v_size), torch.float32)
-        ops.gla_scan(proj, decay, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D, V, D ** -0.5)
+        chunks, least, others = self._chunked(ctx, proj)
+        if others:
+            ops.gla_scan(proj, decay, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D, V, D ** -0.5,
+                         below=least if chunks else None)
+        if chunks:
+            length = ops.gla_chunk_tokens()
+            workspace = ctx.buffer("gla.chunks", (chunks * length, -(-H * (D * V + 64) // length)), torch.float32)
+            ops.gla_chunked(proj, decay, ctx.req_indptr, ctx.slots, cache.state, o, workspace, ctx.num_requests, chunks,
+                            least, H, D, V, D ** -0.5)
         out = ctx.buffer("gla.out", (tokens, self.v_size), ctx.dtype)
         ops.gla_finish(o, proj, 2 * self.k_size + self.v_size, self.norm_weight, out, H, V, self.eps)
         if not self.o_proj.accumulate_later(ctx, out, acc):
