@@ -357,10 +357,11 @@ template <int TILE_M, int TILE_N> constexpr int TILE_SMEM = 2 * TILE_K * (TILE_M
 
 // A thread's outputs: rows 4 ty + {0..3} and TILE_M / 2 + 4 ty + {0..3}, columns 4 tx + {0..3} and (TC 8)
 // TILE_N / 2 + 4 tx + {0..3}, so that a quarter warp's 16-byte reads lie side by side.
-template <int TILE_M, int TILE_N, int TC, int CLUSTER>
+// BESIDE: the tiles from number ``whole`` on of a product whose others are the launch just before; else those below it.
+template <int TILE_M, int TILE_N, int TC, int CLUSTER, bool BESIDE>
 __global__ void __launch_bounds__(TILE_THREADS<TILE_M, TILE_N, TC>, (TC == 8 ? 256 : 512) / TILE_THREADS<TILE_M, TILE_N, TC>)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                     float* __restrict__ out, int M, int N, int K, int ldx, int ldw, int ldo, int accum) {
+                     float* __restrict__ out, int M, int N, int K, int ldx, int ldw, int ldo, int accum, int whole) {
   constexpr int NT = TILE_THREADS<TILE_M, TILE_N, TC>;
   constexpr int XS = TILE_M + 4, WS = TILE_N + 4;
   constexpr int STAGE = TILE_K * (XS + WS);
@@ -370,11 +371,21 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
   const int tid = threadIdx.x;
   const int tx = tid % (TILE_N / TC), ty = tid / (TILE_N / TC);
   const int rank = CLUSTER > 1 ? (int)cluster_rank() : 0;
-  const int m0 = blockIdx.y * TILE_M, n0 = (int)(blockIdx.x / CLUSTER) * TILE_N;
+  int m0 = blockIdx.y * TILE_M, n0 = (int)(blockIdx.x / CLUSTER) * TILE_N;
+  if constexpr (BESIDE) {
+    const int tile = whole + (int)(blockIdx.x / CLUSTER), across = (N + TILE_N - 1) / TILE_N;
+    m0 = tile / across * TILE_M;
+    n0 = tile % across * TILE_N;
+  } else if (CLUSTER == 1 && (int)(blockIdx.y * gridDim.x + blockIdx.x) >= whole) {
+    return;  // another launch's tile
+  }
   const int piece = piece_length(K);
   const int k_begin = CLUSTER > 1 ? min(K, rank * 4 * piece) : 0;
   const int k_end = CLUSTER > 1 ? min(K, k_begin + 4 * piece) : K;
-  tl::pdl_wait();               // everything before us in the stream is complete and visible
+  // Everything before us in the stream is complete and visible after the wait.  The launch just before a BESIDE one is the same
+  // product's other tiles, of which this one reads nothing and every block of which has waited, or left, before this grid
+  // could start; the wait moves to the end.
+  if (!BESIDE) tl::pdl_wait();
   tl::pdl_launch_dependents();  // the next kernel may start its own prologue
 
   float4 xr[X4], wr[W4];
@@ -503,6 +514,7 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
     put(out + (size_t)(m0 + r) * ldo + n0 + c, bias, accum, n0 + c, v);
   }
   if (CLUSTER > 1) cluster_sync();  // nobody leaves while a peer may still read its memory
+  if (BESIDE) tl::pdl_wait();
 }
 
 template <int CLUSTER, typename Kernel, typename... Args>
@@ -573,12 +585,19 @@ int launch_tiles(const float* x, const float* w, const float* bias, float* out, 
   const int across = (N + TILE_N - 1) / TILE_N, down = (M + TILE_M - 1) / TILE_M;
   const long long blocks = (long long)across * down, room = resident<TILE_M, TILE_N, TC>();
   constexpr int NT = TILE_THREADS<TILE_M, TILE_N, TC>;
-  static bool configured[2] = {false, false};
+  static bool configured[3] = {false, false, false};
   if ((K > 160 && 4 * blocks <= room) || (K >= 512 && blocks < room))
-    return launch_clusters<4>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 4>, configured[1], dim3(4 * across, down), NT,
-                              TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
-  return launch_clusters<1>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 1>, configured[0], dim3(across, down), NT,
-                            TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum);
+    return launch_clusters<4>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 4, false>, configured[1], dim3(4 * across, down), NT,
+                              TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum, (int)blocks);
+  // A last wave that is nearly empty takes as long as a full one: its tiles go to four blocks each, which start beside the
+  // blocks that are still at work.  (K x N 896 x 9728: 509 rows, 608 tiles for 296 blocks, 249 -> 212 us; 256 rows 159 -> 119;
+  // 3584 x 3584, 700 rows: 614 -> 494.)
+  const long long rest = blocks % room, whole = K >= 512 && blocks > room && 4 * rest <= room ? blocks - rest : blocks;
+  const int rc = launch_clusters<1>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 1, false>, configured[0], dim3(across, down), NT,
+                                    TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum, (int)whole);
+  if (rc || whole == blocks) return rc;
+  return launch_clusters<4>(gemm_f32_tile_kernel<TILE_M, TILE_N, TC, 4, true>, configured[2], dim3(4 * (unsigned)rest), NT,
+                            TILE_SMEM<TILE_M, TILE_N>, stream, x, w, bias, out, M, N, K, ldx, ldw, ldo, accum, (int)whole);
 }
 
 int launch_f32(const float* x, const float* w, const float* bias, float* out, int accum, int M, int N, int K, int ldx,
