@@ -201,6 +201,67 @@ def test_delta_scan_blocks_kept_apart(H, D, requests):
         assert torch.equal(again[r], state[r])
 
 
+@pytest.mark.parametrize("lens,H,D,rank,pad", [([8], 1, 64, 16, 0), ([37, 9, 1, 8, 16, 100], 2, 64, 16, 0), ([37, 3], 2, 24, 5, 0),
+                                               ([50, 2, 41], 3, 40, 7, 0), ([23], 1, 4, 2, 0), ([300], 2, 64, 64, 3)])
+def test_delta_rule_chunk_by_chunk(lens, H, D, rank, pad):
+    """Against the recurrence in float64, and no further from it than the token-wise kernels (by a half at most: single
+    sums of few terms vary); requests below ``least`` and padding lanes leave state and output to the other kernel."""
+    from torchlet_b200 import ops
+
+    size, T, R = H * D, sum(lens), len(lens)
+    proj = rand(T, 5 * size + rank + pad, seed=1).to(DEV)[:, :5 * size + rank]
+    w2, w0, bias = rand(rank, size, seed=2, scale=rank ** -0.5).to(DEV), rand(size, seed=3).to(DEV), rand(size, seed=4).to(DEV)
+    start = rand(R + 1, H, D, D, seed=5, scale=0.3).to(DEV)
+    indptr = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots = torch.arange(R, dtype=torch.int32, device=DEV)
+
+    def chunked(least, slots):
+        state, out = start.clone(), torch.full((T, size), float("nan"), device=DEV)
+        chunks = sum(-(-n // ops.delta_chunk_tokens()) for n in lens if n >= least)
+        records = torch.full((chunks * H * ops.delta_chunk_record(),), float("nan"), device=DEV)
+        ops.delta_chunked(proj, w2, w0, bias, indptr, slots, state, out, records, R, chunks, least, H, D, rank)
+        return out, state
+
+    def token_wise(below):
+        state, out = start.clone(), torch.full((T, size), float("nan"), device=DEV)
+        gates = torch.empty(T, H * 3 * D, device=DEV)
+        ops.delta_prepare(proj, w2, w0, bias, gates, H, D, rank)
+        ops.delta_scan(proj, gates, indptr, slots, state, out, R, H, D, below=below)
+        return out, state
+
+    x = proj.double()
+    r, k, v = (x[:, i * size:(i + 1) * size].view(T, H, D) for i in range(3))
+    a = torch.sigmoid(x[:, 4 * size:5 * size] + bias.double()).view(T, H, D)
+    inner = torch.tanh(x[:, 5 * size:5 * size + rank]) @ w2.double() + w0.double()
+    w = torch.exp(-math.exp(-0.5) * torch.sigmoid(inner)).view(T, H, D)
+    u = k / torch.sqrt(k.pow(2).sum(-1, keepdim=True) + 1e-6)
+    want, ends = [], []
+    for q in range(R):
+        S = start[q].double()
+        for t in range(int(indptr[q]), int(indptr[q + 1])):
+            seen = u[t][:, None, :] @ S
+            S = w[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :] - (a[t] * u[t])[:, :, None] * seen
+            want.append((r[t][:, None, :] @ S).reshape(1, size))
+        ends.append(S)
+    want, ends = torch.cat(want), torch.stack(ends)
+    error = lambda got, right: ((got.double() - right).norm() / right.norm()).item()
+    out, state = chunked(1, slots)
+    plain_out, plain_state = token_wise(None)
+    assert error(out, want) <= max(1.5 * error(plain_out, want), 1e-7)
+    assert error(state[:R], ends) <= max(1.5 * error(plain_state[:R], ends), 1e-7)
+    assert torch.equal(state[R], start[R])
+    # the two kernels side by side share the requests by length
+    some, some_state = chunked(9, slots)
+    rest, rest_state = token_wise(9)
+    for q, n in enumerate(lens):
+        rows = slice(int(indptr[q]), int(indptr[q + 1]))
+        mine, other = ((some, some_state), (rest, rest_state)) if n >= 9 else ((rest, rest_state), (some, some_state))
+        assert torch.equal(mine[0][rows], out[rows] if n >= 9 else plain_out[rows])
+        assert torch.isnan(other[0][rows]).all() and torch.equal(other[1][q], start[q])
+    padded, padded_state = chunked(1, torch.full_like(slots, -1))
+    assert (padded == 0).all() and torch.equal(padded_state, start)
+
+
 @pytest.mark.parametrize("T,H,N,K,gap", [(1, 1, 8, 64, 0), (129, 3, 72, 64, 8), (300, 4, 256, 192, 0), (257, 5, 520, 128, 24)])
 def test_products_by_heads_in_one_launch(T, H, N, K, gap):
     """Against float64 within the rounding of the bfloat16 result; columns between the heads' stay as they were."""

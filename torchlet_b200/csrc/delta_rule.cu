@@ -122,7 +122,7 @@ template <int DK, bool VEC, int COLS, bool LONG>
 __global__ void __launch_bounds__(COLS * KS / (COLS == DK ? 2 : 1))
 delta_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ gates,
                   const int* __restrict__ req_indptr, const int* __restrict__ slots, float* __restrict__ state,
-                  float* __restrict__ out, int heads, int dim, int max_slots) {
+                  float* __restrict__ out, int heads, int dim, int below, int max_slots) {
   tl::pdl_launch_dependents();
   tl::pdl_wait();
   constexpr int CPL = COLS == DK ? 2 : 1;  // columns a lane serves
@@ -141,6 +141,7 @@ delta_scan_kernel(const float* __restrict__ proj, int proj_stride, const float* 
   }
   const int hd = heads * dim;
   const int first = req_indptr[req], last = req_indptr[req + 1];
+  if (last - first >= below) return;  // its tokens are another kernel's
   const int slot = slots[req];
   const bool live = TL_DEBUG_OK(slot >= -1 && slot < max_slots, TL_DEBUG_SLOT, slot) && slot >= 0;
   if (!live) {  // a padding lane of a captured step: no state is touched
@@ -387,9 +388,11 @@ int tl_delta_prepare(const float* proj, int proj_stride, const float* w2t, const
   return TL_LAUNCH_CHECK();
 }
 
-// state: float32 [max_slots, heads, dim, dim]; out: float32 [tokens, heads * dim]; tokens: of all requests.
+// state: float32 [max_slots, heads, dim, dim]; out: float32 [tokens, heads * dim]; tokens: of all requests;
+// requests of ``below`` tokens and more are left out (delta_chunked.cu).
 int tl_delta_scan(const float* proj, int proj_stride, const float* gates, const int* req_indptr, const int* slots,
-                  float* state, float* out, int requests, int heads, int dim, int tokens, int max_slots, cudaStream_t stream) {
+                  float* state, float* out, int requests, int heads, int dim, int tokens, int below,
+                  int max_slots, cudaStream_t stream) {
   if (requests <= 0) return 0;
   if (dim <= 0 || dim > 256 || heads > 65535) return TL_ERR_UNSUPPORTED;
   dim3 grid(requests, heads);
@@ -401,7 +404,7 @@ int tl_delta_scan(const float* proj, int proj_stride, const float* gates, const 
   const bool long_portions = vec && (dim > 128 || tokens >= (dim > 64 ? 4ll : 8ll) * requests);
 #define TL_SCAN_INSTANCE(DK, VEC, COLS, LONG)                                                                       \
   scan_launch(delta_scan_kernel<DK, VEC, COLS, LONG>, grid, COLS * KS / (COLS == DK ? 2 : 1), long_walk,             \
-              sizeof(float) * 2 * scan_chunk(DK) * 6 * DK, stream, proj, proj_stride, gates, req_indptr, slots, state, out, heads, dim, max_slots)
+              sizeof(float) * 2 * scan_chunk(DK) * 6 * DK, stream, proj, proj_stride, gates, req_indptr, slots, state, out, heads, dim, below, max_slots)
 #define TL_SCAN_COLS(DK, COLS)                          \
   if (long_portions) TL_SCAN_INSTANCE(DK, true, COLS, true);    \
   else if (vec) TL_SCAN_INSTANCE(DK, true, COLS, (DK > 128)); \

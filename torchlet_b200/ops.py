@@ -131,7 +131,7 @@ _SIGNATURES = {
     "delta_rule": {
         "tl_delta_prepare": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_void_p],
-        "tl_delta_scan": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+        "tl_delta_scan": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_int, c_int, c_void_p],
         "tl_delta_finish": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
                             c_void_p],
@@ -154,6 +154,13 @@ _SIGNATURES = {
                                     c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
                                     c_void_p, c_int, c_void_p],
         "tl_latent_attention_mma_debug_error": [c_void_p],
+    },
+    "delta_chunked": {
+        "tl_delta_chunk_tokens": [],
+        "tl_delta_chunk_record": [],
+        "tl_delta_chunked": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+        "tl_delta_chunked_debug_error": [c_void_p],
     },
     "gla_chunked": {
         "tl_gla_chunk_tokens": [],
@@ -535,16 +542,46 @@ def delta_prepare(proj, w2, w0, a_bias, gates, heads: int, dim: int, rank: int) 
     _check(code, "delta_prepare")
 
 
-def delta_scan(proj, gates, req_indptr, slots, state, out, requests: int, heads: int, dim: int) -> None:
+def delta_scan(proj, gates, req_indptr, slots, state, out, requests: int, heads: int, dim: int, below: int | None = None) -> None:
     """Walks each request's tokens of the step through its slot's state [H, D, D] (float32);
-    ``out`` float32 [T, H D] receives S_t^T r_t.  A request whose slot is negative is padding."""
+    ``out`` float32 [T, H D] receives S_t^T r_t.  A request whose slot is negative is padding; requests of ``below`` tokens
+    and more are left out."""
     _need_cuda(proj, gates, req_indptr, slots, state, out)
     assert state.dtype == out.dtype == torch.float32 and state.is_contiguous() and out.is_contiguous()
     assert state.shape[1:] == (heads, dim, dim) and req_indptr.dtype == slots.dtype == torch.int32
     code = _fn("delta_rule", "tl_delta_scan")(proj.data_ptr(), proj.stride(0), gates.data_ptr(), req_indptr.data_ptr(),
                                               slots.data_ptr(), state.data_ptr(), out.data_ptr(), requests, heads, dim,
-                                              out.shape[0], state.shape[0], _stream())
+                                              out.shape[0], (1 << 30) if below is None else int(below), state.shape[0], _stream())
     _check(code, "delta_scan")
+
+
+def delta_chunk_tokens() -> int:
+    """Tokens a chunk of ``delta_chunked`` has."""
+    return _fn("delta_chunked", "tl_delta_chunk_tokens")()
+
+
+def delta_chunk_record() -> int:
+    """Float32 numbers of a (chunk, head) in ``delta_chunked``'s records."""
+    return _fn("delta_chunked", "tl_delta_chunk_record")()
+
+
+def delta_chunked(proj, w2, w0, a_bias, req_indptr, slots, state, out, records, requests: int, chunks: int, least: int,
+                  heads: int, dim: int, rank: int) -> None:
+    """``delta_prepare`` and ``delta_scan`` for the requests of at least ``least`` tokens, ``delta_chunk_tokens()`` tokens a step
+    of the recurrence (csrc/delta_chunked.cu); the other requests' rows and states stay as they are.  ``chunks``: how many
+    these requests have in all; ``records``: float32, chunks * heads * delta_chunk_record() numbers."""
+    _need_cuda(proj, w2, w0, a_bias, req_indptr, slots, state, out, records)
+    assert proj.dtype == w2.dtype == w0.dtype == a_bias.dtype == state.dtype == out.dtype == records.dtype == torch.float32
+    assert proj.stride(1) == 1 and proj.shape[1] == 5 * heads * dim + rank and w2.is_contiguous() and w2.shape == (rank, heads * dim)
+    assert w0.is_contiguous() and a_bias.is_contiguous() and w0.numel() == a_bias.numel() == heads * dim
+    assert state.is_contiguous() and out.is_contiguous() and records.is_contiguous()
+    assert out.numel() == proj.shape[0] * heads * dim and records.numel() >= chunks * heads * delta_chunk_record()
+    assert state.shape[1:] == (heads, dim, dim) and req_indptr.dtype == slots.dtype == torch.int32
+    code = _fn("delta_chunked", "tl_delta_chunked")(proj.data_ptr(), proj.stride(0), w2.data_ptr(), w0.data_ptr(), a_bias.data_ptr(),
+                                                    req_indptr.data_ptr(), slots.data_ptr(), state.data_ptr(), out.data_ptr(),
+                                                    records.data_ptr(), requests, chunks, least, heads, dim, rank, state.shape[0],
+                                                    _stream())
+    _check(code, "delta_chunked", 2)
 
 
 def delta_finish(o, proj, weight, out, heads: int, dim: int, eps: float) -> None:
@@ -1734,7 +1771,7 @@ def debug_errors() -> list:
     in the ordinary build (``TORCHLET_B200_DEBUG`` unset), whose kernels carry no checks."""
     found = []
     for library in ("elementwise", "attention_generic", "attention_mma", "decode_fused", "slots", "stream_ops",
-                    "delta_rule", "latent_attention", "latent_attention_mma", "gla", "gla_chunked", "gated_attention", "hyper",
+                    "delta_rule", "delta_chunked", "latent_attention", "latent_attention_mma", "gla", "gla_chunked", "gated_attention", "hyper",
                     "pooled_attention", "ssm", "time_mixing", "token_shift", "qkv_prepare", "token_embed",
                     "attention_mixed_decode"):
         if any(name in _functions for name in _SIGNATURES[library]):

@@ -17,12 +17,27 @@ o [hidden, H D].
 """
 from __future__ import annotations
 
+import functools
+
+import numpy as np
 import torch
 
 from .. import ops
 from ..config.spec import PartSpec
 from .base import MIXERS, Mixer, StateSpec, TensorSpec
 from .linear import Linear
+
+
+# Tokens from which on a request's portion goes chunk by chunk in the bfloat16 engine (csrc/delta_chunked.cu), and how many
+# blocks of 16 columns an SM at most: the chunks shorten a chain that waits; where blocks enough are there to fill its waits,
+# their larger preparation costs more (32 heads of 64: 1 request of 32 tokens 22 -> 18 us, of 2,048 429 -> 286; 4 of 64
+# 41 -> 37, of 128 61 -> 64, of 512 236 -> 252; 32 of 64 183 -> 245).
+LEAST_CHUNKED, BLOCKS_AN_SM, COLUMNS = 32, 2, 16
+
+
+@functools.lru_cache(maxsize=None)
+def _sm_count(device_index: int) -> int:
+    return torch.cuda.get_device_properties(device_index).multi_processor_count
 
 
 @MIXERS.register("general_delta")
@@ -65,14 +80,37 @@ class GeneralDeltaMixer(Mixer):
         self.w0, self.a_bias, self.norm_weight = f32("w0"), f32("a.b"), f32("norm")
         self.w2 = f32("w2").t().contiguous()  # [rank, H D]: the threads of a block read consecutive entries
 
+    def _chunked(self, ctx) -> tuple:
+        """(chunks of the requests whose portions go chunk by chunk, whether other requests are in the step).  Only in the
+        bfloat16 engine: the float32 engine's numbers do not depend on how a sequence is cut."""
+        if ctx.decode_only or ctx.dtype != torch.bfloat16 or self.head_dim > 64 or self.head_dim % 4:
+            return 0, True
+        key = ("delta_chunked", self.num_heads, self.head_dim)
+        plan = ctx.plans.get(key)
+        if plan is None:
+            lengths = np.diff(ctx.req_indptr_host)
+            long = lengths[lengths >= LEAST_CHUNKED]
+            if long.size * self.num_heads * -(-self.head_dim // COLUMNS) > BLOCKS_AN_SM * _sm_count(torch.cuda.current_device()):
+                long = long[:0]
+            plan = ctx.plans[key] = (int((-(-long // ops.delta_chunk_tokens())).sum()), long.size < lengths.size)
+        return plan
+
     def forward(self, ctx, x, acc, cache) -> None:
         tokens, H, D = x.shape[0], self.num_heads, self.head_dim
         proj = ctx.buffer("delta.proj", (tokens, 5 * self.size + self.rank), torch.float32)
         self.in_proj.forward(x, proj)
-        gates = ctx.buffer("delta.gates", (tokens, H * 3 * D), torch.float32)
-        ops.delta_prepare(proj, self.w2, self.w0, self.a_bias, gates, H, D, self.rank)
         o = ctx.buffer("delta.o", (tokens, self.size), torch.float32)
-        ops.delta_scan(proj, gates, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D)
+        chunks, others = self._chunked(ctx)
+        if others:
+            gates = ctx.buffer("delta.gates", (tokens, H * 3 * D), torch.float32)
+            ops.delta_prepare(proj, self.w2, self.w0, self.a_bias, gates, H, D, self.rank)
+            ops.delta_scan(proj, gates, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D,
+                           below=LEAST_CHUNKED if chunks else None)
+        if chunks:
+            length = ops.delta_chunk_tokens()
+            records = ctx.buffer("delta.records", (chunks * length, H * ops.delta_chunk_record() // length), torch.float32)
+            ops.delta_chunked(proj, self.w2, self.w0, self.a_bias, ctx.req_indptr, ctx.slots, cache.state, o, records,
+                              ctx.num_requests, chunks, LEAST_CHUNKED, H, D, self.rank)
         out = ctx.buffer("delta.out", (tokens, self.size), ctx.dtype)
         ops.delta_finish(o, proj, self.norm_weight, out, H, D, self.eps)
         if not self.o_proj.accumulate_later(ctx, out, acc):
