@@ -31,56 +31,59 @@ constexpr float DECAY_RATE = 0.6065306597126334f;  // exp(-1/2)
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 
-constexpr int PREP_TOKENS = 8;  // tokens a block of the prepare kernel takes: a W2 entry is read once for all
+// Tokens a block of the prepare kernel takes: eight, so that a W2 entry is read once for all, or one where the grid of eights
+// would leave most SMs idle (8 tokens, 32 heads of 64, in a decode step: 20.4 -> 6.8 us; the bits
+// are the same).
+constexpr int PREP_TOKENS = 8;
 
 // w2t: W2 transposed, [rank, heads * dim], so that the threads of a block read consecutive entries.
-template <int NT>
+template <int NT, int TOKENS>
 __global__ void __launch_bounds__(NT)
 delta_prepare_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ w2t,
                      const float* __restrict__ w0, const float* __restrict__ a_bias, float* __restrict__ gates,
                      int tokens, int heads, int dim, int rank) {
   tl::pdl_launch_dependents();
   tl::pdl_wait();
-  extern __shared__ float lowrank[];  // tanh(l): PREP_TOKENS x rank floats
-  __shared__ float scratch[PREP_TOKENS][32];
-  const int t0 = blockIdx.x * PREP_TOKENS, h = blockIdx.y, i = threadIdx.x;
-  const int count = tokens - t0 < PREP_TOKENS ? tokens - t0 : PREP_TOKENS;
+  extern __shared__ float lowrank[];  // tanh(l): TOKENS x rank floats
+  __shared__ float scratch[TOKENS][32];
+  const int t0 = blockIdx.x * TOKENS, h = blockIdx.y, i = threadIdx.x;
+  const int count = tokens - t0 < TOKENS ? tokens - t0 : TOKENS;
   const int hd = heads * dim;
-  for (int e = threadIdx.x; e < PREP_TOKENS * rank; e += NT) {
+  for (int e = threadIdx.x; e < TOKENS * rank; e += NT) {
     const int tt = e / rank, j = e - tt * rank;
     lowrank[e] = tt < count ? tanhf(proj[(size_t)(t0 + tt) * proj_stride + 5 * hd + j]) : 0.f;
   }
   __syncthreads();
   const bool on = i < dim;
   const int c = h * dim + (on ? i : 0);
-  float inner[PREP_TOKENS];
+  float inner[TOKENS];
 #pragma unroll
-  for (int tt = 0; tt < PREP_TOKENS; ++tt) inner[tt] = w0[c];
+  for (int tt = 0; tt < TOKENS; ++tt) inner[tt] = w0[c];
   if (on) {
-#pragma unroll 8
+#pragma unroll(TOKENS == 1 ? 32 : 8)
     for (int j = 0; j < rank; ++j) {
       const float w = w2t[(size_t)j * hd + c];
 #pragma unroll
-      for (int tt = 0; tt < PREP_TOKENS; ++tt) inner[tt] = fmaf(w, lowrank[tt * rank + j], inner[tt]);
+      for (int tt = 0; tt < TOKENS; ++tt) inner[tt] = fmaf(w, lowrank[tt * rank + j], inner[tt]);
     }
   }
   // the tokens' keys are read and their squares summed together (the additions of block_sum, one barrier for all): a token after
   // the other the kernel waited eight times for a read and two barriers.  2,048 tokens, 32 heads of 64: 80 us against 90.
-  float k[PREP_TOKENS], ss[PREP_TOKENS];
+  float k[TOKENS], ss[TOKENS];
 #pragma unroll
-  for (int tt = 0; tt < PREP_TOKENS; ++tt) k[tt] = on && tt < count ? proj[(size_t)(t0 + tt) * proj_stride + hd + c] : 0.f;
+  for (int tt = 0; tt < TOKENS; ++tt) k[tt] = on && tt < count ? proj[(size_t)(t0 + tt) * proj_stride + hd + c] : 0.f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int tt = 0; tt < PREP_TOKENS; ++tt) {
+  for (int tt = 0; tt < TOKENS; ++tt) {
     ss[tt] = warp_sum(k[tt] * k[tt]);
     if (lane == 0) scratch[tt][warp] = ss[tt];
   }
   __syncthreads();
 #pragma unroll
-  for (int tt = 0; tt < PREP_TOKENS; ++tt) ss[tt] = warp_sum(lane < NT / 32 ? scratch[tt][lane] : 0.f);
+  for (int tt = 0; tt < TOKENS; ++tt) ss[tt] = warp_sum(lane < NT / 32 ? scratch[tt][lane] : 0.f);
   if (!on) return;
 #pragma unroll
-  for (int tt = 0; tt < PREP_TOKENS; ++tt) {
+  for (int tt = 0; tt < TOKENS; ++tt) {
     if (tt >= count) break;  // (the same for every thread of the block)
     const float w = expf(-DECAY_RATE * sigmoidf_(inner[tt]));
     const float a = sigmoidf_(proj[(size_t)(t0 + tt) * proj_stride + 4 * hd + c] + a_bias[c]);
@@ -374,17 +377,23 @@ int tl_delta_prepare(const float* proj, int proj_stride, const float* w2t, const
                      float* gates, int tokens, int heads, int dim, int rank, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (dim <= 0 || dim > 1024 || heads > 65535 || rank <= 0 || rank > 1024) return TL_ERR_UNSUPPORTED;
-  dim3 grid((tokens + PREP_TOKENS - 1) / PREP_TOKENS, heads);
-  const size_t smem = (size_t)PREP_TOKENS * rank * sizeof(float);
-#define TL_PREPARE(NT)                                                                                            \
-  tl::launch_kernel(delta_prepare_kernel<NT>, grid, NT, smem, stream, proj, proj_stride, w2t, w0, a_bias, gates,  \
+  const bool singly = (long long)((tokens + PREP_TOKENS - 1) / PREP_TOKENS) * heads <= sm_count();
+  const int each = singly ? 1 : PREP_TOKENS;
+  dim3 grid((tokens + each - 1) / each, heads);
+  const size_t smem = (size_t)each * rank * sizeof(float);
+#define TL_PREPARE_TOKENS(NT, TOKENS)                                                                                      \
+  tl::launch_kernel(delta_prepare_kernel<NT, TOKENS>, grid, NT, smem, stream, proj, proj_stride, w2t, w0, a_bias, gates,   \
                     tokens, heads, dim, rank)
+#define TL_PREPARE(NT)                            \
+  if (singly) TL_PREPARE_TOKENS(NT, 1);           \
+  else TL_PREPARE_TOKENS(NT, PREP_TOKENS)
   if (dim <= 32) { TL_PREPARE(32); }
   else if (dim <= 64) { TL_PREPARE(64); }
   else if (dim <= 128) { TL_PREPARE(128); }
   else if (dim <= 256) { TL_PREPARE(256); }
   else { TL_PREPARE(1024); }
 #undef TL_PREPARE
+#undef TL_PREPARE_TOKENS
   return TL_LAUNCH_CHECK();
 }
 
