@@ -278,6 +278,61 @@ def test_products_by_heads_in_one_launch(T, H, N, K, gap):
     assert (got[..., N:] == 7.0).all()
 
 
+@pytest.mark.parametrize("lens,H,D,R,V,rank,page_size", [([128], 1, 64, 16, 64, 64, 16), ([257, 2, 130], 2, 128, 64, 128, 72, 8),
+                                                          ([129, 300], 3, 64, 32, 128, 40, 16), ([513, 127], 2, 128, 48, 64, 64, 32)])
+def test_latent_attention_of_whole_prompts(lens, H, D, R, V, rank, page_size):
+    """Rows, expansion and attention against float64 over the bfloat16 cache rows: queries, keys, values and P are rounded to
+    bfloat16 once (2^-9 each of a weighted mean, whose weights the rounded scores move by a little more)."""
+    from torchlet_b200 import ops
+
+    T, bf = sum(lens), torch.bfloat16
+    q = rand(T, H * (D + R), seed=1).to(DEV)
+    rows = rand(T, rank + R, seed=2).to(DEV).to(bf)
+    uk, uv = rand(H * D, rank, seed=3, scale=rank ** -0.5).to(DEV).to(bf), rand(H * V, rank, seed=4, scale=rank ** -0.5).to(DEV).to(bf)
+    inv_freq = (10000.0 ** (-2.0 * torch.arange(R // 2, dtype=torch.float64) / R)).float().to(DEV)
+    need = [-(-n // page_size) for n in lens]
+    order = torch.randperm(sum(need), generator=torch.Generator().manual_seed(5)) + 1
+    pages = torch.full((sum(need) + 1, 1, 1, page_size, rank + R), float("nan"), device=DEV, dtype=bf)
+    table = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    positions = torch.cat([torch.arange(n) for n in lens]).to(torch.int32)
+    token_req = torch.cat([torch.full((n,), r) for r, n in enumerate(lens)]).to(torch.int32)
+    at = 0
+    for r, n in enumerate(need):
+        table[r, :n] = order[at:at + n]
+        at += n
+    where = table[token_req.long(), (positions // page_size).long()].long()
+    pages[where.to(DEV), 0, 0, (positions % page_size).long().to(DEV)] = rows
+    indptr = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    step = ops.latent_prompt_tokens()
+    tiles = [(r, row) for r, n in enumerate(lens) for row in range(0, n, step)]
+    tile_req, tile_row = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in zip(*tiles))
+    queries, c, k_rot = (torch.empty(T, n, device=DEV, dtype=bf) for n in (H * (D + 64), rank, 64))
+    ops.latent_prompt_rows(q, inv_freq, positions.to(DEV), token_req.to(DEV), table.to(DEV), pages, page_size, queries, c, k_rot, H, D, R, R)
+    assert torch.equal(c, rows[:, :rank]) and torch.equal(k_rot[:, :R], rows[:, rank:]) and not k_rot[:, R:].any()
+    keys, values = torch.empty(T, H * D, device=DEV, dtype=bf), torch.empty(T, H * V, device=DEV, dtype=bf)
+    ops.gemm_tc(c, uk, keys, None, ops.EPI_STORE_BF16)
+    ops.gemm_tc(c, uv, values, None, ops.EPI_STORE_BF16)
+    out = torch.full((T, H * V), float("nan"), device=DEV, dtype=bf)
+    scale = (D + R) ** -0.5
+    ops.latent_prompt(queries, keys, k_rot, values, indptr, tile_req, tile_row, len(tiles), out, H, D, R, V, scale)
+    assert ops.latent_prompt_error() == 0
+    x = q.double().view(T, H, D + R)
+    angle = positions.to(DEV).double()[:, None, None] * inv_freq.double()
+    a, b = x[..., D:D + R // 2], x[..., D + R // 2:]
+    turned = torch.cat((a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()), -1)
+    got = queries.double().view(T, H, D + 64)
+    assert (got[..., D:D + R] - turned).abs().max() <= 2.0 ** -8 * turned.abs().max() and not got[..., D + R:].any()
+    for r, n in enumerate(lens):
+        s = slice(int(indptr[r]), int(indptr[r + 1]))
+        kept = rows[s].double()
+        k = torch.einsum("sc,hdc->hsd", kept[:, :rank], uk.double().view(H, D, rank))
+        v = torch.einsum("sc,hvc->hsv", kept[:, :rank], uv.double().view(H, V, rank))
+        score = torch.einsum("thd,hsd->hts", x[s, :, :D], k) + torch.einsum("thr,sr->hts", turned[s], kept[:, rank:])
+        score = (score * scale).masked_fill(torch.ones(n, n, device=DEV).triu(1).bool(), -math.inf)
+        want = (torch.softmax(score, -1) @ v).transpose(0, 1).reshape(n, H * V)
+        assert (out[s].double() - want).abs().max() <= 2e-2 * want.abs().max()
+
+
 def latent_setup(H, rank, rot, page_size, num_pages, dtype):
     pages = torch.full((num_pages, 1, 1, page_size, rank + rot), float("nan"), device=DEV, dtype=dtype)
     return pages

@@ -155,6 +155,15 @@ _SIGNATURES = {
                                     c_void_p, c_int, c_void_p],
         "tl_latent_attention_mma_debug_error": [c_void_p],
     },
+    "latent_prompt": {
+        "tl_latent_prompt_error": [],
+        "tl_latent_prompt_tokens": [],
+        "tl_latent_prompt_rows": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
+                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+        "tl_latent_prompt": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
+                             c_int, c_int, c_int, c_float, c_void_p],
+        "tl_latent_prompt_debug_error": [c_void_p],
+    },
     "delta_chunked": {
         "tl_delta_chunk_tokens": [],
         "tl_delta_chunk_record": [],
@@ -1263,6 +1272,49 @@ def latent_absorb_q(q, uk, inv_freq, positions, q_abs, heads, dim, rot_dim, rot_
     _check(code, "latent_absorb_q")
 
 
+def latent_prompt_tokens() -> int:
+    """Tokens of a request that a CTA of ``latent_prompt`` takes."""
+    return _fn("latent_prompt", "tl_latent_prompt_tokens")()
+
+
+def latent_prompt_rows(q, inv_freq, positions, token_req, block_table, pages, page_size, queries, c, k_rot, heads, dim, rot_dim,
+                       rot_dims) -> None:
+    """What ``latent_prompt`` and the products before it read, in bfloat16: the queries with their rotated part,
+    [T, H (dim + 64)], and the tokens' cache rows apart, c [T, rank] and k_rot [T, 64] (csrc/latent_prompt.cu)."""
+    _need_cuda(q, inv_freq, positions, token_req, block_table, pages, queries, c, k_rot)
+    tokens, rank = c.shape
+    assert q.dtype == torch.float32 and q.stride(1) == 1 and q.shape == (tokens, heads * (dim + rot_dim))
+    assert pages.dtype == queries.dtype == c.dtype == k_rot.dtype == torch.bfloat16 and pages.is_contiguous()
+    assert pages.shape[-1] == rank + rot_dim and positions.numel() >= tokens
+    assert queries.is_contiguous() and queries.shape == (tokens, heads * (dim + 64))
+    assert c.is_contiguous() and k_rot.is_contiguous() and k_rot.shape == (tokens, 64)
+    code = _fn("latent_prompt", "tl_latent_prompt_rows")(
+        q.data_ptr(), q.stride(0), inv_freq.data_ptr(), positions.data_ptr(), token_req.data_ptr(), block_table.data_ptr(),
+        block_table.shape[1], pages.data_ptr(), page_size, pages.shape[0], queries.data_ptr(), c.data_ptr(), k_rot.data_ptr(),
+        tokens, heads, dim, rot_dim, rot_dims, rank, _stream())
+    _check(code, "latent_prompt_rows")
+
+
+def latent_prompt(queries, keys, k_rot, values, req_indptr, tile_req, tile_row, tiles, out, heads, dim, rot_dim, vdim,
+                  scale) -> None:
+    """Causal attention of whole prompts over expanded keys [T, H dim] (with k_rot [T, 64], which all heads share) and values
+    [T, H vdim] on tcgen05 (csrc/latent_prompt.cu), bfloat16: no request has cached tokens.  ``tile_req``, ``tile_row``: the
+    request and first token (a multiple of ``latent_prompt_tokens()``) of each CTA, which cover every request."""
+    _need_cuda(queries, keys, k_rot, values, req_indptr, tile_req, tile_row, out)
+    tokens = queries.shape[0]
+    for t, width in ((queries, heads * (dim + 64)), (keys, heads * dim), (k_rot, 64), (values, heads * vdim), (out, heads * vdim)):
+        assert t.dtype == torch.bfloat16 and t.is_contiguous() and t.shape == (tokens, width)
+    code = _fn("latent_prompt", "tl_latent_prompt")(
+        queries.data_ptr(), keys.data_ptr(), k_rot.data_ptr(), values.data_ptr(), req_indptr.data_ptr(), tile_req.data_ptr(),
+        tile_row.data_ptr(), tiles, out.data_ptr(), tokens, heads, dim, rot_dim, vdim, float(scale), _stream())
+    _check(code, "latent_prompt")
+
+
+def latent_prompt_error() -> int:
+    """0, or the code a bounded wait in the prompt form of the latent attention left when it gave up."""
+    return _fn("latent_prompt", "tl_latent_prompt_error")()
+
+
 def latent_attention(q_abs, pages, block_table, token_req, positions, out, tokens, heads, dk, dv, page_size,
                      scale, window=None) -> None:
     """Causal attention of every (token, head) over the cached rows of its request, in the latent
@@ -1771,7 +1823,7 @@ def debug_errors() -> list:
     in the ordinary build (``TORCHLET_B200_DEBUG`` unset), whose kernels carry no checks."""
     found = []
     for library in ("elementwise", "attention_generic", "attention_mma", "decode_fused", "slots", "stream_ops",
-                    "delta_rule", "delta_chunked", "latent_attention", "latent_attention_mma", "gla", "gla_chunked", "gated_attention", "hyper",
+                    "delta_rule", "delta_chunked", "latent_attention", "latent_attention_mma", "latent_prompt", "gla", "gla_chunked", "gated_attention", "hyper",
                     "pooled_attention", "ssm", "time_mixing", "token_shift", "qkv_prepare", "token_embed",
                     "attention_mixed_decode"):
         if any(name in _functions for name in _SIGNATURES[library]):
@@ -1790,7 +1842,7 @@ def raise_on_wait_errors() -> None:
     stream, so it sees every kernel launched before it."""
     for library, read in (("gemm_tc", gemm_tc_error), ("attention_tc", attention_tc_error),
                           ("attention_mma", attention_mma_error), ("attention_spread", attention_spread_error),
-                          ("attention_mixed_decode", attention_mixed_decode_error)):
+                          ("attention_mixed_decode", attention_mixed_decode_error), ("latent_prompt", latent_prompt_error)):
         if any(name in _functions for name in _SIGNATURES[library]):
             code = read()
             if code:

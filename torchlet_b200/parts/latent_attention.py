@@ -9,7 +9,8 @@ cache row is [c (kv_rank) | k_rot (rot_dim)], shared by all heads.
 The attention itself runs in the latent space (csrc/latent_attention.cu): W_uk,h is folded into
 the query and W_uv,h applied after the weighted sum of cached rows, so no key or value of a
 cached token is ever expanded and prompt portions, single tokens and mixed batches are one code
-path.  A layer with ``kv_from`` has no W_dkv and reads another layer's cache rows.
+path.  In the bfloat16 engine a step of whole prompts, which sees no keys but its own tokens', expands those
+instead (``prompt_tiles``, csrc/latent_prompt.cu).  A layer with ``kv_from`` has no W_dkv and reads another layer's cache rows.
 
 Options: ``rot_dim`` 0: no rotated part (no positions at all; the cache row is c alone); ``window``: a query at position i
 sees the keys j with 0 <= i - j < window only (None: all before it); ``q_rank`` None: there is no query latent, q = W_q x (tensor ``q`` instead of dq, dq.norm, uq);
@@ -82,6 +83,26 @@ def row_tiles(ctx, heads: int, window=None):
             both = ctx.upload(np.concatenate([req[order], row[order]]))
             plan = (both[:len(tile_req)], both[len(tile_req):], len(tile_req), 1)
         ctx.plans[key] = plan
+    return plan
+
+
+def prompt_tiles(ctx):
+    """(tile_req, tile_row, tiles) for a step of whole prompts on csrc/latent_prompt.cu, planned once a step, or None where some
+    request decodes or has cached tokens (whose keys would have to be expanded in every step), or where the step has fewer
+    tokens than the per-head products of the latent form take."""
+    if ctx.decode_only:
+        return None
+    plan = ctx.plans.get("latent_attention.prompt", False)
+    if plan is False:
+        lengths = np.diff(ctx.req_indptr_host)
+        plan = None
+        if int(lengths.sum()) >= MIN_TOKENS_FOR_HEAD_PRODUCTS and lengths.min() > 1 and not ctx.kv_before_host[:lengths.size].any():
+            step = ops.latent_prompt_tokens()
+            tiles = [(row, r) for r, n in enumerate(lengths) for row in range(0, int(n), step)]
+            tiles.sort(key=lambda t: -min(t[0] + step, int(lengths[t[1]])))  # those that see the most keys first
+            both = ctx.upload(np.asarray([r for _, r in tiles] + [row for row, _ in tiles], dtype=np.int32))
+            plan = (both[:len(tiles)], both[len(tiles):], len(tiles))
+        ctx.plans["latent_attention.prompt"] = plan
     return plan
 
 
@@ -183,6 +204,9 @@ class LatentAttentionMixer(Mixer):
         f32 = lambda name: tensors[prefix + name].to(device=device, dtype=torch.float32).contiguous()
         self.q_norm = f32("dq.norm") if self.q_rank else None
         self.kv_norm = f32("dkv.norm") if self.own_kv else None
+        # sizes of the prompt form, whose keys and values are expanded
+        self.prompt_form = (dtype == torch.bfloat16 and D in (64, 128) and self.v_dim in (64, 128) and 0 < R <= 64
+                            and R % 16 == 0 and self.kv_rank % 8 == 0 and self.window is None and self.scale > 0)
         # base^(-2i/dims), taken in float64 and rounded once
         i = torch.arange(self.rot_dims // 2, dtype=torch.float64)
         self.inv_freq = (self.rot_base ** (-2.0 * i / max(self.rot_dims, 1))).to(torch.float32).to(device)
@@ -203,6 +227,15 @@ class LatentAttentionMixer(Mixer):
             self.uq_proj.forward(c_q, q)
         else:  # the queries are rows of the first product
             q = down[:, latent_width:latent_width + H * (self.head_dim + self.rot_dim)]
+        prompts = prompt_tiles(ctx) if self.prompt_form else None
+        out = ctx.buffer("latent.out", (tokens, H * self.v_dim), ctx.dtype)
+        if prompts is not None:
+            self.attend_prompts(ctx, q, cache, prompts, out)
+            if self.gate:
+                ops.gate_mul_(out, down[:, self.gate_offset:])
+            if not self.o_proj.accumulate_later(ctx, out, acc):
+                self.o_proj.forward(out, acc, accumulate=True)
+            return
         q_abs = ctx.buffer("latent.q_abs", (tokens, H * self.row), ctx.dtype)
         per_head_products = self.uk_heads is not None and tokens >= MIN_TOKENS_FOR_HEAD_PRODUCTS
         one_launch = self.head_dim % 64 == 0 and self.kv_rank % 64 == 0  # else a launch a head
@@ -229,7 +262,6 @@ class LatentAttentionMixer(Mixer):
         else:
             ops.latent_attention(q_abs, cache.pages, cache.block_table, ctx.token_req, ctx.positions, o_lat, tokens, H,
                                  self.row, self.kv_rank, cache.page_size, self.scale, window=self.window)
-        out = ctx.buffer("latent.out", (tokens, H * self.v_dim), ctx.dtype)
         if per_head_products:
             V, rank = self.v_dim, self.kv_rank
             if one_launch:
@@ -245,3 +277,19 @@ class LatentAttentionMixer(Mixer):
             ops.gate_mul_(out, down[:, self.gate_offset:])
         if not self.o_proj.accumulate_later(ctx, out, acc):
             self.o_proj.forward(out, acc, accumulate=True)
+
+    def attend_prompts(self, ctx, q, cache, prompts, out) -> None:
+        """Whole prompts: keys and values of the step's tokens expanded from their cache rows, then plain causal attention."""
+        tokens, H, D, V = q.shape[0], self.num_heads, self.head_dim, self.v_dim
+        queries = ctx.buffer("latent.queries", (tokens, H * (D + 64)), ctx.dtype)
+        c = ctx.buffer("latent.c", (tokens, self.kv_rank), ctx.dtype)
+        k_rot = ctx.buffer("latent.k_rot", (tokens, 64), ctx.dtype)
+        ops.latent_prompt_rows(q, self.inv_freq, ctx.positions, ctx.token_req, cache.block_table, cache.pages, cache.page_size,
+                               queries, c, k_rot, H, D, self.rot_dim, self.rot_dims)
+        keys = ctx.buffer("latent.keys", (tokens, H * D), ctx.dtype)
+        values = ctx.buffer("latent.values", (tokens, H * V), ctx.dtype)
+        ops.gemm_tc(c, self.uk, keys, None, ops.EPI_STORE_BF16)
+        ops.gemm_tc(c, self.uv, values, None, ops.EPI_STORE_BF16)
+        tile_req, tile_row, tiles = prompts
+        ops.latent_prompt(queries, keys, k_rot, values, ctx.req_indptr, tile_req, tile_row, tiles, out, H, D, self.rot_dim, V,
+                          self.scale)
