@@ -943,3 +943,20 @@ def test_decode_attention_around_the_depth_of_its_rings(nh, nkv, d, page, splits
         weight = torch.softmax(q @ rows[r][0][:, first:].transpose(1, 2) * d ** -0.5, -1)
         want = (weight @ rows[r][1][:, first:]).reshape(nh * d)
         assert (out[r].cpu().double() - want).abs().max() <= 1e-2 * max(1.0, want.abs().max().item()), n
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 9728, 896), (509, 9728, 512), (300, 12000, 516), (137, 16896, 640)])
+def test_float32_products_whose_last_wave_goes_beside(M, N, K):
+    """A nearly empty last wave of 128 x 64 tiles (148 SMs: 304 or 608 tiles for 296 blocks; the others: whatever the GPU has)
+    runs as clusters beside the other tiles: every row has the bits it has alone."""
+    from torchlet_b200 import ops
+
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    start = torch.randn(M, N, generator=g).to(DEV)
+    out = start.clone()
+    ops.gemm_simt(x, w, out, accumulate=True)
+    for m in (0, 1, 127, 128, M // 2, M - 2, M - 1):
+        alone = start[m:m + 1].clone()
+        ops.gemm_simt(x[m:m + 1], w, alone, accumulate=True)
+        assert torch.equal(alone[0], out[m]), m
