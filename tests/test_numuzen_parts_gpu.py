@@ -484,3 +484,26 @@ def test_router_options_and_ties():
     ops.moe_route(x.to(DEV), router.to(DEV), choice, weight, softmax_scores=True)
     z = router[:, 0].double()
     close(weight[1], torch.softmax(z, 0)[[1, 2, 4]], 1e-6, "softmax scores")
+
+
+@pytest.mark.parametrize("tokens,hidden,experts,top,dtype", [(1184, 2048, 8, 2, torch.bfloat16), (1191, 72, 40, 3, torch.bfloat16),
+                                                             (1300, 500, 8, 1, torch.float32), (1187, 1000, 33, 4, torch.bfloat16)])
+def test_routing_many_tokens_gives_the_bits_of_one(tokens, hidden, experts, top, dtype):
+    """From eight tokens an SM on a block takes eight tokens: choices, weights and the always-on expert's gate are those of a
+    step of one token."""
+    from torchlet_b200 import ops
+
+    x, router = rand(tokens, hidden, seed=1).to(DEV).to(dtype), rand(experts, hidden, seed=2, scale=hidden ** -0.5).to(DEV)
+    gate_w, bias = rand(hidden, seed=3, scale=hidden ** -0.5).to(DEV), rand(experts, seed=4).to(DEV)
+
+    def route(rows):
+        n = rows.shape[0]
+        choice = torch.empty(n, top, dtype=torch.int32, device=DEV)
+        weight, gate = torch.empty(n, top, device=DEV), torch.empty(n, device=DEV)
+        ops.moe_route(rows, router, choice, weight, False, True, 1, 1, 1e-20, token_gate=(gate_w, gate), bias=bias)
+        return choice, weight, gate
+
+    many = route(x)
+    for t in (0, 1, 7, 8, 100, tokens - 9, tokens - 2, tokens - 1):
+        for a, b in zip(many, route(x[t:t + 1])):
+            assert torch.equal(a[t:t + 1], b), t
