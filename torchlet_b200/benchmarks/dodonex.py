@@ -128,9 +128,9 @@ def time_decode(model, batch: int, context: int, steps: int, warmup: int = 4) ->
 
 
 KERNEL_CLASSES = {
-    "latent attention": ("latent_attention_mma", "latent_attention"),
-    "latent prepare/absorb/expand": ("latent_prepare", "latent_absorb_q", "latent_expand_o"),
-    "delta rule": ("delta_prepare", "delta_scan", "delta_finish"),
+    "latent attention": ("latent_attention_mma", "latent_attention", "latent_prompt"),
+    "latent prepare/absorb/expand": ("latent_prepare", "latent_absorb_q", "latent_expand_o", "latent_prompt_rows"),
+    "delta rule": ("delta_prepare", "delta_scan", "delta_chunked", "delta_finish"),
     "clamped glu": ("clamped_glu",),
     "token input (elementwise)": ("gated_token_embed", "rms_scaled_add"),
     "residual (zero, scaled add)": ("fill_zero", "scaled_add"),

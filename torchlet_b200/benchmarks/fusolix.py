@@ -58,7 +58,7 @@ KERNEL_CLASSES = {
 
 NUMUZEN_CLASSES = {
     "attention (norm, rotation, cache write, scores and values)": ("normed_qk_store", "attention_tc", "attention_mma", "attention_generic"),
-    "gla (decay, scan, finish)": ("gla_decay", "gla_scan", "gla_finish"),
+    "gla (decay, scan, finish)": ("gla_decay", "gla_scan", "gla_chunked", "gla_finish"),
     "side stream (zero, norm behind the sub-layer)": ("fill_zero", "rms_scaled_add"),
     "routing (route, plan, scatter, combine)": ("moe_route", "moe_plan", "moe_scatter", "moe_combine"),
     "expert products": ("gemm_tc_grouped", "moe_gemm_simt"),

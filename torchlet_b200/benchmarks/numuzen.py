@@ -44,7 +44,7 @@ def numuzen_config(size: str, layers: int, experts: int = 8, top: int = 2, windo
 
 
 KERNEL_CLASSES = {
-    "gla (decay, scan, finish)": ("gla_decay", "gla_scan", "gla_finish"),
+    "gla (decay, scan, finish)": ("gla_decay", "gla_scan", "gla_chunked", "gla_finish"),
     "attention (norm, rotation, cache write)": ("normed_qk_store",),
     "attention (scores and values)": ("attention_mma", "attention_generic"),
     "routing (route, plan, scatter, combine)": ("moe_route", "moe_plan", "moe_scatter", "moe_combine"),
