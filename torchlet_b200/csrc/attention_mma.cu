@@ -682,7 +682,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const Params
     tile_end = min(tile_end, tile_begin + per);
   }
   const int num_tiles = max(0, tile_end - tile_begin);
-  if (warp == WARPS) {  // a lane a barrier: one thread would spend a tenth of a microsecond on them
+  if (warp == WARPS) {  // a lane a barrier
     if (lane < 4 * STAGES) {
       tc::mbar_init(&k_full[lane], lane < 2 * STAGES ? 1 : WARPS);
       tc::mbar_fence_init();
@@ -695,57 +695,40 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const Params
     // ---- the requesting warp: one lane a page, whose keys (or values) of this head are one box [slab of 64][token].  Pages
     // past the request's last key or past the table are read from page 0 (always there; their keys are masked and their
     // value rows cleared before use).
-    const int pages_per_tile = BLOCK_N / p.page_size, my_page = lane & 15, upper = lane >> 4;
-    const bool copies = my_page < pages_per_tile;  // at most 8 pages a tile
+    const int pages_per_tile = BLOCK_N / p.page_size;
     auto page_of = [&](const int t) {
-      const int index = (tile_begin + t) * pages_per_tile + my_page;
-      return copies && t < num_tiles && index < p.table_width && index * p.page_size <= hi_key ? table[index] : 0;
+      const int index = (tile_begin + t) * pages_per_tile + lane;
+      return lane < pages_per_tile && t < num_tiles && index < p.table_width && index * p.page_size <= hi_key ? table[index] : 0;
     };
-    auto copy = [&](const int t, const int is_v, const int page) {
-      const int slot = t % STAGES;
-      tc::tma_load_3d((is_v ? v_ring : k_ring) + slot * TILE + my_page * p.page_size * D, &map_kv, (is_v ? v_full : k_full) + slot, 0,
-                      ((page * 2 + is_v) * p.nkv + kvh) * p.page_size, 0);
-    };
-    // Tiles that lie wholly before the step's own tokens were written by earlier steps: as many as the rings hold are requested
-    // before the wait, keys by the lower and values by the upper half of the warp.
-    const int depth = min(STAGES, num_tiles);
-    int page[STAGES], first = 0;
-#pragma unroll
-    for (int t = 0; t < STAGES; ++t) page[t] = page_of(t);
-    if (my_page == 0)
-      for (int t = 0; t < depth; ++t) tc::mbar_expect_tx((upper ? v_full : k_full) + t, TILE * 2);
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < STAGES; ++t)
-      if (t < depth && t == first && (tile_begin + t) * BLOCK_N + BLOCK_N - 1 < before) {
-        if (copies) copy(t, upper, page[t]);
-        ++first;
-      }
-    // With late_wait the kernel before this one is the prompt portions' attention, which is independent of this one and whose
-    // every CTA had waited for this step's keys before this grid could start.
-    if (!p.late_wait) tl::pdl_wait();
-    tl::pdl_launch_dependents();  // a CTA has signalled when ALL its warps have, or have left
-#pragma unroll
-    for (int t = 0; t < STAGES; ++t)
-      if (t >= first && t < depth && copies) copy(t, upper, page[t]);
-    // Then a tile a turn, its keys before the values of the one before it: that is the order in which the slots are read.
+    // tiles that lie wholly before the step's own tokens were written by earlier steps and are requested before the wait.
+    // With late_wait the kernel before this one is the prompt portions' attention, which is independent of this one and
+    // whose every CTA had waited for this step's keys before this grid could start.
+    bool waited = p.late_wait;
     auto request = [&](const int t, const int is_v, const int page) {
+      if (!waited && (tile_begin + t) * BLOCK_N + BLOCK_N - 1 >= before) {
+        tl::pdl_wait();
+        waited = true;
+      }
       const int slot = t % STAGES;
-      tc::mbar_wait((is_v ? v_read : k_read) + slot, (t / STAGES - 1) & 1, abort_flag, &g_error_word, 2);
-      if (lane == 0) tc::mbar_expect_tx((is_v ? v_full : k_full) + slot, TILE * 2);
+      uint64_t* full = (is_v ? v_full : k_full) + slot;
+      if (t >= STAGES) tc::mbar_wait((is_v ? v_read : k_read) + slot, (t / STAGES - 1) & 1, abort_flag, &g_error_word, 2);
+      if (lane == 0) tc::mbar_expect_tx(full, TILE * 2);
       __syncwarp();
-      if (copies && !upper) copy(t, is_v, page);
+      if (lane < pages_per_tile)
+        tc::tma_load_3d((is_v ? v_ring : k_ring) + slot * TILE + lane * p.page_size * D, &map_kv, full, 0,
+                        ((page * 2 + is_v) * p.nkv + kvh) * p.page_size, 0);
       __syncwarp();
     };
-    int page_now = page_of(STAGES), page_before = 0;
-    for (int t = STAGES; t <= num_tiles && num_tiles > STAGES && !*abort_flag; ++t) {
-      const int page_next = page_of(t + 1);  // read a tile before it is needed
-      if (t < num_tiles) request(t, 0, page_now);
-      if (t > STAGES) request(t - 1, 1, page_before);
-      page_before = page_now;
-      page_now = page_next;
+    int page = page_of(0), page_next = page_of(1);
+    if (num_tiles > 0) request(0, 0, page);
+    for (int t = 0; t < num_tiles && !*abort_flag; ++t) {
+      const int page_after = page_of(t + 2);  // read a tile before it is needed
+      if (t + 1 < num_tiles) request(t + 1, 0, page_next);
+      request(t, 1, page);
+      page = page_next;
+      page_next = page_after;
     }
-    if (p.late_wait) tl::pdl_wait();  // (no thread of the grid ends before the grids before it)
+    if (!waited || p.late_wait) tl::pdl_wait();  // (no thread of the grid ends before the grids before it)
     return;
   }
 
