@@ -171,6 +171,33 @@ def test_gla_chunk_by_chunk(lens, H, D, V):
     assert (padded == 0).all() and torch.equal(padded_state, start)
 
 
+@pytest.mark.parametrize("at", [1, 3, 6, 15, 16, 45, 63, 64, 74])
+@pytest.mark.parametrize("V,value", [(128, math.inf), (40, math.nan)])
+def test_gla_chunks_keep_values_without_a_number_from_earlier_tokens(at, V, value):
+    """An infinite or NaN value reaches its own token and those after it, as in the scan; the tokens before it, of its chunk too,
+    have the bits they have without it."""
+    from torchlet_b200 import ops
+
+    T, H, D = 80, 2, 64
+    clean = rand(T, 2 * H * D + H * V, seed=4).to(DEV)
+    proj = clean.clone()
+    proj[at, 2 * H * D + V + 5] = value  # channel 5 of the second head
+    decay = torch.sigmoid(rand(T, H * D, seed=5, scale=2.0)).pow(1 / 8.0).to(DEV)
+    indptr, slots = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([0, T], [0]))
+
+    def run(rows):
+        state, out = torch.zeros(1, H, D, V, device=DEV), torch.full((T, H * V), -1.0, device=DEV)
+        chunks = -(-T // ops.gla_chunk_tokens())
+        workspace = torch.empty(chunks * H * (D * V + 64), device=DEV)
+        ops.gla_chunked(rows, decay, indptr, slots, state, out, workspace, 1, chunks, 1, H, D, V, 1.0)
+        return out
+
+    out, right = run(proj), run(clean)
+    assert not out[at:, V + 5].isfinite().any()
+    out[at:, V + 5] = right[at:, V + 5]
+    assert torch.equal(out, right)
+
+
 @pytest.mark.parametrize("H,D,V,requests", [(4, 64, 32, 1), (40, 64, 72, 2), (30, 128, 64, 8), (75, 32, 40, 4)])
 def test_gla_scan_blocks_kept_apart(H, D, V, requests):
     """Portions of 64 tokens and more take shared memory by how many blocks an SM has: one, two, four, more; the bits are

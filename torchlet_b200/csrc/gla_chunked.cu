@@ -125,16 +125,20 @@ __device__ __forceinline__ void ones_past(float* a, int count, int dim) {
 
 // sum[4 rows][8 columns] += x[rows][n] y[n][columns], n a multiple of 16, each sixteen products on their own first (one chain
 // of 128 additions rounds further off than the scan's short ones).  x: four rows from ``x`` on, LD apart; y: rows of VT floats,
-// the thread's columns are 4 jg and VT / 2 + 4 jg.
-template <int VT>
-__device__ __forceinline__ void tile_fma(float2 (&sum)[4][4], const float* x, const float* y, int n, int jg) {
+// the thread's columns are 4 jg and VT / 2 + 4 jg.  CAUSAL: of the last sixteen products row r takes those up to number
+// ``last`` + r only (``last`` a multiple of 4): a factor behind them is never multiplied, not even with zero, which would make
+// NaN of an infinite one.
+template <int VT, bool CAUSAL>
+__device__ __forceinline__ void tile_fma(float2 (&sum)[4][4], const float* x, const float* y, int n, int jg, int last = 12) {
 #pragma unroll 1
   for (int k = 0; k < n; k += 16) {
     unsigned long long acc[4][4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0ull;
+    const int stop = CAUSAL && k + 16 >= n ? last : 16;
 #pragma unroll
     for (int kk = 0; kk < 16; kk += 4) {
+      if (CAUSAL && kk > stop) break;
       float4 a[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(x + r * LD + k + kk);
@@ -144,6 +148,7 @@ __device__ __forceinline__ void tile_fma(float2 (&sum)[4][4], const float* x, co
         const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(y + (k + kk + e) * VT + VT / 2 + 4 * jg);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
+          if (CAUSAL && e > r && kk == stop) continue;
           const unsigned long long s = twice(e == 0 ? a[r].x : e == 1 ? a[r].y : e == 2 ? a[r].z : a[r].w);
           fma2(acc[r][0], s, b0.x);
           fma2(acc[r][1], s, b0.y);
@@ -210,7 +215,7 @@ gla_chunk_state_kernel(const Args p) {
   const int jg = tid % JG, ig = tid / JG;
   if (ig >= DK / 4) return;
   float2 acc[4][4] = {};
-  tile_fma<VT>(acc, k + ig * 4 * LD, v, (count + 15) / 16 * 16, jg);
+  tile_fma<VT, false>(acc, k + ig * 4 * LD, v, (count + 15) / 16 * 16, jg);
   float* dst = p.sums + ((size_t)blockIdx.x * p.heads + h) * p.dim * p.vdim + col0;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -405,8 +410,8 @@ gla_chunk_out_kernel(const Args p) {
   const int jg = tid % JG, tg = tid / JG;
   if (tg >= CHUNK / 4 || tg * 4 >= count) return;
   float2 acc[4][4] = {};
-  tile_fma<VT>(acc, q + tg * 4 * LD, S, DK, jg);
-  tile_fma<VT>(acc, A + tg * 4 * LD, v, (tg * 4 / SUB + 1) * SUB, jg);
+  tile_fma<VT, false>(acc, q + tg * 4 * LD, S, DK, jg);
+  tile_fma<VT, true>(acc, A + tg * 4 * LD, v, (tg * 4 / SUB + 1) * SUB, jg, tg * 4 % SUB);
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int t = tg * 4 + r;
