@@ -201,6 +201,37 @@ def test_delta_scan_blocks_kept_apart(H, D, requests):
         assert torch.equal(again[r], state[r])
 
 
+def test_delta_scans_of_two_threads_keep_their_shared_memory():
+    """Two engines in two threads launch the same kernel with one and with four blocks an SM, which take unlike amounts of shared
+    memory: neither launch is refused, and the bits are those of one thread alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from torchlet_b200 import ops
+
+    D, n = 16, 64
+
+    def inputs(H):
+        proj, gates = rand(n, 5 * H * D, seed=H).to(DEV), torch.rand(n, H * 3 * D, generator=torch.Generator().manual_seed(H)).to(DEV) / D
+        return proj, gates, *(torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([0, n], [0]))
+
+    def launch(H, given, times):
+        state, out = torch.zeros(1, H, D, D, device=DEV), torch.empty(n, H * D, device=DEV)
+        for _ in range(times):
+            state.zero_()
+            ops.delta_scan(*given, state, out, 1, H, D)
+        return out, state
+
+    heads = (8, 500)  # (a block a head at this head size)
+    given = {H: inputs(H) for H in heads}
+    want = {H: launch(H, given[H], 1) for H in heads}
+    torch.cuda.synchronize()
+    with ThreadPoolExecutor(4) as pool:
+        jobs = [(H, pool.submit(launch, H, given[H], 2000)) for H in heads * 2]
+        for H, job in jobs:
+            for a, b in zip(job.result(), want[H]):
+                assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("lens,H,D,rank,pad", [([8], 1, 64, 16, 0), ([37, 9, 1, 8, 16, 100], 2, 64, 16, 0), ([37, 3], 2, 24, 5, 0),
                                                ([50, 2, 41], 3, 40, 7, 0), ([23], 1, 4, 2, 0), ([300], 2, 64, 64, 3)])
 def test_delta_rule_chunk_by_chunk(lens, H, D, rank, pad):

@@ -9,6 +9,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <utility>
+
 #define TL_DTYPE_F32 0
 #define TL_DTYPE_BF16 1
 
@@ -127,6 +130,28 @@ inline size_t spread_smem(long long blocks, int sms, size_t used) {
   if (share < 1 || share > 4) return 0;
   const size_t least = SM_BYTES / (share + 1) + 16 - RESERVED;  // share + 1 blocks of this size no longer fit
   return least > used ? (least - used + 15) / 16 * 16 : 0;
+}
+
+// Launches KERNEL, whose blocks have ``fixed`` static and ``dynamic`` dynamic shared memory, kept apart where ``apart``.  The
+// kernel's limit is raised once a device, to the most any launch can ask for: were it set to each launch's own size, a second
+// thread could lower it between another's setting and its launch, which would then be refused.
+template <auto KERNEL, typename... Args>
+inline cudaError_t launch_apart(dim3 grid, dim3 block, bool apart, int sms, size_t fixed, size_t dynamic, cudaStream_t stream,
+                                Args&&... args) {
+  static std::atomic<unsigned long long> raised{0};
+  const size_t more = apart ? spread_smem((long long)grid.x * grid.y * grid.z, sms, fixed + dynamic) : 0;
+  if (dynamic + more > 0) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = 1ull << (device & 63);
+    if (device > 63 || !(raised.load(std::memory_order_acquire) & bit)) {
+      e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(dynamic + spread_smem(1, 1, fixed + dynamic)));
+      if (e != cudaSuccess) return e;
+      raised.fetch_or(bit, std::memory_order_release);
+    }
+  }
+  return launch_kernel(KERNEL, grid, block, dynamic + more, stream, std::forward<Args>(args)...);
 }
 
 // The first key position a query at position ``pos`` sees, by the mask code all paged attention kernels share:

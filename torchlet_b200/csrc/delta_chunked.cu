@@ -399,13 +399,9 @@ int tl_delta_chunked(const float* proj, int proj_stride, const float* w2t, const
   tl::launch_kernel(delta_chunk_prepare_kernel, dim3(chunks, heads), DK, (size_t)CHUNK * rank * sizeof(float), stream, proj,
                     proj_stride, w2t, w0, a_bias, req_indptr, records, requests, least, heads, dim, rank);
   const dim3 grid(requests, heads, (dim + COLS - 1) / COLS);
-  constexpr size_t USED = (size_t)STAGES * STAGE * sizeof(float);
   // (the blocks of requests without chunks leave at once; the others walk long enough that their places matter)
-  const size_t smem = USED + tl::spread_smem((long long)grid.x * grid.y * grid.z, sm_count(), USED);
-  const cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024);
-  if (e != cudaSuccess) return (int)e;
-  tl::launch_kernel(delta_chunk_scan_kernel, grid, SCAN_THREADS, smem, stream, (const float*)records, req_indptr, slots, state, out,
-                    requests, least, heads, dim, max_slots);
+  tl::launch_apart<delta_chunk_scan_kernel>(grid, SCAN_THREADS, true, sm_count(), 0, (size_t)STAGES * STAGE * sizeof(float), stream,
+                                            (const float*)records, req_indptr, slots, state, out, requests, least, heads, dim, max_slots);
   return TL_LAUNCH_CHECK();
 }
 

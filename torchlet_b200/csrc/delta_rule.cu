@@ -358,14 +358,6 @@ bool split_columns(int requests, int heads, int dim, int tokens) {
   return pairs <= sm_count();
 }
 
-// ``apart``: the blocks walk long enough (64 tokens) that their places matter more than the larger shared memory's carve-out.
-template <typename... KArgs, typename... Args>
-void scan_launch(void (*kernel)(KArgs...), dim3 grid, int threads, bool apart, size_t used, cudaStream_t stream, Args... args) {
-  size_t smem = apart ? tl::spread_smem((long long)grid.x * grid.y * grid.z, sm_count(), used) : 0;
-  if (smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) smem = 0;
-  tl::launch_kernel(kernel, grid, threads, smem, stream, args...);
-}
-
 }  // namespace
 
 TL_DEBUG_READER(tl_delta_rule_debug_error)
@@ -409,11 +401,14 @@ int tl_delta_scan(const float* proj, int proj_stride, const float* gates, const 
                    (reinterpret_cast<uintptr_t>(gates) & 15) == 0;
   const bool split = split_columns(requests, heads, dim, tokens);
   // (head sizes up to 64: a chunk of 8 tokens; up to 128: 4 tokens 8.2 -> 7.6 us, 2 equal; beyond: 1 token 20 us against 22)
+  // the blocks walk long enough that their places matter more than the larger shared memory's carve-out
   const bool long_walk = tokens >= 64ll * requests;
   const bool long_portions = vec && (dim > 128 || tokens >= (dim > 64 ? 4ll : 8ll) * requests);
 #define TL_SCAN_INSTANCE(DK, VEC, COLS, LONG)                                                                       \
-  scan_launch(delta_scan_kernel<DK, VEC, COLS, LONG>, grid, COLS * KS / (COLS == DK ? 2 : 1), long_walk,             \
-              sizeof(float) * 2 * scan_chunk(DK) * 6 * DK, stream, proj, proj_stride, gates, req_indptr, slots, state, out, heads, dim, below, max_slots)
+  tl::launch_apart<delta_scan_kernel<DK, VEC, COLS, LONG>>(grid, COLS * KS / (COLS == DK ? 2 : 1), long_walk, sm_count(), \
+                                                          sizeof(float) * 2 * scan_chunk(DK) * 6 * DK, 0, stream, proj,  \
+                                                          proj_stride, gates, req_indptr, slots, state, out, heads, dim, \
+                                                          below, max_slots)
 #define TL_SCAN_COLS(DK, COLS)                          \
   if (long_portions) TL_SCAN_INSTANCE(DK, true, COLS, true);    \
   else if (vec) TL_SCAN_INSTANCE(DK, true, COLS, (DK > 128)); \

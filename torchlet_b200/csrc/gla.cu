@@ -511,14 +511,6 @@ __global__ void rotate_heads_kernel(float* __restrict__ rows, int stride, const 
   head[i + half] = v * c + u * s;
 }
 
-// ``apart``: the blocks walk long enough (64 tokens) that their places matter more than the larger shared memory's carve-out.
-template <typename... KArgs, typename... Args>
-void scan_launch(void (*kernel)(KArgs...), dim3 grid, int threads, bool apart, int sms, size_t used, cudaStream_t stream, Args... args) {
-  size_t smem = apart ? tl::spread_smem((long long)grid.x * grid.y * grid.z, sms, used) : 0;
-  if (smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) smem = 0;
-  tl::launch_kernel(kernel, grid, threads, smem, stream, args...);
-}
-
 }  // namespace
 
 TL_DEBUG_READER(tl_gla_debug_error)
@@ -570,12 +562,13 @@ int tl_gla_scan(const float* proj, int proj_stride, const float* decay, const in
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   }
   const bool narrow = vec && (long long)requests * heads * ((vdim + COLS_NARROW - 1) / COLS_NARROW) <= sms;
+  // the blocks walk long enough that their places matter more than the larger shared memory's carve-out
   const bool long_walk = tokens >= 64ll * requests;
 #define TL_SCAN_ONE(DK, VEC, MODE, COLS)                                                                                   \
-  scan_launch(gla_scan_kernel<DK, VEC, MODE, COLS>, dim3(requests, heads, (vdim + COLS - 1) / COLS),                       \
-              lanes_a_column(DK) * COLS, long_walk, sms, sizeof(float) * STAGES * scan_chunk(DK, MODE) * scan_row(DK, MODE, COLS), \
-              stream, proj, proj_stride, decay, req_indptr, slots, state, out, heads, qk_heads, dim, vdim, below, max_slots, \
-              qscale, bonus, k_offset, v_offset)
+  tl::launch_apart<gla_scan_kernel<DK, VEC, MODE, COLS>>(                                                                  \
+      dim3(requests, heads, (vdim + COLS - 1) / COLS), lanes_a_column(DK) * COLS, long_walk, sms,                          \
+      sizeof(float) * STAGES * scan_chunk(DK, MODE) * scan_row(DK, MODE, COLS), 0, stream, proj, proj_stride, decay,       \
+      req_indptr, slots, state, out, heads, qk_heads, dim, vdim, below, max_slots, qscale, bonus, k_offset, v_offset)
 #define TL_SCAN_MODE(DK, MODE)                                    \
   {                                                               \
     if (narrow) TL_SCAN_ONE(DK, true, MODE, COLS_NARROW);         \
