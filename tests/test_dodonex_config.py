@@ -154,3 +154,20 @@ def test_row_tiles_of_the_latent_attention_start_with_those_that_see_the_most_ke
     seen = [min(before[r] + start // heads + 1, window or 10 ** 9) for r, start in pairs]
     assert seen == sorted(seen, reverse=True)
     assert pairs[0][0] == (0 if window is None else min(r for r, n in enumerate(new) if before[r] + n >= 300))
+
+
+@pytest.mark.parametrize("chunks,room", [([7], 3), ([7], 7), ([5, 2, 9, 2, 1], 5), ([5, 2, 9, 2, 1], 6), ([5, 2, 9, 2, 1], 40), ([1] * 8, 8),
+                                         ([250, 4, 4], 107), ([], 4)])
+def test_passes_of_the_delta_rule_take_every_chunk_once_and_fit(chunks, room):
+    import numpy as np
+
+    from torchlet_b200.ops import delta_chunk_passes
+
+    chunks = np.array(chunks, dtype=np.int64)
+    passes = delta_chunk_passes(chunks, room)
+    assert [lo for lo, _, _ in passes] == [0] * bool(passes) + [hi for _, hi, _ in passes[:-1]]
+    assert (passes[-1][1] if passes else 0) == chunks.max(initial=0)
+    for lo, hi, count in passes:
+        assert hi > lo and count == (np.minimum(chunks, hi) - np.minimum(chunks, lo)).sum() <= room
+        wider = (np.minimum(chunks, hi + 1) - np.minimum(chunks, lo)).sum()
+        assert wider > room or wider == count  # no pass is narrower than it has to be

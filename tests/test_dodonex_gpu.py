@@ -61,6 +61,26 @@ def test_steps_of_many_tokens(dtype):
     cases.assert_close(cases.replay(runner, "b", ids, [30, 270]), want, dtype, "270 behind 30")
 
 
+def test_scratch_memory_of_the_delta_rule_is_that_of_one_token_and_stays():
+    """What the first decode step allocates for the recurrence serves every later step of the token budget: a long portion, and
+    many that each end in a chunk of a few tokens."""
+    from torchlet_b200.engine import StepEntry
+
+    runner = cases.make_runner("R", "bfloat16", slots=20, num_pages=80, budget=512)
+
+    def step(lengths):
+        for r, n in enumerate(lengths):
+            runner.admit(r)
+        runner.step([StepEntry(r, cases.make_ids("R", n, r), []) for r, n in enumerate(lengths)])
+        for r in range(len(lengths)):
+            runner.finish(r)
+        return {key: (t.data_ptr(), t.numel()) for key, t in runner._buffers.items() if key.startswith("delta.")}
+
+    first = step([1])
+    for lengths in ([500], [33] * 15, [1, 480, 3], [41] * 12):
+        assert step(lengths) == first
+
+
 @pytest.mark.parametrize("name", ["P", "R"])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_unequal_batches_with_pages_and_slots_used_again(name, dtype):

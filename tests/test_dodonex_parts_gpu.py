@@ -3,6 +3,7 @@ tests/plain_dodonex.py, at sizes of their own, with inputs designed so that a fa
 key among hundreds, a key at a page's border, stale pages full of NaN, a state that must carry)."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -307,6 +308,35 @@ def test_products_by_heads_in_one_launch(T, H, N, K, gap):
     bound = 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * torch.einsum("thk,hnk->thn", x.double().view(T, H, K).abs(), w.double().abs())
     assert ((got[..., :N].double() - want).abs() <= bound).all()
     assert (got[..., N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("room", [5, 6, 9, 14, 18])
+def test_delta_chunks_in_passes_give_the_bits_of_one(room):
+    """Records for fewer chunks than the step has: the passes cut every request, continue its state and leave the shorter
+    requests and padding lanes alone."""
+    from torchlet_b200 import ops
+
+    lens, least, H, D, rank = [37, 9, 3, 70, 16, 1, 8], 8, 2, 40, 5
+    size, T, R = H * D, sum(lens), len(lens)
+    proj = rand(T, 5 * size + rank, seed=1).to(DEV)
+    w2, w0, bias = rand(rank, size, seed=2, scale=rank ** -0.5).to(DEV), rand(size, seed=3).to(DEV), rand(size, seed=4).to(DEV)
+    indptr = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 1, 0, 4, -1, 5, 2], dtype=torch.int32, device=DEV)
+    each, floats = np.array([-(-n // 8) for n in lens if n >= least]), H * ops.delta_chunk_record()
+    chunks = int(each.sum())
+    assert ops.delta_chunk_tokens() == 8 and chunks == 19
+
+    def run(room):
+        state, out = rand(6, H, D, D, seed=5, scale=0.3).to(DEV), torch.full((T, size), -1.0, device=DEV)
+        records = torch.full((room * floats + 7,), float("nan"), device=DEV)
+        passes = ops.delta_chunk_passes(each, room)
+        assert len(passes) > (room < chunks)
+        ops.delta_chunked(proj, w2, w0, bias, indptr, slots, state, out, records, R, chunks, least, H, D, rank, passes)
+        assert torch.isnan(records[room * floats:]).all()
+        return out, state
+
+    for a, b in zip(run(room), run(chunks)):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("lens,H,D,R,V,rank,page_size", [([128], 1, 64, 16, 64, 64, 16), ([257, 2, 130], 2, 128, 64, 128, 72, 8),

@@ -42,11 +42,16 @@ constexpr int GROUP = CHUNK * COLS / 2 * 4 + CHUNK * COLS, RECORD = COLUMNS + GR
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 
-// Requests of ``least`` tokens and more are cut into chunks, in the order of the requests; the others have none here.
-__device__ __forceinline__ int chunks_of(const int* req_indptr, int requests, int least, int req) {
-  const int n = req < requests ? req_indptr[req + 1] - req_indptr[req] : 0;
-  return n >= least ? (n + CHUNK - 1) / CHUNK : 0;
-}
+// Requests of ``least`` tokens and more are cut into chunks; the others have none here.  A launch takes chunks [lo, hi) of each,
+// in the order of the requests.
+struct Pass {
+  const int* req_indptr;
+  int requests, least, lo, hi;
+  __device__ __forceinline__ int chunks_of(int req) const {
+    const int n = req < requests ? req_indptr[req + 1] - req_indptr[req] : 0;
+    return n >= least ? max(0, min((n + CHUNK - 1) / CHUNK, hi) - lo) : 0;
+  }
+};
 
 // Sums the 64 values of every lane over the warp: lane l is left with values 2 l and 2 l + 1, in v[0] and v[1].
 __device__ __forceinline__ void scatter_sums(float (&v)[64], int lane) {
@@ -64,8 +69,8 @@ __host__ __device__ constexpr int upto(int t, int s) { return 28 + t * (t + 1) /
 
 __global__ void __launch_bounds__(DK)
 delta_chunk_prepare_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ w2t,
-                           const float* __restrict__ w0, const float* __restrict__ a_bias, const int* __restrict__ req_indptr,
-                           float* __restrict__ records, int requests, int least, int heads, int dim, int rank) {
+                           const float* __restrict__ w0, const float* __restrict__ a_bias, const Pass pass,
+                           float* __restrict__ records, int heads, int dim, int rank) {
   tl::pdl_launch_dependents();
   extern __shared__ __align__(16) float lowrank[];  // tanh(l): [rank][CHUNK]
   __shared__ float squares[2][CHUNK];
@@ -75,8 +80,8 @@ delta_chunk_prepare_kernel(const float* __restrict__ proj, int proj_stride, cons
   const int hd = heads * dim;
   // the request and the tokens of this chunk (every warp by itself)
   int id = blockIdx.x, first = -1, count = 0;
-  for (int base = 0; base < requests; base += 32) {
-    const int mine = chunks_of(req_indptr, requests, least, base + lane);
+  for (int base = 0; base < pass.requests; base += 32) {
+    const int mine = pass.chunks_of(base + lane);
     int sum = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -86,8 +91,8 @@ delta_chunk_prepare_kernel(const float* __restrict__ proj, int proj_stride, cons
     const unsigned beyond = __ballot_sync(0xffffffffu, sum > id);
     if (beyond) {
       const int at = __ffs(beyond) - 1;
-      first = req_indptr[base + at] + (id - __shfl_sync(0xffffffffu, sum - mine, at)) * CHUNK;
-      count = min(CHUNK, req_indptr[base + at + 1] - first);
+      first = pass.req_indptr[base + at] + (pass.lo + id - __shfl_sync(0xffffffffu, sum - mine, at)) * CHUNK;
+      count = min(CHUNK, pass.req_indptr[base + at + 1] - first);
       break;
     }
     id -= __shfl_sync(0xffffffffu, sum, 31);
@@ -234,19 +239,19 @@ constexpr int STAGE = (COPIED + 31) / 32 * 32;
 // chosen by lane, lane p walks the tokens and the two vectors in the order of (slot XOR its own number): the slot a lane
 // keeps in a round is always the lower one.
 __global__ void __launch_bounds__(SCAN_THREADS, 2)
-delta_chunk_scan_kernel(const float* __restrict__ records, const int* __restrict__ req_indptr, const int* __restrict__ slots,
-                        float* __restrict__ state, float* __restrict__ out, int requests, int least, int heads, int dim,
-                        int max_slots) {
+delta_chunk_scan_kernel(const float* __restrict__ records, const Pass pass, const int* __restrict__ slots,
+                        float* __restrict__ state, float* __restrict__ out, int heads, int dim, int max_slots) {
   tl::pdl_launch_dependents();
   extern __shared__ __align__(128) float smem[];  // [STAGES][STAGE]
   const int req = blockIdx.x, h = blockIdx.y, group = blockIdx.z, tid = threadIdx.x, lane = tid & 31;
   const int part = lane & 15, pair = (tid >> 5) * 2 + (lane >> 4);  // this lane's rows 4 part .., columns 2 pair and 2 pair + 1
-  const int chunks = chunks_of(req_indptr, requests, least, req);
+  const int chunks = pass.chunks_of(req);
   int before = 0;
-  for (int base = 0; base < req; base += 32) before += base + lane < req ? chunks_of(req_indptr, requests, least, base + lane) : 0;
+  for (int base = 0; base < req; base += 32) before += base + lane < req ? pass.chunks_of(base + lane) : 0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-  const int first = req_indptr[req], last = req_indptr[req + 1];
+  // the request's tokens in this pass
+  const int first = pass.req_indptr[req] + pass.lo * CHUNK, last = min(pass.req_indptr[req + 1], first + chunks * CHUNK);
   tl::pdl_wait();
   if (chunks == 0) return;
   const int hd = heads * dim, col = group * COLS + 2 * pair;
@@ -386,22 +391,25 @@ extern "C" {
 int tl_delta_chunk_tokens() { return CHUNK; }
 int tl_delta_chunk_record() { return RECORD; }
 
-// The requests of at least ``least`` tokens, which have ``chunks`` chunks in all; the others' rows of ``out`` and their states
-// are left as they are.  proj rows, w2t, w0, a_bias as tl_delta_prepare's; state and out as tl_delta_scan's; records: chunks *
+// Chunks [lo, hi) of the requests of at least ``least`` tokens, ``chunks`` in all; the other requests' rows of ``out`` and their
+// states are left as they are.  A step's chunks may go in several such passes, lo ascending: each continues from the states the
+// one before it left, the bits are the same, and the scratch memory need not hold the whole step.
+// proj rows, w2t, w0, a_bias as tl_delta_prepare's; state and out as tl_delta_scan's; records: chunks *
 // heads * tl_delta_chunk_record() floats.  Head sizes up to 64, multiples of 4; everything starts on 16-byte boundaries.
 int tl_delta_chunked(const float* proj, int proj_stride, const float* w2t, const float* w0, const float* a_bias,
                      const int* req_indptr, const int* slots, float* state, float* out, float* records, int requests, int chunks,
-                     int least, int heads, int dim, int rank, int max_slots, cudaStream_t stream) {
+                     int lo, int hi, int least, int heads, int dim, int rank, int max_slots, cudaStream_t stream) {
   if (requests <= 0 || chunks <= 0) return 0;
-  if (dim <= 0 || dim > DK || dim % 4 || heads <= 0 || heads > 65535 || rank <= 0 || rank > 1024 || least < 1 ||
+  if (dim <= 0 || dim > DK || dim % 4 || heads <= 0 || heads > 65535 || rank <= 0 || rank > 1024 || least < 1 || lo < 0 || hi <= lo ||
       (((uintptr_t)state | (uintptr_t)out | (uintptr_t)records) & 15))
     return TL_ERR_UNSUPPORTED;
+  const Pass pass{req_indptr, requests, least, lo, hi};
   tl::launch_kernel(delta_chunk_prepare_kernel, dim3(chunks, heads), DK, (size_t)CHUNK * rank * sizeof(float), stream, proj,
-                    proj_stride, w2t, w0, a_bias, req_indptr, records, requests, least, heads, dim, rank);
-  const dim3 grid(requests, heads, (dim + COLS - 1) / COLS);
+                    proj_stride, w2t, w0, a_bias, pass, records, heads, dim, rank);
   // (the blocks of requests without chunks leave at once; the others walk long enough that their places matter)
-  tl::launch_apart<delta_chunk_scan_kernel>(grid, SCAN_THREADS, true, sm_count(), 0, (size_t)STAGES * STAGE * sizeof(float), stream,
-                                            (const float*)records, req_indptr, slots, state, out, requests, least, heads, dim, max_slots);
+  tl::launch_apart<delta_chunk_scan_kernel>(dim3(requests, heads, (dim + COLS - 1) / COLS), SCAN_THREADS, true, sm_count(), 0,
+                                            (size_t)STAGES * STAGE * sizeof(float), stream, (const float*)records, pass, slots, state,
+                                            out, heads, dim, max_slots);
   return TL_LAUNCH_CHECK();
 }
 

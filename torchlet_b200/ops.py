@@ -11,6 +11,7 @@ import ctypes
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
+import numpy as np
 import torch
 
 from .csrc.build import DEBUG_BUILD, load_library
@@ -168,7 +169,7 @@ _SIGNATURES = {
         "tl_delta_chunk_tokens": [],
         "tl_delta_chunk_record": [],
         "tl_delta_chunked": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "tl_delta_chunked_debug_error": [c_void_p],
     },
     "gla_chunked": {
@@ -574,23 +575,45 @@ def delta_chunk_record() -> int:
     return _fn("delta_chunked", "tl_delta_chunk_record")()
 
 
+def delta_chunk_passes(chunks, room: int) -> list:
+    """How requests of ``chunks`` chunks each (numpy integers, at most ``room`` requests) go in passes of at most ``room`` chunks,
+    as ``delta_chunked`` takes it: [(lo, hi, chunks of the pass)], each pass chunks [lo, hi) of every request, so that all
+    requests are walked side by side."""
+    passes, lo, longest = [], 0, int(chunks.max(initial=0))
+    while lo < longest:
+        left = np.maximum(chunks - lo, 0)
+        fits, beyond = 1, longest - lo + 1  # the widest pass that fits: at least one chunk of every request does
+        if int(left.sum()) <= room:
+            fits = longest - lo
+        while beyond - fits > 1:
+            middle = (fits + beyond) // 2
+            fits, beyond = (middle, beyond) if int(np.minimum(left, middle).sum()) <= room else (fits, middle)
+        passes.append((lo, lo + fits, int(np.minimum(left, fits).sum())))
+        lo += fits
+    return passes
+
+
 def delta_chunked(proj, w2, w0, a_bias, req_indptr, slots, state, out, records, requests: int, chunks: int, least: int,
-                  heads: int, dim: int, rank: int) -> None:
+                  heads: int, dim: int, rank: int, passes=None) -> None:
     """``delta_prepare`` and ``delta_scan`` for the requests of at least ``least`` tokens, ``delta_chunk_tokens()`` tokens a step
     of the recurrence (csrc/delta_chunked.cu); the other requests' rows and states stay as they are.  ``chunks``: how many
-    these requests have in all; ``records``: float32, chunks * heads * delta_chunk_record() numbers."""
+    these requests have in all; ``records``: float32, heads * delta_chunk_record() numbers for each chunk of the largest of
+    ``passes`` (``delta_chunk_passes``; default: all in one; the bits are the same)."""
     _need_cuda(proj, w2, w0, a_bias, req_indptr, slots, state, out, records)
     assert proj.dtype == w2.dtype == w0.dtype == a_bias.dtype == state.dtype == out.dtype == records.dtype == torch.float32
     assert proj.stride(1) == 1 and proj.shape[1] == 5 * heads * dim + rank and w2.is_contiguous() and w2.shape == (rank, heads * dim)
     assert w0.is_contiguous() and a_bias.is_contiguous() and w0.numel() == a_bias.numel() == heads * dim
     assert state.is_contiguous() and out.is_contiguous() and records.is_contiguous()
-    assert out.numel() == proj.shape[0] * heads * dim and records.numel() >= chunks * heads * delta_chunk_record()
+    passes = passes or [(0, 1 << 30, chunks)]
+    assert out.numel() == proj.shape[0] * heads * dim and sum(n for _, _, n in passes) == chunks
+    assert records.numel() >= max(n for _, _, n in passes) * heads * delta_chunk_record()
     assert state.shape[1:] == (heads, dim, dim) and req_indptr.dtype == slots.dtype == torch.int32
-    code = _fn("delta_chunked", "tl_delta_chunked")(proj.data_ptr(), proj.stride(0), w2.data_ptr(), w0.data_ptr(), a_bias.data_ptr(),
-                                                    req_indptr.data_ptr(), slots.data_ptr(), state.data_ptr(), out.data_ptr(),
-                                                    records.data_ptr(), requests, chunks, least, heads, dim, rank, state.shape[0],
-                                                    _stream())
-    _check(code, "delta_chunked", 2)
+    for lo, hi, count in passes:
+        code = _fn("delta_chunked", "tl_delta_chunked")(
+            proj.data_ptr(), proj.stride(0), w2.data_ptr(), w0.data_ptr(), a_bias.data_ptr(), req_indptr.data_ptr(),
+            slots.data_ptr(), state.data_ptr(), out.data_ptr(), records.data_ptr(), requests, count, lo, hi, least, heads, dim,
+            rank, state.shape[0], _stream())
+        _check(code, "delta_chunked", 2)
 
 
 def delta_finish(o, proj, weight, out, heads: int, dim: int, eps: float) -> None:

@@ -33,6 +33,9 @@ from .linear import Linear
 # their larger preparation costs more (32 heads of 64: 1 request of 32 tokens 22 -> 18 us, of 2,048 429 -> 286; 4 of 64
 # 41 -> 37, of 128 61 -> 64, of 512 236 -> 252; 32 of 64 183 -> 245).
 LEAST_CHUNKED, BLOCKS_AN_SM, COLUMNS = 32, 2, 16
+# The chunks' records: as many bytes at most (two passes over half of the chunks each: 2,048 tokens of 32 heads 292 -> 298 us; 121
+# MB in one), but room for so many chunks, and for so many more than whole ones where requests end in a part of one.
+RECORD_BYTES, LEAST_ROOM, PARTIAL_CHUNKS = 128 << 20, 64, 16
 
 
 @functools.lru_cache(maxsize=None)
@@ -80,19 +83,37 @@ class GeneralDeltaMixer(Mixer):
         self.w0, self.a_bias, self.norm_weight = f32("w0"), f32("a.b"), f32("norm")
         self.w2 = f32("w2").t().contiguous()  # [rank, H D]: the threads of a block read consecutive entries
 
-    def _chunked(self, ctx) -> tuple:
-        """(chunks of the requests whose portions go chunk by chunk, whether other requests are in the step).  Only in the
-        bfloat16 engine: the float32 engine's numbers do not depend on how a sequence is cut."""
-        if ctx.decode_only or ctx.dtype != torch.bfloat16 or self.head_dim > 64 or self.head_dim % 4:
-            return 0, True
-        key = ("delta_chunked", self.num_heads, self.head_dim)
+    def _scratch_rows(self, rows: int, chunked: bool) -> tuple:
+        """(rows of the scratch memory of an engine whose steps bring up to ``rows`` tokens, chunks it has room for).  It holds the
+        gates, [tokens, H 3 D], and in their turn the records of a step's chunks (2.4 times the gates at D 64), but no more than
+        ``RECORD_BYTES`` of them: a step of more chunks goes in passes.  The size does not depend on the step, so the first one
+        allocates it for good."""
+        if not chunked:
+            return rows, 0
+        record = self.num_heads * ops.delta_chunk_record()
+        room = -(-rows // ops.delta_chunk_tokens()) + PARTIAL_CHUNKS
+        room = max(LEAST_ROOM, min(room, RECORD_BYTES // (4 * record)))
+        return max(rows, -(-room * record // (3 * self.size))), room
+
+    def _plan(self, ctx, tokens: int) -> tuple:
+        """(scratch memory, its rows for the gates, the passes of the requests whose portions go chunk by chunk, their chunks,
+        whether other requests are in the step), the same for every such layer of a step.  Chunks only in the bfloat16 engine: the
+        float32 engine's numbers do not depend on how a sequence is cut."""
+        key = ("delta_rule", self.num_heads, self.head_dim)
         plan = ctx.plans.get(key)
         if plan is None:
-            lengths = np.diff(ctx.req_indptr_host)
-            long = lengths[lengths >= LEAST_CHUNKED]
-            if long.size * self.num_heads * -(-self.head_dim // COLUMNS) > BLOCKS_AN_SM * _sm_count(torch.cuda.current_device()):
-                long = long[:0]
-            plan = ctx.plans[key] = (int((-(-long // ops.delta_chunk_tokens())).sum()), long.size < lengths.size)
+            chunked = ctx.dtype == torch.bfloat16 and self.head_dim <= 64 and self.head_dim % 4 == 0
+            rows, room = self._scratch_rows(max(ctx.token_capacity, tokens), chunked)
+            work = ctx.buffer(f"delta.work{self.head_dim}", (rows, 3 * self.size), torch.float32)
+            passes, chunks, others = None, 0, True
+            if chunked and not ctx.decode_only:
+                lengths = np.diff(ctx.req_indptr_host)
+                long = lengths[lengths >= LEAST_CHUNKED]
+                blocks = long.size * self.num_heads * -(-self.head_dim // COLUMNS)
+                if 0 < long.size <= room and blocks <= BLOCKS_AN_SM * _sm_count(torch.cuda.current_device()):
+                    each = -(-long // ops.delta_chunk_tokens())
+                    passes, chunks, others = ops.delta_chunk_passes(each, room), int(each.sum()), long.size < lengths.size
+            plan = ctx.plans[key] = (work, work[:tokens], passes, chunks, others)
         return plan
 
     def forward(self, ctx, x, acc, cache) -> None:
@@ -100,17 +121,14 @@ class GeneralDeltaMixer(Mixer):
         proj = ctx.buffer("delta.proj", (tokens, 5 * self.size + self.rank), torch.float32)
         self.in_proj.forward(x, proj)
         o = ctx.buffer("delta.o", (tokens, self.size), torch.float32)
-        chunks, others = self._chunked(ctx)
+        work, gates, passes, chunks, others = self._plan(ctx, tokens)
         if others:
-            gates = ctx.buffer("delta.gates", (tokens, H * 3 * D), torch.float32)
             ops.delta_prepare(proj, self.w2, self.w0, self.a_bias, gates, H, D, self.rank)
             ops.delta_scan(proj, gates, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D,
                            below=LEAST_CHUNKED if chunks else None)
-        if chunks:
-            length = ops.delta_chunk_tokens()
-            records = ctx.buffer("delta.records", (chunks * length, H * ops.delta_chunk_record() // length), torch.float32)
-            ops.delta_chunked(proj, self.w2, self.w0, self.a_bias, ctx.req_indptr, ctx.slots, cache.state, o, records,
-                              ctx.num_requests, chunks, LEAST_CHUNKED, H, D, self.rank)
+        if chunks:  # their records take the place of the gates, which nothing reads any more
+            ops.delta_chunked(proj, self.w2, self.w0, self.a_bias, ctx.req_indptr, ctx.slots, cache.state, o, work,
+                              ctx.num_requests, chunks, LEAST_CHUNKED, H, D, self.rank, passes)
         out = ctx.buffer("delta.out", (tokens, self.size), ctx.dtype)
         ops.delta_finish(o, proj, self.norm_weight, out, H, D, self.eps)
         if not self.o_proj.accumulate_later(ctx, out, acc):
