@@ -171,3 +171,15 @@ def test_passes_of_the_delta_rule_take_every_chunk_once_and_fit(chunks, room):
         assert hi > lo and count == (np.minimum(chunks, hi) - np.minimum(chunks, lo)).sum() <= room
         wider = (np.minimum(chunks, hi + 1) - np.minimum(chunks, lo)).sum()
         assert wider > room or wider == count  # no pass is narrower than it has to be
+
+
+@pytest.mark.parametrize("lengths,least", [
+    ([2048], 32), ([32, 50], 32),  # nobody else: the token-wise kernels do not run
+    ([31], 96), ([1, 200], 256), ([1, 300], 256),  # a scan of few requests and many tokens is quick
+    ([1] * 8 + [95], 96), ([1] * 8 + [96, 40], 96), ([1] * 32 + [500], 96), ([1] * 8 + [900], 256)])
+def test_portions_of_the_delta_rule_that_go_in_chunks(lengths, least):
+    import numpy as np
+
+    from torchlet_b200.parts.delta_rule import portions_in_chunks
+
+    assert portions_in_chunks(np.array(lengths)) == least

@@ -107,3 +107,14 @@ def test_plain_recurrence_in_portions_and_plain_window():
                                        torch.eye(9, dtype=torch.float64), 1.0, None, 3)
     assert torch.allclose(out[8], torch.tensor([0, 0, 0, 0, 0, 0, .25, .25, .25], dtype=torch.float64))
     assert torch.allclose(out[0], torch.tensor([.5, 0, 0, 0, 0, 0, 0, 0, 0], dtype=torch.float64))
+
+
+@pytest.mark.parametrize("lengths,least", [
+    ([1] * 8 + [319], 0), ([1] * 8 + [320], 192), ([319], 0), ([1, 160, 160], 0), ([192, 192, 191], 192), ([1] * 64, 0),
+    ([64] * 16, 64), ([63] * 20, 0), ([1, 1023], 192), ([1, 1024], 64)])
+def test_portions_of_the_linear_attention_that_go_in_chunks(lengths, least):
+    import numpy as np
+
+    from torchlet_b200.parts.gla import portions_in_chunks
+
+    assert portions_in_chunks(np.array(lengths)) == least

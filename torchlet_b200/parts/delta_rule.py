@@ -32,7 +32,20 @@ from .linear import Linear
 # blocks of 16 columns an SM at most: the chunks shorten a chain that waits; where blocks enough are there to fill its waits,
 # their larger preparation costs more (32 heads of 64: 1 request of 32 tokens 22 -> 18 us, of 2,048 429 -> 286; 4 of 64
 # 41 -> 37, of 128 61 -> 64, of 512 236 -> 252; 32 of 64 183 -> 245).
-LEAST_CHUNKED, BLOCKS_AN_SM, COLUMNS = 32, 2, 16
+# Beside other requests, which keep the two token-wise kernels, two kernels more have to be won back (32 heads of 64 and 8
+# decoding requests: 32 tokens 33 -> 36 us, 64 44 -> 44, 96 61 -> 52, 128 77 -> 59, 512 258 -> 153), all the more where the step
+# brings 64 tokens a request, since the token-wise scan of all then splits its columns (1 decoding request: 128 tokens 49 -> 58,
+# 192 63 -> 66, 256 77 -> 74, 512 132 -> 119).
+LEAST_CHUNKED, LEAST_BESIDE, LEAST_BESIDE_FEW, BLOCKS_AN_SM, COLUMNS = 32, 96, 256, 2, 16
+
+
+def portions_in_chunks(lengths) -> int:
+    """The fewest tokens of a portion that goes chunk by chunk in a step of requests with so many (numpy integers)."""
+    if lengths.min() >= LEAST_CHUNKED:
+        return LEAST_CHUNKED
+    return LEAST_BESIDE_FEW if lengths.sum() >= 64 * lengths.size else LEAST_BESIDE
+
+
 # The chunks' records: as many bytes at most (two passes over half of the chunks each: 2,048 tokens of 32 heads 292 -> 298 us; 121
 # MB in one), but room for so many chunks, and for so many more than whole ones where requests end in a part of one.
 RECORD_BYTES, LEAST_ROOM, PARTIAL_CHUNKS = 128 << 20, 64, 16
@@ -45,7 +58,7 @@ def _sm_count(device_index: int) -> int:
 
 @MIXERS.register("general_delta")
 class GeneralDeltaMixer(Mixer):
-    graph_safe = True  # nothing is planned on the host: requests and slots are read on the device
+    graph_safe = True  # a step of single tokens plans nothing on the host: requests and slots are read on the device
 
     def __init__(self, spec: PartSpec):
         super().__init__(spec)
@@ -96,8 +109,8 @@ class GeneralDeltaMixer(Mixer):
         return max(rows, -(-room * record // (3 * self.size))), room
 
     def _plan(self, ctx, tokens: int) -> tuple:
-        """(scratch memory, its rows for the gates, the passes of the requests whose portions go chunk by chunk, their chunks,
-        whether other requests are in the step), the same for every such layer of a step.  Chunks only in the bfloat16 engine: the
+        """(scratch memory, its rows for the gates, the passes of the requests whose portions go chunk by chunk, their chunks and
+        fewest tokens, whether other requests are in the step), the same for every such layer of a step.  Chunks only in the bfloat16 engine: the
         float32 engine's numbers do not depend on how a sequence is cut."""
         key = ("delta_rule", self.num_heads, self.head_dim)
         plan = ctx.plans.get(key)
@@ -105,15 +118,16 @@ class GeneralDeltaMixer(Mixer):
             chunked = ctx.dtype == torch.bfloat16 and self.head_dim <= 64 and self.head_dim % 4 == 0
             rows, room = self._scratch_rows(max(ctx.token_capacity, tokens), chunked)
             work = ctx.buffer(f"delta.work{self.head_dim}", (rows, 3 * self.size), torch.float32)
-            passes, chunks, others = None, 0, True
-            if chunked and not ctx.decode_only:
+            passes, chunks, least, others = None, 0, 0, True
+            if chunked and not ctx.decode_only and ctx.max_q_len >= LEAST_CHUNKED:
                 lengths = np.diff(ctx.req_indptr_host)
-                long = lengths[lengths >= LEAST_CHUNKED]
+                least = portions_in_chunks(lengths)
+                long = lengths[lengths >= least]
                 blocks = long.size * self.num_heads * -(-self.head_dim // COLUMNS)
                 if 0 < long.size <= room and blocks <= BLOCKS_AN_SM * _sm_count(torch.cuda.current_device()):
                     each = -(-long // ops.delta_chunk_tokens())
                     passes, chunks, others = ops.delta_chunk_passes(each, room), int(each.sum()), long.size < lengths.size
-            plan = ctx.plans[key] = (work, work[:tokens], passes, chunks, others)
+            plan = ctx.plans[key] = (work, work[:tokens], passes, chunks, least, others)
         return plan
 
     def forward(self, ctx, x, acc, cache) -> None:
@@ -121,14 +135,14 @@ class GeneralDeltaMixer(Mixer):
         proj = ctx.buffer("delta.proj", (tokens, 5 * self.size + self.rank), torch.float32)
         self.in_proj.forward(x, proj)
         o = ctx.buffer("delta.o", (tokens, self.size), torch.float32)
-        work, gates, passes, chunks, others = self._plan(ctx, tokens)
+        work, gates, passes, chunks, least, others = self._plan(ctx, tokens)
         if others:
             ops.delta_prepare(proj, self.w2, self.w0, self.a_bias, gates, H, D, self.rank)
             ops.delta_scan(proj, gates, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D,
-                           below=LEAST_CHUNKED if chunks else None)
+                           below=least if chunks else None)
         if chunks:  # their records take the place of the gates, which nothing reads any more
             ops.delta_chunked(proj, self.w2, self.w0, self.a_bias, ctx.req_indptr, ctx.slots, cache.state, o, work,
-                              ctx.num_requests, chunks, LEAST_CHUNKED, H, D, self.rank, passes)
+                              ctx.num_requests, chunks, least, H, D, self.rank, passes)
         out = ctx.buffer("delta.out", (tokens, self.size), ctx.dtype)
         ops.delta_finish(o, proj, self.norm_weight, out, H, D, self.eps)
         if not self.o_proj.accumulate_later(ctx, out, acc):

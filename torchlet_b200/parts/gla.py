@@ -27,15 +27,24 @@ from .linear import Linear
 
 
 # Tokens from which on a request's portion goes chunk by chunk in the bfloat16 engine (csrc/gla_chunked.cu): few tokens are
-# through the scan before three kernels have ended (16 heads of 64 x 128, one request: 128 tokens 21 us against 33, 256 38
-# against 36, 2,048 275 against 76), many keep all SMs at work (4 x 128: 41 against 37; 32 x 64: 128 against 85; but 64 x 32:
-# 137 against 136, 128 x 16: 159 against 343).
-LEAST_ALONE, LEAST_OF_MANY, MANY = 192, 64, 1024
+# through the scan before three kernels have ended (16 heads of 64 x 128, one request: 128 tokens 20 us against 33, 192 29
+# against 35, 256 37 against 36, 320 46 against 35, 2,048 275 against 76), many keep all SMs at work (4 x 128: 41 against 37; 32 x
+# 64: 128 against 85; but 64 x 32: 137 against 136, 128 x 16: 159 against 343).  Beside decoding requests the chunks win earlier on
+# the GPU (8 of them: 128 tokens 47 against 35, 256 85 against 35), but a step of fewer than ``FEW`` tokens in chunks waits for
+# the host, which launches three kernels a layer more (8 + 256 tokens at eight layers: 2.07 ms a step against 2.18).
+LEAST_ALONE, LEAST_OF_MANY, FEW, MANY = 192, 64, 320, 1024
+
+
+def portions_in_chunks(lengths) -> int:
+    """The fewest tokens of a portion that goes chunk by chunk in a step of requests with so many (numpy integers); 0: none."""
+    if lengths[lengths >= LEAST_OF_MANY].sum() >= MANY:
+        return LEAST_OF_MANY
+    return LEAST_ALONE if lengths[lengths >= LEAST_ALONE].sum() >= FEW else 0
 
 
 @MIXERS.register("gated_linear_attention")
 class GatedLinearAttention(Mixer):
-    graph_safe = True  # nothing is planned on the host: requests and slots are read on the device
+    graph_safe = True  # a step of single tokens plans nothing on the host: requests and slots are read on the device
 
     def __init__(self, spec: PartSpec):
         super().__init__(spec)
@@ -80,14 +89,14 @@ class GatedLinearAttention(Mixer):
     def _chunked(self, ctx, proj) -> tuple:
         """(chunks of the requests whose portions go chunk by chunk, the fewest tokens of one, whether other requests are in
         the step).  Only in the bfloat16 engine: the float32 engine's numbers do not depend on how a sequence is cut."""
-        if (ctx.decode_only or ctx.dtype != torch.bfloat16 or self.head_dim > 64 or self.head_dim % 4 or self.v_dim % 4
-                or proj.stride(0) % 4):
+        if (ctx.decode_only or ctx.max_q_len < LEAST_OF_MANY or ctx.dtype != torch.bfloat16 or self.head_dim > 64
+                or self.head_dim % 4 or self.v_dim % 4 or proj.stride(0) % 4):
             return 0, 0, True
         plan = ctx.plans.get("gla_chunked")
         if plan is None:
             lengths = np.diff(ctx.req_indptr_host)
-            least = LEAST_OF_MANY if lengths[lengths >= LEAST_OF_MANY].sum() >= MANY else LEAST_ALONE
-            long = lengths[lengths >= least]
+            least = portions_in_chunks(lengths)
+            long = lengths[lengths >= least] if least else lengths[:0]
             plan = ctx.plans["gla_chunked"] = (int((-(-long // ops.gla_chunk_tokens())).sum()), least, long.size < lengths.size)
         return plan
 

@@ -90,13 +90,13 @@ def prompt_tiles(ctx):
     """(tile_req, tile_row, tiles) for a step of whole prompts on csrc/latent_prompt.cu, planned once a step, or None where some
     request decodes or has cached tokens (whose keys would have to be expanded in every step), or where the step has fewer
     tokens than the per-head products of the latent form take."""
-    if ctx.decode_only:
+    if ctx.decode_only or ctx.num_tokens < MIN_TOKENS_FOR_HEAD_PRODUCTS:
         return None
     plan = ctx.plans.get("latent_attention.prompt", False)
     if plan is False:
         lengths = np.diff(ctx.req_indptr_host)
         plan = None
-        if int(lengths.sum()) >= MIN_TOKENS_FOR_HEAD_PRODUCTS and lengths.min() > 1 and not ctx.kv_before_host[:lengths.size].any():
+        if lengths.min() > 1 and not ctx.kv_before_host[:lengths.size].any():
             step = ops.latent_prompt_tokens()
             tiles = [(row, r) for r, n in enumerate(lengths) for row in range(0, int(n), step)]
             tiles.sort(key=lambda t: -min(t[0] + step, int(lengths[t[1]])))  # those that see the most keys first
