@@ -49,6 +49,27 @@ def test_the_stream_after_every_layer(dtype):
         cases.assert_close(got.cpu(), want.float(), dtype, f"stream after layer {i}")
 
 
+def test_scratch_memory_of_the_linear_attention_stays():
+    """What the first long portion allocates for its chunks serves every later step of the token budget, such as one whose
+    requests each end in a chunk of one token."""
+    from torchlet_b200.engine import StepEntry
+
+    runner = cases.make_runner(cases.variant("R", "bfloat16"), "bfloat16", slots=20, num_pages=80, budget=512)
+
+    def step(lengths):
+        for r, n in enumerate(lengths):
+            runner.admit(r)
+        runner.step([StepEntry(r, cases.make_ids("R", n, r), []) for r, n in enumerate(lengths)])
+        for r in range(len(lengths)):
+            runner.finish(r)
+        return {key: (t.data_ptr(), t.numel()) for key, t in runner._buffers.items() if key.startswith("gla.")}
+
+    first = step([500])
+    assert any(key.startswith("gla.chunks") for key in first)
+    for lengths in ([257, 255], [193, 193, 1], [320, 64, 64]):
+        assert step(lengths) == first
+
+
 @pytest.mark.parametrize("name", ["P", "Q", "R"])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_prefill_then_token_by_token(name, dtype):

@@ -112,8 +112,10 @@ class GatedLinearAttention(Mixer):
             ops.gla_scan(proj, decay, ctx.req_indptr, ctx.slots, cache.state, o, ctx.num_requests, H, D, V, D ** -0.5,
                          below=least if chunks else None)
         if chunks:
-            length = ops.gla_chunk_tokens()
-            workspace = ctx.buffer("gla.chunks", (chunks * length, -(-H * (D * V + 64) // length)), torch.float32)
+            # room for the chunks of any step of the token budget: portions of a chunk and a token have two chunks each
+            rows = max(ctx.token_capacity, tokens)
+            most = 2 * -(-rows // ops.gla_chunk_tokens())
+            workspace = ctx.buffer("gla.chunks", (rows, -(-most * H * (D * V + 64) // rows)), torch.float32)
             ops.gla_chunked(proj, decay, ctx.req_indptr, ctx.slots, cache.state, o, workspace, ctx.num_requests, chunks,
                             least, H, D, V, D ** -0.5)
         out = ctx.buffer("gla.out", (tokens, self.v_size), ctx.dtype)
