@@ -80,7 +80,7 @@ def bench_attention(args) -> None:
     scale = d ** -0.5
     group = nh // nkv
     if q_len == 1:
-        splits = args.splits or decode_splits(n, nkv, total, head_dim=d)
+        splits = args.splits or decode_splits(n, nkv, total, head_dim=d, page_size=page)
         run = lambda i: ops.attention_mma(qkv, pages, table, indptr, kv_before, None, None, n, out, n, nh, nkv, d, page,
                                           None, scale, rows16=True, splits=splits)
         kv_bytes = n * total * 2 * nkv * d * 2
@@ -143,7 +143,7 @@ def bench_mixed_attention(args) -> None:
     token_req = to(list(range(n)) + [n] * portion)
     scale = d ** -0.5
     p_splits = prompt_splits(len(starts) * nkv, behind + portion)
-    d_splits = decode_splits(n, nkv, max(lengths), head_dim=d)
+    d_splits = decode_splits(n, nkv, max(lengths), head_dim=d, page_size=page)
 
     def run(beside: bool) -> None:
         merge = ops.attention_tc(qkv, pages, table, indptr, kv_before, tile_req, tile_row, len(starts), out, nh, nkv, d,

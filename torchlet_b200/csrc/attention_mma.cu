@@ -1067,13 +1067,17 @@ bool decode_tma_enabled() {
   return value == 1;
 }
 
+// Whether 16-row tiles run on the decode kernel: pages its TMA boxes divide a key tile into.
+bool takes_decode_kernel(int page_size) {
+  return decode_tma_enabled() && page_size >= 8 && page_size % 8 == 0 && BLOCK_N % page_size == 0;
+}
+
 template <int D, bool EXTRAS>
 int launch_for(const Params& p, long long num_pages, int tiles, bool rows16, cudaStream_t stream) {
   if (!rows16) return launch<D, false, EXTRAS>(p, tiles, stream);
   CUtensorMap map_kv;
   memset(&map_kv, 0, sizeof(map_kv));
-  const bool tma = decode_tma_enabled() && num_pages > 0 && p.page_size >= 8 && p.page_size % 8 == 0 &&
-                   BLOCK_N % p.page_size == 0 &&
+  const bool tma = num_pages > 0 && takes_decode_kernel(p.page_size) &&
                    cached_map(&map_kv, p.pages, (uint64_t)num_pages * 2 * p.nkv * p.page_size, D, (uint32_t)p.page_size);
   return tma ? launch_decode<D, EXTRAS>(map_kv, p, tiles, stream) : launch<D, true, EXTRAS>(p, tiles, stream);
 }
@@ -1088,6 +1092,9 @@ extern "C" {
 long long tl_attention_mma_workspace(int tiles, int nh, int d, int splits) {
   return splits > 1 ? (long long)tiles * nh * splits * (d + 2) * 4 : 0;
 }
+
+// CTAs of a decode step (16-row tiles) that lie on an SM together.
+int tl_attention_mma_decode_ctas(int d, int page_size) { return takes_decode_kernel(page_size) ? decode_ctas(d) : 3; }
 
 // Reads and clears the code that a bounded wait left when it gave up (0: none).
 int tl_attention_mma_error() {

@@ -8,6 +8,7 @@ a kernel refuses, or a missing library is an error here.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
@@ -75,6 +76,7 @@ _SIGNATURES = {
                                 c_int, c_int, c_void_p, c_longlong, c_void_p, c_int, c_float, c_int, c_void_p, c_void_p,
                                 c_longlong, c_void_p, c_void_p, c_void_p],
         "tl_attention_mma_error": [],
+        "tl_attention_mma_decode_ctas": [c_int, c_int],
         "tl_attention_mma_debug_error": [c_void_p],
     },
     "decode_fused": {
@@ -1819,6 +1821,12 @@ def attention_mixed_decode_error() -> int:
 def attention_spread_error() -> int:
     """0, or the code a bounded wait in the prompt kernel for mixed scores left when it gave up."""
     return _fn("attention_spread", "tl_attention_spread_error")()
+
+
+@functools.lru_cache(maxsize=None)
+def attention_mma_decode_ctas(d: int, page_size: int) -> int:
+    """CTAs of ``attention_mma`` with 16-row tiles that lie on an SM together."""
+    return _fn("attention_mma", "tl_attention_mma_decode_ctas")(d, page_size)
 
 
 def attention_mma_error() -> int:

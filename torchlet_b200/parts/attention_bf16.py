@@ -32,17 +32,18 @@ def _sm_count(device_index: int) -> int:
     return torch.cuda.get_device_properties(device_index).multi_processor_count
 
 
-def decode_splits(num_requests: int, num_kv_heads: int, max_kv_len: int, device=None, head_dim: int = 128) -> int:
+def decode_splits(num_requests: int, num_kv_heads: int, max_kv_len: int, device=None, head_dim: int = 128,
+                  page_size: int = 16) -> int:
     """CTAs the grid of a decode step holds for the keys of one (request, KV head): as many as
-    fill ONE wave (two CTAs are resident per SM at head_dim 128, three at 64), at most 64, and no more than the longest
-    request the step may meet could use at 192 keys a split (three of the kernel's key tiles; 128
+    fill ONE wave (two CTAs are resident per SM at head_dim 128, three at 64 and where the page size does not suit the
+    decode kernel), at most 64, and no more than the longest request the step may meet could use at 192 keys a split (three of the kernel's key tiles; 128
     and 256 were measured: 192 is 0.4-0.9 % of a decode step better at batch 1 to 4).  ``max_kv_len`` is that longest
     length: the step's own longest request, or, where the step is captured in a CUDA graph, the
     engine's length limit.  How many of them a request really uses is decided on the device from
     its own length (csrc/attention_mma.cu, ``effective_splits``), so a grid sized for the limit
     costs a short request nothing but CTAs that leave at once."""
     index = torch.cuda.current_device() if device is None or device.index is None else device.index
-    resident = (2 if head_dim == 128 else 3) * _sm_count(index)
+    resident = ops.attention_mma_decode_ctas(head_dim, page_size) * _sm_count(index)
     room = max(1, resident // max(1, num_requests * num_kv_heads))
     return max(1, min(room, -(-max_kv_len // MIN_KEYS_A_SPLIT), 64))
 
@@ -145,7 +146,7 @@ def forward(mixer, ctx, qkv, cache, out, gate=None, prior=None) -> bool:
             softcap=softcap, sink=sink, gate=gate, prior=prior)
     if plan["decode"] is not None:
         tile_req, count = plan["decode"]
-        splits = decode_splits(count, nkv, ctx.max_kv_len, qkv.device, d)
+        splits = decode_splits(count, nkv, ctx.max_kv_len, qkv.device, d, cache.page_size)
         ops.attention_mma(qkv, cache.pages, cache.block_table, ctx.req_indptr, ctx.kv_before, tile_req, None,
                           count, rows16=True, splits=splits, late_wait=beside, **common)
     if merge_portions is not None:
