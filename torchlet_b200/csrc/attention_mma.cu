@@ -31,6 +31,7 @@
 #include <math.h>
 
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "common.cuh"
@@ -722,13 +723,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const Params
     if (num_tiles > 0) request(0, 0, page);
     for (int t = 0; t < num_tiles && !*abort_flag; ++t) {
       const int page_after = page_of(t + 2);  // read a tile before it is needed
-      // Keys come a tile before the values, except where the next keys would have to wait for the preceding kernel, by themselves
-      // (the step's own token's) or for the ring (whose readers wait for q): old values are requested ahead of that wait.
-      const bool values_first = !waited && t < STAGES && t + 1 < num_tiles &&
-                                (t + 1 == STAGES || (tile_begin + t + 1) * BLOCK_N + BLOCK_N - 1 >= before);
-      if (values_first) request(t, 1, page);
       if (t + 1 < num_tiles) request(t + 1, 0, page_next);
-      if (!values_first) request(t, 1, page);
+      request(t, 1, page);
       page = page_next;
       page_next = page_after;
     }
