@@ -514,7 +514,8 @@ def test_router_options_and_ties():
 
 
 @pytest.mark.parametrize("tokens,hidden,experts,top,dtype", [(1184, 2048, 8, 2, torch.bfloat16), (1191, 72, 40, 3, torch.bfloat16),
-                                                             (1300, 500, 8, 1, torch.float32), (1187, 1000, 33, 4, torch.bfloat16)])
+                                                             (1300, 500, 8, 1, torch.float32), (1187, 1000, 33, 4, torch.bfloat16),
+                                                             (1200, 12288, 4, 2, torch.bfloat16)])
 def test_routing_many_tokens_gives_the_bits_of_one(tokens, hidden, experts, top, dtype):
     """From eight tokens an SM on a block takes eight tokens: choices, weights and the always-on expert's gate are those of a
     step of one token."""

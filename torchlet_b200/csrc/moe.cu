@@ -30,9 +30,23 @@ using namespace tl;
 constexpr int ROUTE_WARPS = 16;  // router rows taken side by side (8: ten rows and a gate's row took two rounds of loads)
 constexpr int MAX_EXPERTS = 256;
 
-// TOKENS router logits (rows ``row``, ``stride`` apart, in shared memory) of one expert by one warp: each lane sums its 32nd of
-// a row in eight independent chains (k = lane, lane + 32, ... in turn; eight loads in flight), so a logit's order of additions
-// depends on the width alone.
+// One router logit by one warp: each lane sums its 32nd of the row in eight independent chains (k = lane,
+// lane + 32, ... in turn; eight loads in flight), so a logit's order of additions depends on the width alone.
+template <typename Row>
+__device__ __forceinline__ float router_logit(const Row* __restrict__ row, const float* __restrict__ w, int hidden, int lane) {
+  float p[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) p[i] = 0.f;
+  int k = lane;
+  for (; k + 224 < hidden; k += 256) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i] = fmaf(to_float(row[k + 32 * i]), w[k + 32 * i], p[i]);
+  }
+  for (; k < hidden; k += 32) p[0] = fmaf(to_float(row[k]), w[k], p[0]);
+  return warp_sum(((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])));
+}
+
+// The same for TOKENS rows (``row``, ``stride`` apart, in shared memory) that share the router's row: the bits are the same.
 template <int TOKENS, typename Row>
 __device__ __forceinline__ void router_logits(float (&out)[TOKENS], const Row* __restrict__ row, int stride, const float* __restrict__ w,
                                               int hidden, int lane) {
@@ -60,6 +74,7 @@ __device__ __forceinline__ void router_logits(float (&out)[TOKENS], const Row* _
   for (int t = 0; t < TOKENS; ++t)
     out[t] = warp_sum(((p[t][0] + p[t][1]) + (p[t][2] + p[t][3])) + ((p[t][4] + p[t][5]) + (p[t][6] + p[t][7])));
 }
+
 // One warp: from a token's router logits (``score``, shared memory, overwritten) to its ``top`` experts and
 // their weights.
 // ``groups`` > 1 with ``keep`` < groups: the experts form ``groups`` equal groups of neighbours, a group is scored by
@@ -152,18 +167,53 @@ __device__ __forceinline__ void choose_experts(float* score, float* pick, const 
     for (int j = lane; j < top; j += 32) weight[j] = (renormalize ? weight[j] / (total + renorm_eps) : weight[j]) * scale;
 }
 
-// A block takes TOKENS tokens, whose rows are staged in shared memory, and a warp the logits of one expert for EACH of them at
-// a time; the first TOKENS warps then choose, a token each.  One token a block reads the whole router from the L2 for every
-// token, which is what many tokens' time goes into (2,048 tokens, 8 experts, 2,048 wide: 22.8 us a token a block, 13.1 with
-// eight); few tokens have the GPU to themselves and wait for one another only with more.  The bits are the same.
-constexpr int ROUTE_TOKENS = 8, ROUTE_EACH = 4;
-template <typename T, int TOKENS, int EACH>
+// One block per token.  The token's row is staged in shared memory as floats; warp w takes the
+// experts w, w + ROUTE_WARPS, ...; the first warp then chooses.
+template <typename T>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
 moe_route_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ router, const float* __restrict__ router_bias,
                  int* __restrict__ choice,
                  float* __restrict__ weight, int tokens, int hidden, int experts, int top, int score_mode,
                  int renormalize, int groups, int keep, float renorm_eps, const float* __restrict__ correction,
                  float scale, const float* __restrict__ gate_w, float* __restrict__ gate_out) {
+  tl::pdl_launch_dependents();
+  tl::pdl_wait();
+  extern __shared__ float xrow[];  // hidden floats
+  __shared__ float all_scores[MAX_EXPERTS];
+  __shared__ float picks[MAX_EXPERTS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x;
+  const T* row = x + (size_t)t * ldx;
+  for (int k = threadIdx.x; k < hidden; k += ROUTE_WARPS * 32) xrow[k] = to_float(row[k]);
+  __syncthreads();
+  for (int e = warp; e < experts; e += ROUTE_WARPS) {
+    const float part = router_logit(xrow, router + (size_t)e * hidden, hidden, lane);
+    if (lane == 0) all_scores[e] = router_bias ? part + router_bias[e] : part;
+  }
+  // a gate of one number a token beside the router (an always-on expert's): sigmoid(gate_w . x), by the last warp
+  if (gate_w && warp == ROUTE_WARPS - 1) {
+    const float z = router_logit(xrow, gate_w, hidden, lane);
+    if (lane == 0) gate_out[t] = 1.f / (1.f + expf(-z));
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  choose_experts(all_scores, correction ? picks : all_scores, correction, experts, top, score_mode, renormalize, lane,
+                 choice + (size_t)t * top, weight + (size_t)t * top, groups, keep, renorm_eps, scale);
+}
+
+// Many tokens: a block takes TOKENS, whose rows are staged in shared memory, and a warp the logits of one expert for EACH of them
+// at a time; the first TOKENS warps then choose, a token each.  One token a block reads the whole router from the L2 for every
+// token, which is what many tokens' time goes into (2,048 tokens, 8 experts, 2,048 wide: 22.8 us a token a block, 13.1 with
+// eight); few tokens have the GPU to themselves, and one a block in this form costs a decode step of eight layers 20 us (its
+// reads of the router are not as far ahead).  The bits are the same.
+constexpr int ROUTE_TOKENS = 8, ROUTE_EACH = 4;
+template <typename T>
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_many_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ router, const float* __restrict__ router_bias,
+                      int* __restrict__ choice, float* __restrict__ weight, int tokens, int hidden, int experts, int top,
+                      int score_mode, int renormalize, int groups, int keep, float renorm_eps, const float* __restrict__ correction,
+                      float scale, const float* __restrict__ gate_w, float* __restrict__ gate_out) {
+  constexpr int TOKENS = ROUTE_TOKENS, EACH = ROUTE_EACH;
   tl::pdl_launch_dependents();
   tl::pdl_wait();
   extern __shared__ __align__(16) unsigned char rows_raw[];  // [TOKENS][hidden]
@@ -393,6 +443,14 @@ moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ position
   }
 }
 
+int sm_count() {
+  static const int sms = [] {
+    int device = 0, n = 0;
+    return cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+  }();
+  return sms;
+}
+
 }  // namespace
 
 extern "C" {
@@ -412,19 +470,23 @@ int tl_moe_route(const void* x, int ldx, int dtype, const float* router, const f
     return TL_ERR_UNSUPPORTED;
   if (groups < 1 || keep < 1 || keep > groups || experts % groups || top > keep * (experts / groups) || groups > 2048)
     return TL_ERR_UNSUPPORTED;
-  if ((size_t)hidden * sizeof(float) > 48 * 1024) return TL_ERR_UNSUPPORTED;
-  const size_t row = (size_t)hidden * (dtype == TL_DTYPE_F32 ? sizeof(float) : sizeof(__nv_bfloat16));
+  const size_t one_row = (size_t)hidden * sizeof(float);
+  if (one_row > 48 * 1024) return TL_ERR_UNSUPPORTED;
+  const size_t rows = ROUTE_TOKENS * (size_t)hidden * (dtype == TL_DTYPE_F32 ? sizeof(float) : sizeof(__nv_bfloat16));
   // several tokens a block where that leaves a block for every SM, and their rows and scores fit the shared memory
-  constexpr int SMS = 148;
-  const bool several = tokens >= SMS * ROUTE_TOKENS && ROUTE_TOKENS * (row + 2 * MAX_EXPERTS * sizeof(float)) <= 48 * 1024;
-#define TL_ROUTE(T, TOKENS, EACH)                                                                                             \
-  tl::launch_kernel(moe_route_kernel<T, TOKENS, EACH>, (unsigned)((tokens + TOKENS - 1) / TOKENS), ROUTE_WARPS * 32, TOKENS * row, \
-                    stream, (const T*)x, ldx, router, router_bias, choice, weight, tokens, hidden, experts, top, score_mode,     \
-                    renormalize, groups, keep, renorm_eps, correction, scale, gate_w, gate_out)
+  const bool several = tokens >= sm_count() * ROUTE_TOKENS && rows + ROUTE_TOKENS * 2 * MAX_EXPERTS * sizeof(float) <= 48 * 1024;
+#define TL_ROUTE(KERNEL, T, BLOCKS, SMEM)                                                                                       \
+  tl::launch_kernel(KERNEL<T>, (unsigned)(BLOCKS), ROUTE_WARPS * 32, SMEM, stream, (const T*)x, ldx, router, router_bias, choice, \
+                    weight, tokens, hidden, experts, top, score_mode, renormalize, groups, keep, renorm_eps, correction, scale,  \
+                    gate_w, gate_out)
+  const int blocks = several ? (tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS : tokens;
   if (dtype == TL_DTYPE_F32) {
-    if (several) TL_ROUTE(float, ROUTE_TOKENS, ROUTE_EACH); else TL_ROUTE(float, 1, 1);
+    if (several) TL_ROUTE(moe_route_many_kernel, float, blocks, rows); else TL_ROUTE(moe_route_kernel, float, blocks, one_row);
   } else {
-    if (several) TL_ROUTE(__nv_bfloat16, ROUTE_TOKENS, ROUTE_EACH); else TL_ROUTE(__nv_bfloat16, 1, 1);
+    static const cudaError_t wide = cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+    if (wide != cudaSuccess) return (int)wide;
+    if (several) TL_ROUTE(moe_route_many_kernel, __nv_bfloat16, blocks, rows);
+    else TL_ROUTE(moe_route_kernel, __nv_bfloat16, blocks, one_row);
   }
 #undef TL_ROUTE
   return TL_LAUNCH_CHECK();
