@@ -888,16 +888,18 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const Params
     vt.next();
     key_first += BLOCK_N;
   };
-  // two tiles a turn, so that the scores change places without copies
+  // A body a tile and moves for the scores, not two tiles a turn: most CTAs have three tiles, and what they wait for is their
+  // first pass through the instructions (one request, 24 layers of head_dim 64: 1,000 tokens 775 -> 763 us a step, 300 766 -> 762).
   float s[2][4], s_next[2][4];
   if (num_tiles > 0) multiply_keys(s);
 #pragma unroll 1
-  for (int t = 0; t < num_tiles; t += 2) {
+  for (int t = 0; t < num_tiles; ++t) {
     if (t + 1 < num_tiles) multiply_keys(s_next);
     finish_tile(s);
-    if (t + 1 >= num_tiles) break;
-    if (t + 2 < num_tiles) multiply_keys(s);
-    finish_tile(s_next);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] = s_next[i][e];
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
