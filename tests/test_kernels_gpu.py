@@ -774,6 +774,9 @@ def test_a_bounded_wait_that_runs_out_is_reported_and_the_device_stays_usable():
     ([9000, 3, 128, 2000] * 10, 8, 8, 64, 64, None, True),  # one item over several CTAs; only some requests of the step
     ([3000, 200, 1023, 4096] * 30, 4, 2, 128, 8, 1024, False),  # a window
     ([40] * 384, 4, 2, 64, 16, None, False),  # more items than CTAs are resident
+    ([9000, 130, 65, 64, 5, 200, 191, 320] * 3, 14, 2, 64, 16, None, False),  # the most pairs that take the short rings
+    ([9000, 130, 65, 64, 5, 200, 191, 320] * 3 + [77], 14, 2, 64, 16, None, False),  # one request more
+    ([20000], 8, 1, 64, 8, None, False),
 ])
 def test_attention_mma_walks_the_tiles_of_all_requests(lens, nh, nkv, d, page, window, subset):
     """Large batches of unequal lengths with the engine's key splits: against float64 within bfloat16's rounding of the

@@ -634,13 +634,15 @@ attention_mma_kernel(const Params p) {
 // 64 of 4,096: 102 -> 89 (6.0 TB/s), 128 of 100 to 1,024: 52 -> 39, 24 of 210 to 2,100: 20.7 -> 16.2, 8 of 4,096: 18.5 -> 16.3;
 // 14 on 2 of 64, 128 of 200 to 2,048: 37 -> 28; one request of 300: 5.5 -> 5.7.
 constexpr int DECODE_THREADS = THREADS + 32;
-__host__ __device__ constexpr int decode_stages(int d) { return d == 128 ? 3 : 4; }
+// Tiles of keys (and of values) in a ring.  At head_dim 64 grids of few requests take three: their CTAs have about three tiles, and
+// the less shared memory lets them start beside the kernel before (24 layers of 14 heads on 2: 1 request of 100 tokens 766 -> 756 us
+// a step, 8 of 300 827 -> 812, 16 of 1,000 870 -> 865, 1 of 4,000 equal; but 32 of 3,000 1,116 -> 1,129, 48 of 150 to 1,500 1,222 -> 1,238).
+__host__ __device__ constexpr int decode_stages(int d, bool few) { return d == 128 || few ? 3 : 4; }
 __host__ __device__ constexpr int decode_ctas(int d) { return d == 128 ? 2 : 3; }  // resident an SM
 
-template <int D, bool EXTRAS>
+template <int D, int STAGES, bool EXTRAS>
 __global__ void __launch_bounds__(DECODE_THREADS, decode_ctas(D))
 attention_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
-  constexpr int STAGES = decode_stages(D);
   constexpr int KSTEPS = D / 16, DTILES = D / 8, TILE = BLOCK_N * D;
   if (threadIdx.x == THREADS) tc::prefetch_tensormap(&map_kv);
   extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1032,16 +1034,15 @@ int launch(const Params& p, int tiles, cudaStream_t stream) {
   return TL_LAUNCH_CHECK();
 }
 
-template <int D, bool EXTRAS>
+template <int D, int STAGES, bool EXTRAS>
 int launch_decode(const CUtensorMap& map_kv, const Params& p, int tiles, cudaStream_t stream) {
-  constexpr int STAGES = decode_stages(D);
   // the rings, Q, the barriers and the abort word, room to start on a 1024-byte boundary
   constexpr int SMEM = (STAGES * 2 * BLOCK_N * D + 16 * D) * 2 + 4 * STAGES * 8 + 16 + 1024;
   static_assert(WARPS * 16 * (D + 2) * 4 <= STAGES * 2 * BLOCK_N * D * 2, "merge buffer fits the rings");
   static_assert(decode_ctas(D) * (SMEM + 1024) <= 228 * 1024, "the CTAs an SM is to hold");
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(attention_decode_kernel<D, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t err = cudaFuncSetAttribute(attention_decode_kernel<D, STAGES, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
@@ -1050,7 +1051,7 @@ int launch_decode(const CUtensorMap& map_kv, const Params& p, int tiles, cudaStr
   // grids are launched WITHOUT overlap: CTAs that start while the small kernel before them
   // still occupies the SMs are placed unevenly, and a bandwidth-bound grid's time is set by
   // its most loaded SM (measured: batch 64 decode lost 9% with an overlapped launch).
-  tl::launch_kernel_opt(tiles <= p.overlap_max_tiles || p.late_wait, attention_decode_kernel<D, EXTRAS>,
+  tl::launch_kernel_opt(tiles <= p.overlap_max_tiles || p.late_wait, attention_decode_kernel<D, STAGES, EXTRAS>,
                         dim3(tiles, p.nkv, p.splits), DECODE_THREADS, SMEM, stream, map_kv, p);
   return TL_LAUNCH_CHECK();
 }
@@ -1065,6 +1066,14 @@ bool decode_tma_enabled() {
   return value == 1;
 }
 
+int sm_count() {
+  static const int sms = [] {
+    int device = 0, n = 0;
+    return cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+  }();
+  return sms;
+}
+
 // Whether 16-row tiles run on the decode kernel: pages its TMA boxes divide a key tile into.
 bool takes_decode_kernel(int page_size) {
   return decode_tma_enabled() && page_size >= 8 && page_size % 8 == 0 && BLOCK_N % page_size == 0;
@@ -1077,7 +1086,9 @@ int launch_for(const Params& p, long long num_pages, int tiles, bool rows16, cud
   memset(&map_kv, 0, sizeof(map_kv));
   const bool tma = num_pages > 0 && takes_decode_kernel(p.page_size) &&
                    cached_map(&map_kv, p.pages, (uint64_t)num_pages * 2 * p.nkv * p.page_size, D, (uint32_t)p.page_size);
-  return tma ? launch_decode<D, EXTRAS>(map_kv, p, tiles, stream) : launch<D, true, EXTRAS>(p, tiles, stream);
+  if (!tma) return launch<D, true, EXTRAS>(p, tiles, stream);
+  if (3ll * tiles * p.nkv <= sm_count()) return launch_decode<D, decode_stages(D, true), EXTRAS>(map_kv, p, tiles, stream);
+  return launch_decode<D, decode_stages(D, false), EXTRAS>(map_kv, p, tiles, stream);
 }
 
 }  // namespace
