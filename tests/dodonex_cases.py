@@ -65,6 +65,17 @@ CASES = {
               layer("general_delta", {"heads": 2, "dim": 64, "decay_rank": 16}, ff=192, limit=1.2),
               layer("latent_attention", latent(4, 32, 16, 32, 64, 48, kv_from=0), ff=192, limit=1.2),
           ]},
+    # head and value sizes whose whole prompts expand their keys and values: a rotation over part of the rotated entries, a
+    # layer on another one's cache, a head size of 128 beside a value size of 64.  Latent attention alone: the delta rule's norm a
+    # head makes of a sequence's first tokens the sign of a product (k . r), which rounding turns where it is small; with weights
+    # off by a relative 2^-9 the float64 logits of a model with two such layers differ by up to 0.4 of their size, of this one by 0.015.
+    "T": {"architecture": "Dodonex", "vocab": 149, "width": 128, "embedding": {"scale": 2.0},
+          "norm": {"eps": 1e-5, "groups": 2}, "residual_mult": 0.4, "logit_scale": 0.8,
+          "layers": [
+              layer("latent_attention", latent(2, 64, 32, 64, 72, 40, dims=16), ff=96, limit=1.2),
+              layer("latent_attention", latent(2, 64, 32, 64, 72, 40, dims=16, kv_from=0), ff=96, limit=1.2),
+              layer("latent_attention", latent(1, 128, 16, 64, 48, 24), ff=96, limit=1.2),
+          ]},
 }
 
 

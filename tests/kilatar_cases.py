@@ -105,6 +105,14 @@ CASES = {
               parallel(chunked(5, 5, 12, 12, 0.3, 1000, rot(300.0, 4, (2.0, 1.0, 3.0, 16))),
                        lightning(2, 10, 14, (0.8, 0.95)), dense(28)),
           ]},
+    # latent attention of sizes whose whole prompts expand their keys and values: direct queries, a gate, an interleaved
+    # rotation over part of the rotated entries
+    "T": {"architecture": "Kilatar", "vocab": 113, "width": 128, "norm": {"eps": 1e-6},
+          "layers": [
+              latent(2, 64, 48, 128, 40, 0.09, rot(1000.0, 32), dense(96)),
+              mamba(2, 24, 8, 1, 2, 1, None),
+              latent(3, 128, 16, 64, 64, 0.08, rot(20000.0, 16), dense(72)),
+          ]},
 }
 
 

@@ -61,6 +61,81 @@ def test_steps_of_many_tokens(dtype):
     cases.assert_close(cases.replay(runner, "b", ids, [30, 270]), want, dtype, "270 behind 30")
 
 
+def _calls(monkeypatch, *names):
+    """How often each of these functions of ``ops`` is called."""
+    from torchlet_b200 import ops
+
+    counts = dict.fromkeys(names, 0)
+    for name in names:
+        def counted(*args, name=name, inner=getattr(ops, name), **kwargs):
+            counts[name] += 1
+            return inner(*args, **kwargs)
+
+        monkeypatch.setattr(ops, name, counted)
+    return counts
+
+
+def _step(runner, portions):
+    """One step of (request, tokens): every position's logits, by request."""
+    from torchlet_b200.engine import StepEntry
+
+    logits = runner.step([StepEntry(r, ids, list(range(len(ids)))) for r, ids in portions]).cpu()
+    return dict(zip([r for r, _ in portions], logits.split([len(ids) for _, ids in portions])))
+
+
+@pytest.mark.parametrize("lengths", [(300,), (257, 2, 130), (40, 256)])
+def test_whole_prompts_with_expanded_keys(lengths, monkeypatch):
+    """Steps of whole prompts on the kernel that expands keys and values, each request then continued behind its cache: one
+    token, and a portion, on the latent form."""
+    counts = _calls(monkeypatch, "latent_prompt", "latent_attention_mma")
+    seqs = [cases.plain_logits("T", n + 34, 60 + n) for n in lengths]
+    runner = cases.make_runner("T", "bfloat16", num_pages=80)
+    for r in range(len(lengths)):
+        runner.admit(r)
+    got = _step(runner, [(r, seqs[r][0][:n]) for r, n in enumerate(lengths)])
+    assert counts["latent_prompt"] == 3 and counts["latent_attention_mma"] == 0
+    for r, n in enumerate(lengths):
+        cases.assert_close(got[r], seqs[r][1][:n], "bfloat16", f"prompt {r}")
+    for first, last in ((0, 1), (1, 34)):
+        got = _step(runner, [(r, seqs[r][0][n + first:n + last]) for r, n in enumerate(lengths)])
+        for r, n in enumerate(lengths):
+            cases.assert_close(got[r], seqs[r][1][n + first:n + last], "bfloat16", f"request {r} behind its prompt")
+    assert counts["latent_prompt"] == 3
+
+
+@pytest.mark.parametrize("before,tokens", [(30, 270), (1, 300)])
+def test_portions_behind_cached_tokens_keep_the_latent_form(before, tokens, monkeypatch):
+    counts = _calls(monkeypatch, "latent_prompt")
+    ids, want = cases.plain_logits("T", before + tokens, 91)
+    got = cases.replay(cases.make_runner("T", "bfloat16"), "a", ids, [before, tokens])
+    cases.assert_close(got, want, "bfloat16", f"{tokens} behind {before}")
+    assert counts["latent_prompt"] == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("decoders,tokens,chunked", [(2, 96, True), (2, 95, False), (1, 256, True), (1, 255, False), (3, 300, True)])
+def test_long_portions_beside_decoding_requests(dtype, decoders, tokens, chunked, monkeypatch):
+    """A prompt in one step with requests that decode: their recurrences run on kernels of their own where the portion's goes
+    chunk by chunk, and every request continues from the state its kernel left."""
+    counts = _calls(monkeypatch, "delta_chunked", "delta_scan")
+    seqs = [cases.plain_logits("R", 20, 70 + r) for r in range(decoders)] + [cases.plain_logits("R", tokens + 5, 80)]
+    runner = cases.make_runner("R", dtype)
+    for r in range(decoders + 1):
+        runner.admit(r)
+    for r in range(decoders):
+        _step(runner, [(r, seqs[r][0][:17])])
+    counts["delta_scan"] = counts["delta_chunked"] = 0
+    order = [decoders] + list(range(decoders)) if decoders == 2 else list(range(decoders + 1))
+    got = _step(runner, [(r, seqs[r][0][:tokens] if r == decoders else seqs[r][0][17:18]) for r in order])
+    assert counts["delta_chunked"] == (chunked and dtype == "bfloat16") and counts["delta_scan"] == 1
+    for r in range(decoders):
+        cases.assert_close(got[r], seqs[r][1][17:18], dtype, f"decoding request {r}")
+    cases.assert_close(got[decoders], seqs[decoders][1][:tokens], dtype, "the portion")
+    got = _step(runner, [(r, seqs[r][0][tokens:] if r == decoders else seqs[r][0][18:]) for r in order])
+    for r in range(decoders + 1):
+        cases.assert_close(got[r], seqs[r][1][tokens if r == decoders else 18:], dtype, f"request {r} afterwards")
+
+
 def test_scratch_memory_of_the_delta_rule_is_that_of_one_token_and_stays():
     """What the first decode step allocates for the recurrence serves every later step of the token budget: a long portion, and
     many that each end in a chunk of a few tokens."""

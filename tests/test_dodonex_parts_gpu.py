@@ -339,6 +339,55 @@ def test_delta_chunks_in_passes_give_the_bits_of_one(room):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("lens,D,V", [([129, 200, 3, 140], 64, 128), ([70, 130, 300], 128, 64)])
+def test_whole_prompts_beside_rows_without_a_number(lens, D, V):
+    """A key tile reaches into the next request's rows: NaN there stays its own."""
+    from torchlet_b200 import ops
+
+    T, H, bf = sum(lens), 2, torch.bfloat16
+    queries, keys, k_rot, values = (rand(T, n, seed=i).to(DEV).to(bf) for i, n in enumerate((H * (D + 64), H * D, 64, H * V)))
+    ends = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    step = ops.latent_prompt_tokens()
+    tile_req, tile_row = (torch.tensor(x, dtype=torch.int32, device=DEV)
+                          for x in zip(*[(r, row) for r, n in enumerate(lens) for row in range(0, n, step)]))
+
+    def run():
+        out = torch.full((T, H * V), -1.0, device=DEV, dtype=bf)
+        ops.latent_prompt(queries, keys, k_rot, values, ends, tile_req, tile_row, tile_req.numel(), out, H, D, 64, V, 0.1)
+        assert ops.latent_prompt_error() == 0
+        return out
+
+    clean = run()
+    for t in (keys, k_rot, values):
+        t[lens[0]:lens[0] + lens[1]] = float("nan")
+    others = [i for i in range(T) if not lens[0] <= i < lens[0] + lens[1]]
+    assert clean.isfinite().all() and torch.equal(run()[others], clean[others])
+
+
+@pytest.mark.parametrize("R,dims", [(32, 16), (48, 48), (64, 2), (16, 0)])
+def test_rows_of_whole_prompts_turn_the_rotated_entries_alone(R, dims):
+    from torchlet_b200 import ops
+
+    T, H, D, rank, page_size, bf = 130, 2, 64, 40, 16, torch.bfloat16
+    q = rand(T, H * (D + R) + 8, seed=1).to(DEV)[:, 8:]  # (a column range of a wider product)
+    pages = rand(10, 1, 1, page_size, rank + R, seed=2).to(DEV).to(bf)
+    table = torch.arange(9, 0, -1, dtype=torch.int32, device=DEV)[None]
+    inv_freq = (500.0 ** (-2.0 * torch.arange(dims // 2, dtype=torch.float64) / max(dims, 1))).float().to(DEV)
+    positions = torch.arange(T, dtype=torch.int32, device=DEV)
+    queries, c, k_rot = (torch.empty(T, n, device=DEV, dtype=bf) for n in (H * (D + 64), rank, 64))
+    ops.latent_prompt_rows(q, inv_freq, positions, torch.zeros_like(positions), table, pages, page_size, queries, c, k_rot, H, D, R, dims)
+    x = q.contiguous().double().view(T, H, D + R)
+    want = torch.zeros(T, H, D + 64, dtype=torch.float64, device=DEV)
+    want[..., :D + R] = x
+    angle = positions.double()[:, None, None] * inv_freq.double()
+    a, b = x[..., D:D + dims // 2], x[..., D + dims // 2:D + dims]
+    want[..., D:D + dims] = torch.cat((a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()), -1)
+    # one rounding to bfloat16, and the float32 angle's own (130 x 2^-24)
+    assert ((queries.double().view_as(want) - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+    rows = pages[table[0].long()].view(-1, rank + R)[:T]
+    assert torch.equal(c, rows[:, :rank]) and torch.equal(k_rot[:, :R], rows[:, rank:]) and not k_rot[:, R:].any()
+
+
 @pytest.mark.parametrize("lens,H,D,R,V,rank,page_size", [([128], 1, 64, 16, 64, 64, 16), ([257, 2, 130], 2, 128, 64, 128, 72, 8),
                                                           ([129, 300], 3, 64, 32, 128, 40, 16), ([513, 127], 2, 128, 48, 64, 64, 32)])
 def test_latent_attention_of_whole_prompts(lens, H, D, R, V, rank, page_size):

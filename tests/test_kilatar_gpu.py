@@ -24,6 +24,22 @@ def test_whole_prompt_and_first_tokens(name, dtype):
         cases.assert_close(got, want, dtype, f"{name} whole {length}")
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_whole_prompts_of_a_gated_latent_attention_without_query_latent(dtype, monkeypatch):
+    """In bfloat16 on the kernel that expands keys and values; the queries are columns of the first product."""
+    from torchlet_b200 import ops
+
+    calls = []
+    inner = ops.latent_prompt
+    monkeypatch.setattr(ops, "latent_prompt", lambda *args, **kwargs: calls.append(1) or inner(*args, **kwargs))
+    ids, want = cases.plain_logits("T", 300, 13)
+    runner = cases.make_runner("T", dtype)
+    cases.assert_close(cases.replay(runner, "a", ids, [300]), want, dtype, "300 tokens")
+    assert len(calls) == (2 if dtype == "bfloat16" else 0)
+    cases.assert_close(cases.replay(runner, "b", ids, [262, 1, 37]), want, dtype, "portions")
+    assert len(calls) == (4 if dtype == "bfloat16" else 0)
+
+
 @pytest.mark.parametrize("name", ["P", "Q"])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_the_stream_after_every_layer_run(name, dtype):

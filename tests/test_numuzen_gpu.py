@@ -49,6 +49,35 @@ def test_the_stream_after_every_layer(dtype):
         cases.assert_close(got.cpu(), want.float(), dtype, f"stream after layer {i}")
 
 
+@pytest.mark.parametrize("decoders,tokens,chunked", [(2, 320, True), (2, 319, False), (0, 333, True)])
+def test_long_portions_beside_decoding_requests(decoders, tokens, chunked, monkeypatch):
+    """A prompt in one step with requests that decode: the portion's linear attention goes chunk by chunk, theirs token by token,
+    and every request continues from the state its kernel left."""
+    from torchlet_b200 import ops
+    from torchlet_b200.engine import StepEntry
+
+    calls = []
+    inner = ops.gla_chunked
+    monkeypatch.setattr(ops, "gla_chunked", lambda *args, **kwargs: calls.append(1) or inner(*args, **kwargs))
+    name = cases.variant("R", "bfloat16")
+    seqs = [cases.plain_logits(name, 20, 70 + r) for r in range(decoders)] + [cases.plain_logits(name, tokens + 5, 80)]
+    runner = cases.make_runner(name, "bfloat16")
+
+    def step(spans):
+        entries = [StepEntry(r, seqs[r][0][a:b], list(range(b - a))) for r, a, b in spans]
+        logits = runner.step(entries).cpu()
+        for (r, a, b), rows in zip(spans, logits.split([b - a for _, a, b in spans])):
+            cases.assert_close(rows, seqs[r][1][a:b], "bfloat16", f"request {r}, tokens {a} to {b}")
+
+    for r in range(decoders + 1):
+        runner.admit(r)
+    for r in range(decoders):
+        step([(r, 0, 17)])
+    step([(decoders, 0, tokens)] + [(r, 17, 18) for r in range(decoders)])
+    assert len(calls) == (1 if chunked else 0)  # (the other such layer's heads are wider than the chunks take)
+    step([(r, 18, 20) for r in range(decoders)] + [(decoders, tokens, tokens + 5)])
+
+
 def test_scratch_memory_of_the_linear_attention_stays():
     """What the first long portion allocates for its chunks serves every later step of the token budget, such as one whose
     requests each end in a chunk of one token."""
