@@ -31,7 +31,6 @@
 #include <math.h>
 
 #include <mutex>
-#include <type_traits>
 #include <unordered_map>
 
 #include "common.cuh"
@@ -632,7 +631,7 @@ attention_mma_kernel(const Params p) {
 // SM: a tile of 64 keys of 128 in 0.77 us (pages of 16 tokens; 0.62 with pages of 64) against 1.28 with a block barrier a tile
 // and the request on a multiplying warp's path.  28 query heads on 4, 64 requests of 300 to 3,000 tokens: 72 -> 48 us (4.4 TB/s),
 // 64 of 4,096: 102 -> 89 (6.0 TB/s), 128 of 100 to 1,024: 52 -> 39, 24 of 210 to 2,100: 20.7 -> 16.2, 8 of 4,096: 18.5 -> 16.3;
-// 14 on 2 of 64, 128 of 200 to 2,048: 37 -> 28; one request of 300: 5.5 -> 5.7.
+// 14 on 2 of 64, 128 of 200 to 2,048: 37 -> 28; a step of 24 such layers, one request of 100 tokens: 759 -> 756, of 1,000 766 -> 760.
 constexpr int DECODE_THREADS = THREADS + 32;
 // Tiles of keys (and of values) in a ring.  At head_dim 64 grids of few requests take three: their CTAs have about three tiles, and
 // the less shared memory lets them start beside the kernel before (24 layers of 14 heads on 2: 1 request of 100 tokens 766 -> 756 us

@@ -19,6 +19,8 @@
 // chunks: 2 CHUNK sums over S that do not wait for one another, then one update of S.  Everything is float32; every decay
 // between two tokens is a product of the decays between them, never a quotient.
 //
+// Error against 64 bits, whose sums differ in their order alone: 1.18e-7 against the scan's 1.13e-7 (random rows), 5.0 against
+// 4.3e-7 (64 nearly equal keys, slow decays), 2.4 against 2.7e-6 (512 of them).
 // One request of 2,048 tokens, 32 heads of 64: prepare 106 and scan 177 us against 80 and 362 token by token (0.69 us a chunk
 // of 8; a chunk's reads one after the other instead of all ahead of their use: 1.1).  The
 // order of a token's additions depends on where its chunk starts, so this form serves the bfloat16 engine; the float32

@@ -9,8 +9,8 @@
 //   proj[t] = [ r (H D) | k (H D) | v (H D) | g (H D) | a' (H D) | l (rank) ].
 //
 // Three kernels:
-//   prepare  one block per (8 tokens, head): w, u and a * u of every key channel;
-//   scan     one block per (request, head): the columns of S are independent of one another;
+//   prepare  one block per (8 tokens, head), or (token, head) where few: w, u and a * u of every key channel;
+//   scan     one block per (request, head) or 16 columns of one: the columns of S are independent of one another;
 //            four lanes share a column, each keeps a quarter of it in registers (and serves two
 //            columns, so that the vectors it reads are used twice), and the block
 //            walks the request's tokens of this step in order; r, k, v, w, u, a*u of a few tokens

@@ -23,7 +23,7 @@
 //       step of 8 tokens at 24 such layers spent 30 ms in its products and spends 1 now.
 //   gemm_f32_tile_kernel    more rows: bound by the shared-memory reads of the 8 x 8 (or 8 x 4) register tile, two 16-byte
 //       reads an operand and k for 64 products.  Where the tiles leave SMs idle, the four blocks of a cluster take a quarter
-//       of K each.  509 tokens, K x N: 896 x 9728 245 us (36 TFLOP/s), 4864 x 896 148 us, 896 x 896 35 us; 42 TFLOP/s on the
+//       of K each.  509 tokens, K x N: 896 x 9728 212 us (42 TFLOP/s), 4864 x 896 148 us, 896 x 896 35 us; 42 TFLOP/s on the
 //       largest products.
 //   gemm_simt_kernel        any type, stride and alignment (the other two copy 16 bytes at a time, float32 alone).
 //

@@ -19,9 +19,9 @@
 // decays; below it as a product of q_t P(start of t's block, t) and k_s P(s, start of t's block).
 //
 // One request of 2,048 tokens, 16 heads of 64 x 128: 76 us for the three against 275 for the scan; 8 heads:
-// 46 against 274.  The order of a
-// token's additions depends on where its chunk starts, so this form serves the bfloat16 engine; the float32 engine, whose
-// logits do not depend on how a sequence is cut, keeps the scan.
+// 46 against 274.  Error against 64 bits, in 1e-7: 1.25 against the scan's 1.20 with decays sigmoid(x)^(1/12), 0.90 against 0.81 with
+// ^(1/2), 2.35 against 3.9 with ^(1/200).  The order of a token's additions depends on where its chunk starts, so this form serves
+// the bfloat16 engine; the float32 engine, whose logits do not depend on how a sequence is cut, keeps the scan.
 #include "common.cuh"
 
 namespace {

@@ -46,7 +46,7 @@ def portions_in_chunks(lengths) -> int:
     return LEAST_BESIDE_FEW if lengths.sum() >= 64 * lengths.size else LEAST_BESIDE
 
 
-# The chunks' records: as many bytes at most (two passes over half of the chunks each: 2,048 tokens of 32 heads 292 -> 298 us; 121
+# The chunks' records: as many bytes at most (two passes over half of the chunks each: 2,048 tokens of 32 heads 292 -> 298 us; 127
 # MB in one), but room for so many chunks, and for so many more than whole ones where requests end in a part of one.
 RECORD_BYTES, LEAST_ROOM, PARTIAL_CHUNKS = 128 << 20, 64, 16
 
